@@ -145,4 +145,22 @@ PARM_FPB_HD float fine_bits(double x, float X) {
     return d2f_bits(x - f2d_bits(X));
 }
 
+// a / b correctly rounded, given y = 1 / b correctly rounded (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): the first correction brings a y within an ulp of a / b,
+// from where the remainder a - b q is exact and q + (a - b q) y rounds to the
+// quotient.  For a and b whose quotient and remainders are far from overflow
+// and underflow; a may be 0.  Five operations where y is needed anyway.
+PARM_FPB_HD double quotient_by_reciprocal(double a, double b, double y) {
+#if defined(__CUDA_ARCH__)
+    const double q0 = __dmul_rn(a, y);
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+#else
+    const double q0 = a * y;
+    const double q1 = std::fma(std::fma(-b, q0, a), y, q0);
+    return std::fma(std::fma(-b, q1, a), y, q1);
+#endif
+}
+
 }  // namespace parm

@@ -27,6 +27,7 @@
 // (the reference adds Vec::Zero()) are skipped after an FP32 screen.
 //
 // Compiled with -fmad=false.
+#include "fpbits.cuh"
 #include "parm_check.cuh"
 
 namespace parm {
@@ -40,7 +41,31 @@ struct PairC {
     double rep;                   // LJAttractFixedRepulse, LJish: the repulsive epsilon;
                                   // LJAttractRepulseSigs: the attractive one (eps_r in eps,
                                   // sig_a in m6)
+    double e12, cut2;             // LJ kinds: 12 eps and cut^2 (set_derived)
+    bool safe;                    // 12 eps is 0 or far from overflow and underflow
+    __device__ __forceinline__ void set_derived() {
+        e12 = 12 * eps;
+        cut2 = third * third;
+        const uint32_t e = ((uint32_t)__double2hiint(e12) >> 20) & 0x7FFu;
+        safe = e12 == 0.0 || (e - 723u < 600u);   // 2^-300 .. 2^300
+    }
 };
+
+// x > y for y >= 0 and x a sum of squares or a quotient of such (+0, positive,
+// +inf or NaN): an integer comparison of the bit patterns, off the FP64 pipe
+// (a NaN is not greater)
+__device__ __forceinline__ bool above(double x, double y) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    return b > (unsigned long long)__double_as_longlong(y) && b <= 0x7FF0000000000000ull;
+}
+
+// 12 eps / rsix * (1 / rsix - 1) (LennardJonesCut::forces and its kin, fmagTimesR)
+__device__ __forceinline__ double lj_fmag(const PairC& p, double rsix) {
+    const double y = 1 / rsix;
+    const uint32_t e = ((uint32_t)__double2hiint(rsix) >> 20) & 0x7FFu;
+    const double q = (p.safe && e - 723u < 600u) ? quotient_by_reciprocal(p.e12, rsix, y) : p.e12 / rsix;
+    return q * (y - 1);
+}
 
 // Pair constants of the indexed kinds, A the pair's first atom (the later one
 // in the neighbour list: its row of the table is used, IEps*Atom::get_epsilon).
@@ -165,6 +190,15 @@ __device__ __forceinline__ PairC combine(const AtomPrm& A, const AtomPrm& B, uin
     return p;
 }
 
+// b^(n - 1) of the soft repulsions: pow(b, 1) == b exactly; the Hertzian
+// exponent 5/2 as b sqrt(b), two roundings (within an ulp and a half, closer
+// to b^1.5 than the device's pow in general, at a tenth of its FP64 operations)
+__device__ __forceinline__ double power_m1(double b, double n) {
+    if (n == 2.0) return b;
+    if (n == 2.5) return b * sqrt(b);
+    return pow(b, n - 1);
+}
+
 // pair force scale s (F = r * s); returns false beyond the cut-off
 template <int KIND>
 __device__ __forceinline__ bool force_scale(const PairC& p, double dsq, uint32_t uni, double& s) {
@@ -212,26 +246,24 @@ __device__ __forceinline__ bool force_scale(const PairC& p, double dsq, uint32_t
         return true;
     } else if constexpr (KIND == KIND_LJCUT || KIND == KIND_LJCUT_IDX) {
         double rsq = (uni & UNI_SIG_ONE) ? dsq : dsq / (p.sig * p.sig);
-        if (rsq > (p.third * p.third)) return false;
+        if (above(rsq, p.cut2)) return false;
         double rsix = rsq * rsq * rsq;
-        double fmagTimesR = 12 * p.eps / rsix * (1 / rsix - 1);
-        s = fmagTimesR / dsq;
+        s = lj_fmag(p, rsix) / dsq;
         return true;
     } else if constexpr (KIND == KIND_REPULSION || KIND == KIND_REPULSION_IDX) {
-        if (dsq > p.sig * p.sig) return false;
+        if (above(dsq, p.sig * p.sig)) return false;
         double R = sqrt(dsq);
         double b = 1.0 - (R / p.sig);
-        double pw = (p.third == 2.0) ? b : pow(b, p.third - 1);   // pow(b, 1) == b exactly
+        double pw = power_m1(b, p.third);
         s = p.eps * pw / p.sig / R;
         return true;
     } else if constexpr (KIND == KIND_LJATTRACT || KIND == KIND_LJATTRACT_IDX) {
         // LJAttractCut::forces (interaction.hpp:219-229)
         if (p.eps == 0) return false;
         double rsq = (uni & UNI_SIG_ONE) ? dsq : dsq / (p.sig * p.sig);
-        if (rsq < 1 || rsq > (p.third * p.third)) return false;
+        if (rsq < 1 || above(rsq, p.cut2)) return false;
         double rsix = rsq * rsq * rsq;
-        double fmagTimesR = 12 * p.eps / rsix * (1 / rsix - 1);
-        s = fmagTimesR / dsq;
+        s = lj_fmag(p, rsix) / dsq;
         return true;
     } else if constexpr (KIND == KIND_LOISOHERN) {
         // LoisOhernPair::forces (interaction.hpp:1729-1743): harmonic to (1 + C) sigma,
@@ -267,10 +299,9 @@ __device__ __forceinline__ bool force_scale(const PairC& p, double dsq, uint32_t
         return true;
     } else {
         double rsq = (uni & UNI_SIG_ONE) ? dsq : dsq / (p.sig * p.sig);
-        if (rsq > 1) return false;
+        if (above(rsq, 1.0)) return false;
         double rsix = rsq * rsq * rsq;
-        double fmagTimesR = 12 * p.eps / rsix * (1 / rsix - 1);
-        s = fmagTimesR / dsq;
+        s = lj_fmag(p, rsix) / dsq;
         return true;
     }
 }
@@ -370,7 +401,7 @@ __device__ __forceinline__ bool drag_force(const PairC& p, const double* r, doub
     double vdot = vij[0] * r[0] + vij[1] * r[1];
     if constexpr (ND == 3) vdot = vdot + vij[2] * r[2];
     double b = 1.0 - (R / p.sig);
-    double pw = (p.third == 2.0) ? b : pow(b, p.third - 1);   // pow(b, 1) == b exactly
+    double pw = power_m1(b, p.third);
     double sr = p.eps * pw / p.sig / R;
 #pragma unroll
     for (int d = 0; d < ND; d++) {
@@ -421,97 +452,198 @@ __device__ __forceinline__ void store3(void* p, uint32_t i, const double* o) {
     static_cast<V*>(p)[i] = t;
 }
 
+// FP32 squared distance of the minimum image (0 when the image is in doubt:
+// disp32 picks it from the coarse parts, which can be off by 1/8, so near half
+// a box length it may take the farther one); `wrap` tells whether the FP64
+// displacement needs the remainder.  It does not when every component is well
+// below half a box length without a shift: |x_i - x_j| < L/2 is its own
+// remainder (the FP32 components are within an ulp or so of the FP64 ones).
 template <int ND>
-__device__ __forceinline__ float d2_32(const SysConst& S, const float4& Ai, const float4& Bi,
-                                       const float4& Aj, const float4& Bj) {
-    float dx = disp32(Ai.x, Aj.x, Bi.x, Bj.x, S.Lhi[0], S.Llo[0], S.invLf[0]);
-    float dy = disp32(Ai.y, Aj.y, Bi.y, Bj.y, S.Lhi[1], S.Llo[1], S.invLf[1]);
-    float d2 = dx * dx + dy * dy;
-    if constexpr (ND == 3) {
-        float dz = disp32(Ai.z, Aj.z, Bi.z, Bj.z, S.Lhi[2], S.Llo[2], S.invLf[2]);
-        d2 += dz * dz;
+__device__ __forceinline__ float image32(const SysConst& S, const float4& Ai, const float4& Bi, const float4& Aj,
+                                         const float4& Bj, bool& wrap) {
+    const float Xi[3] = {Ai.x, Ai.y, Ai.z}, Xj[3] = {Aj.x, Aj.y, Aj.z};
+    const float Fi[3] = {Bi.x, Bi.y, Bi.z}, Fj[3] = {Bj.x, Bj.y, Bj.z};
+    float d2 = 0.f;
+    bool doubt = false;
+    wrap = false;
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        const float r = disp32(Xi[d], Xj[d], Fi[d], Fj[d], S.Lhi[d], S.Llo[d], S.invLf[d]);
+        d2 += r * r;
+        doubt = doubt || fabsf(r) > 0.499f * S.Lhi[d] - 0.13f;
+        wrap = wrap || !(fabsf((Xi[d] - Xj[d]) + (Fi[d] - Fj[d])) < 0.49f * S.Lhi[d]);
     }
-    return d2;
+    return doubt ? 0.f : d2;
 }
 
+// ---------------------------------------------------------------------------
+// Forces, one CTA of F64_THREADS threads per F64_ATOMS consecutive atoms.
+// What bounds it: the FP64 pipe (2 lanes per clock and SM), about 40 FP64
+// operations per interacting LJ pair.  A thread that walked one atom's list
+// kept a third of its lanes idle in the FP64 part (the listed pairs beyond the
+// cut-off) and left small systems with one warp per scheduler in a serial
+// chain over the whole list.  So, in rounds of F64_CHUNK list entries:
+//   1. a warp per atom screens the entries in FP32, 32 at a time, and appends
+//      the survivors to the atom's segment in list order;
+//   2. the CTA's survivors are numbered consecutively and evaluated one per
+//      thread, so that the FP64 warps are full; each pair's force goes to its
+//      place in the segment;
+//   3. one lane per (atom, component) adds the segment in order: the sums are
+//      the reference's, bit for bit (a pair that turns out not to interact
+//      adds +0, which changes no sum that starts at +0).
+// Measured (one GB300, LJ, ~72 listed pairs per atom, thread-per-atom kernel
+// -> this one): 379 -> 23.4 us at 1000 atoms, 385 -> 161 us at 29,667,
+// 8.03 -> 4.39 ms at 1,048,576; FP64 pipe 72 % busy at 29,667.
+// ---------------------------------------------------------------------------
+constexpr int F64_THREADS = 128;
+constexpr uint32_t F64_ATOMS = 8;    // x 3 components: the lanes of the summing warp
+constexpr uint32_t F64_CHUNK = 96;   // list entries per atom and round (whole LJ lists in one round)
+constexpr uint32_t F64_SEG = F64_CHUNK + 1;   // odd: the summing lanes read different banks
+
 template <int ND, int KIND, int MODE>
-__global__ void __launch_bounds__(BLOCK) k_force64(DevCtx c) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < c.n && c.active[c.atom_sys[i]];
+__global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
+    __shared__ double pf[ND][F64_ATOMS * F64_SEG];      // pair forces
+    __shared__ uint32_t pj[F64_ATOMS * F64_CHUNK];      // surviving neighbours
+    __shared__ uint8_t pw[F64_ATOMS * F64_CHUNK];       // 1: the minimum image needs the remainder
+    __shared__ double xs[ND][F64_ATOMS];
+    __shared__ uint32_t nn_s[F64_ATOMS], cnt[F64_ATOMS];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t i0 = blockIdx.x * F64_ATOMS;
     const uint32_t uni = c.uniform;
-    double f[3] = {0.0, 0.0, 0.0};
-    uint32_t s = 0;
-    bool member = false;
-    if (active) {
-        s = c.atom_sys[i];
-        member = c.rank[i] != NOT_MEMBER;
+    const bool all_uni = (uni & UNI_ALL) == UNI_ALL;
+    if (tid < F64_ATOMS) {
+        const uint32_t i = i0 + tid;
+        const bool go = i < c.n && c.active[c.atom_sys[i]] && c.rank[i] != NOT_MEMBER;
+        nn_s[tid] = go ? c.nnb[i] : 0u;
+        double xi[3] = {0, 0, 0};
+        if (go) load3<ND>(c.x, i, xi);
+#pragma unroll
+        for (int d = 0; d < ND; d++) xs[d][tid] = xi[d];
     }
-    if (member) {
-        const SysConst& S = c.sys[s];
-        double xi[3] = {0, 0, 0}, vi[3] = {0, 0, 0};
-        load3<ND>(c.x, i, xi);
-        if constexpr (KIND == KIND_REPULSIONDRAG) load3<ND>(c.v, i, vi);
-        const float4 Ai = c.pos[2 * (size_t)(i)], Bi = c.pos[2 * (size_t)(i) + 1];
-        const AtomPrm Pi = c.prm[i];
-        const float4 Qi = c.prm32[i];
-        const uint32_t nn = c.nnb[i];
-        const uint32_t* nb = c.nbr + (size_t)i * c.maxnb;
-        for (uint32_t k = 0; k < nn; k++) {
-            const uint32_t j = __ldg(nb + k);
-            float4 Aj, Bj;
-            ld_pos(c.pos, j, Aj, Bj);
-            float4 Qj = Qi;
-            if ((uni & UNI_ALL) != UNI_ALL) Qj = c.prm32[j];
-            // (the FP32 screen is per-axis periodic: not for a sheared box)
-            if (!S.lees && beyond32<KIND>(d2_32<ND>(S, Ai, Bi, Aj, Bj), Qi, Qj, uni)) continue;
-            double xj[3] = {0, 0, 0};
+    __syncthreads();
+    uint32_t nmax = 0;
+#pragma unroll
+    for (uint32_t a = 0; a < F64_ATOMS; a++) nmax = max(nmax, nn_s[a]);
+    const uint32_t sa = tid % F64_ATOMS, sd = tid / F64_ATOMS;   // summing lane: atom, component
+    double fsum = 0.0;
+    PairC pc;
+    bool have = false;
+    for (uint32_t base = 0; base < nmax; base += F64_CHUNK) {
+        for (uint32_t a = warp; a < F64_ATOMS; a += F64_THREADS / 32) {
+            const uint32_t hi = min(nn_s[a], base + F64_CHUNK);
+            uint32_t m = 0;
+            if (base < hi) {
+                const uint32_t i = i0 + a;
+                const SysConst& S = c.sys[c.atom_sys[i]];
+                const uint32_t* nb = c.nbr + (size_t)i * c.maxnb;
+                float4 Ai, Bi;
+                ld_pos(c.pos, i, Ai, Bi);
+                const float4 Qi = c.prm32[i];
+                for (uint32_t k0 = base; k0 < hi; k0 += 32u) {
+                    const uint32_t k = k0 + lane;
+                    bool keep = false, wrap = true;
+                    uint32_t j = 0;
+                    if (k < hi) {
+                        j = __ldg(nb + k);
+                        float4 Aj, Bj;
+                        ld_pos(c.pos, j, Aj, Bj);
+                        float4 Qj = Qi;
+                        if (!all_uni) Qj = c.prm32[j];
+                        // (the FP32 screen is per-axis periodic: not for a sheared box)
+                        const float d2 = image32<ND>(S, Ai, Bi, Aj, Bj, wrap);
+                        keep = S.lees || !beyond32<KIND>(d2, Qi, Qj, uni);
+                    }
+                    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, keep);
+                    if (keep) {
+                        const uint32_t q = a * F64_CHUNK + m + __popc(mask & ((1u << lane) - 1u));
+                        pj[q] = j;
+                        pw[q] = wrap ? 1 : 0;
+                    }
+                    m += __popc(mask);
+                }
+            }
+            if (lane == 0) cnt[a] = m;
+        }
+        __syncthreads();
+        uint32_t total = 0;
+#pragma unroll
+        for (uint32_t a = 0; a < F64_ATOMS; a++) total += cnt[a];
+        for (uint32_t t = tid; t < total; t += F64_THREADS) {
+            uint32_t a = 0, m = t;
+            while (m >= cnt[a]) m -= cnt[a++];
+            const uint32_t i = i0 + a, j = pj[a * F64_CHUNK + m];
+            const SysConst& S = c.sys[c.atom_sys[i]];
+            double xj[3] = {0, 0, 0}, r[3] = {0, 0, 0}, fo[3] = {0, 0, 0};
             load3<ND>(c.x, j, xj);
-            double r[3] = {0, 0, 0};
             if (S.lees) {
+                const double xi[3] = {xs[0][a], xs[1][a], ND == 3 ? xs[ND - 1][a] : 0.0};
                 lees_diff<ND>(S, xi, xj, r);
             } else {
 #pragma unroll
-                for (int d = 0; d < ND; d++) r[d] = remainder_exact(xi[d] - xj[d], S.L[d], S.invL[d], S.halfL[d]);
+                for (int d = 0; d < ND; d++) r[d] = xs[d][a] - xj[d];
+                if (pw[a * F64_CHUNK + m]) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) r[d] = remainder_exact(r[d], S.L[d], S.invL[d], S.halfL[d]);
+                }
             }
             double dsq = r[0] * r[0] + r[1] * r[1];
             if constexpr (ND == 3) dsq = dsq + r[2] * r[2];
-            AtomPrm Pj = Pi;
-            if ((uni & UNI_ALL) != UNI_ALL) Pj = c.prm[j];
-            PairC pc;
-            if constexpr (idx_kind<KIND>()) {
-                // the pair's first atom is the one of higher neighbour-list rank
-                const uint32_t ti = __float_as_uint(Qi.x), tj = __float_as_uint(Qj.x);
-                pc = (c.rank[i] > c.rank[j]) ? combine_idx<KIND>(c, Pi, Pj, ti, tj, uni)
-                                             : combine_idx<KIND>(c, Pj, Pi, tj, ti, uni);
-            } else {
-                pc = combine<KIND>(Pi, Pj, uni);
+            if (!all_uni || !have) {
+                const AtomPrm Pi = c.prm[i];
+                if constexpr (idx_kind<KIND>()) {
+                    // the pair's first atom is the one of higher neighbour-list rank
+                    const uint32_t ti = __float_as_uint(c.prm32[i].x), tj = __float_as_uint(c.prm32[j].x);
+                    pc = (c.rank[i] > c.rank[j]) ? combine_idx<KIND>(c, Pi, c.prm[j], ti, tj, uni)
+                                                 : combine_idx<KIND>(c, c.prm[j], Pi, tj, ti, uni);
+                } else {
+                    pc = combine<KIND>(Pi, all_uni ? Pi : c.prm[j], uni);
+                }
+                pc.set_derived();
+                have = true;
             }
             if constexpr (KIND == KIND_REPULSIONDRAG) {
-                double vj[3] = {0, 0, 0}, fo[3];
+                double vi[3] = {0, 0, 0}, vj[3] = {0, 0, 0};
+                load3<ND>(c.v, i, vi);
                 load3<ND>(c.v, j, vj);
-                if (!drag_force<ND>(pc, r, dsq, vi, vj, fo)) continue;
-#pragma unroll
-                for (int d = 0; d < ND; d++) f[d] = f[d] + fo[d];
+                if (!drag_force<ND>(pc, r, dsq, vi, vj, fo)) fo[0] = fo[1] = fo[2] = 0.0;
             } else {
                 double sc;
-                if (!force_scale<KIND>(pc, dsq, uni, sc)) continue;
+                if (force_scale<KIND>(pc, dsq, uni, sc)) {
 #pragma unroll
-                for (int d = 0; d < ND; d++) f[d] = f[d] + r[d] * sc;
+                    for (int d = 0; d < ND; d++) fo[d] = r[d] * sc;
+                }
             }
+#pragma unroll
+            for (int d = 0; d < ND; d++) pf[d][a * F64_SEG + m] = fo[d];
         }
+        __syncthreads();
+        if (sd < ND) {
+            const double* p = &pf[sd][sa * F64_SEG];
+            const uint32_t m = cnt[sa];
+#pragma unroll 4
+            for (uint32_t k = 0; k < m; k++) fsum = fsum + p[k];
+        }
+        __syncthreads();
     }
-    if (active) {
-        store3<ND>(c.f, i, f);
-        if constexpr (MODE == FM_FORCES_A) {
-            // Collection::set_forces(true): a = f/m, zero for m <= 0 or inf
-            const double m = c.m[i];
-            double a[3] = {0, 0, 0};
-            if (mobile64(m)) {
+    // the components of an atom meet in its segment
+    if (sd < ND) pf[sd][sa * F64_SEG] = fsum;
+    __syncthreads();
+    if (tid >= F64_ATOMS) return;
+    const uint32_t i = i0 + tid;
+    if (i >= c.n || !c.active[c.atom_sys[i]]) return;
+    double f[3] = {0, 0, 0};
 #pragma unroll
-                for (int d = 0; d < ND; d++) a[d] = f[d] / m;
-            }
-            store3<ND>(c.a, i, a);
+    for (int d = 0; d < ND; d++) f[d] = pf[d][tid * F64_SEG];
+    store3<ND>(c.f, i, f);
+    if constexpr (MODE == FM_FORCES_A) {
+        // Collection::set_forces(true): a = f/m, zero for m <= 0 or inf
+        const double m = c.m[i];
+        double a[3] = {0, 0, 0};
+        if (mobile64(m)) {
+#pragma unroll
+            for (int d = 0; d < ND; d++) a[d] = f[d] / m;
         }
+        store3<ND>(c.a, i, a);
     }
 }
 
@@ -552,6 +684,7 @@ __global__ void __launch_bounds__(BLOCK) k_eval64(DevCtx c, int what) {
                                        __float_as_uint(c.prm32[j].x), uni);
             else
                 pc = combine<KIND>(Pi, c.prm[j], uni);
+            pc.set_derived();
             if (what == EV_ENERGY || what == EV_CONTACTS || what == EV_OVERLAPS) {
                 double e = pair_energy<KIND>(pc, dsq, uni);
                 if (what == EV_ENERGY) acc[0] = acc[0] + e;
@@ -588,9 +721,9 @@ __global__ void __launch_bounds__(BLOCK) k_eval64(DevCtx c, int what) {
 
 template <int ND, int KIND>
 static void force64_nd_kind(const DevCtx& c, cudaStream_t s, int mode) {
-    unsigned g = grid_for(c.n);
-    if (mode == FM_FORCES_A) k_force64<ND, KIND, FM_FORCES_A><<<g, BLOCK, 0, s>>>(c);
-    else k_force64<ND, KIND, FM_FORCES><<<g, BLOCK, 0, s>>>(c);
+    const unsigned g = grid_for(c.n, F64_ATOMS);
+    if (mode == FM_FORCES_A) k_force64<ND, KIND, FM_FORCES_A><<<g, F64_THREADS, 0, s>>>(c);
+    else k_force64<ND, KIND, FM_FORCES><<<g, F64_THREADS, 0, s>>>(c);
 }
 
 template <int ND>
