@@ -391,6 +391,11 @@ int parm_debug_fpbits(const double* d, const float* f, uint32_t n, float* d2f, d
  * chosen from the density.  Results do not depend on it. */
 int parm_debug_stage_cap(parm_system* s, uint32_t cap);
 
+/* Test hook: whether an FP64 handle keeps pair-force slots (1: each pair is
+ * evaluated once) or evaluates each pair for both of its atoms (0); -1: by the
+ * library's rule.  Results do not depend on it. */
+int parm_debug_pair_slots(parm_system* s, int keep);
+
 #ifdef __cplusplus
 }
 #endif

@@ -110,6 +110,7 @@ SIGNATURES = {
     "parm_get_threads_per_atom": (C.c_int, [_h, _u32p]),
     "parm_set_active": (C.c_int, [_h, C.POINTER(C.c_uint8)]),
     "parm_debug_stage_cap": (C.c_int, [_h, C.c_uint32]),
+    "parm_debug_pair_slots": (C.c_int, [_h, C.c_int]),
     "parm_timing": (C.c_int, [_h, C.c_int]),
     "parm_timing_read": (C.c_int, [_h, _dp, _u64p, _dp, _u64p]),
     "parm_last_launches": (C.c_int, [_h, _u64p]),

@@ -132,6 +132,8 @@ struct parm_system {
     void* cell_mem = nullptr;
     void* nbr_mem = nullptr;
     void* tlst_mem = nullptr;
+    void* pairf_mem = nullptr;   // FP64 path: pair-force slots and their indices
+    void* slots_mem = nullptr;
     void* excl_mem = nullptr;
     double* staging = nullptr;
     size_t staging_bytes = 0;
@@ -154,6 +156,7 @@ struct parm_system {
     bool stg_pending = false;    // grids changed under staged lists: switch back once every system rebuilt
     std::vector<uint32_t> stg_mark;   // which() of each system when the grids changed
     uint32_t stage_cap_override = 0;  // test hook (parm_debug_stage_cap)
+    int want_slots = -1;              // test hook (parm_debug_pair_slots): 0 / 1, else by the rule
     double cell_scale = 1.0;          // cells no narrower than cell_scale x the list radius
     // page-locked words read back on the stream: [0] status, [1] rebuild
     // chains, [2, 2 + nsys) which() before a call, [2 + nsys, 2 + 2 nsys) after
@@ -168,6 +171,8 @@ struct parm_system {
         if (cell_mem) cudaFree(cell_mem);
         if (nbr_mem) cudaFree(nbr_mem);
         if (tlst_mem) cudaFree(tlst_mem);
+        if (pairf_mem) cudaFree(pairf_mem);
+        if (slots_mem) cudaFree(slots_mem);
         if (blk_mem) cudaFree(blk_mem);
         if (tab_mem) cudaFree(tab_mem);
         if (nbr16_mem) cudaFree(nbr16_mem);
@@ -515,8 +520,46 @@ struct parm_system {
                 TRY(sync_status());
             }
         }
+        TRY(plan_slots());
         clear_graphs();
         return PARM_OK;
+    }
+
+    // Pair-force slots of the FP64 path (pair64.cu): one per listed pair, so
+    // n * maxnb / 2 of them always suffice (16 or 32 bytes each, and 4 bytes per
+    // list entry for the indices).  Kept for the laws that most listed pairs
+    // take part in (LJ and its kin) from 16,384 atoms: evaluating each pair once
+    // then saves more than the second kernel and the slots cost (in-graph forces
+    // with / without: 45 / 37 us at 4096 LJ atoms, 57 / 59 at 8000, 115 / 158 at
+    // 29,667, 3350 / 4370 at 1,048,576; contact laws, where a few entries of
+    // each list interact: 20 / 16 us on 5003 spheres, 64 / 54 on 65,536 disks).
+    // And where they take at most a quarter of the free device memory and 32 GB:
+    // a larger handle evaluates each pair twice instead, which needs none of it.
+    bool slots_pay() const {
+        if (want_slots >= 0) return want_slots != 0;
+        const bool lj = kind == PARM_LJCUT || kind == PARM_LJATTRACTCUT ||
+                        (kind >= PARM_LJCUT_IEPSISIG && kind <= PARM_LJISH) || kind == PARM_LJATTRACTREPULSESIGS;
+        return lj && n >= 16384;
+    }
+    int plan_slots() {
+        if (prec != PREC_FP64 || (!c.pairf && !slots_pay())) return PARM_OK;
+        if (pairf_mem) cudaFree(pairf_mem);
+        if (slots_mem) cudaFree(slots_mem);
+        pairf_mem = slots_mem = nullptr;
+        c.pairf = nullptr;
+        c.slots = nullptr;
+        const size_t entries = (size_t)n * c.maxnb;
+        const size_t pb = entries / 2 * vbytes() + vbytes(), sb = entries * 4;
+        size_t freeb = 0, totalb = 0;
+        CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
+        if (!slots_pay() || pb + sb > std::min<size_t>(freeb / 4, (size_t)32 << 30)) return PARM_OK;
+        CUDA_TRY(cudaMalloc(&pairf_mem, pb));
+        CUDA_TRY(cudaMalloc(&slots_mem, sb));
+        c.pairf = pairf_mem;
+        c.slots = static_cast<uint32_t*>(slots_mem);
+        launch_half(c, st, 1);   // of the current lists
+        CUDA_TRY(cudaGetLastError());
+        return sync_status();
     }
 
     int request_rebuild_all() {
@@ -999,10 +1042,11 @@ struct parm_system {
     // forces (+ the cell-block kernel's band pass for the LJ cut-off)
     uint64_t step_kernels() const {
         return 3 + ((c.prec == PREC_MIXED && c.staged && kind == PARM_LJCUT) ? 1 : 0) +
+               (c.pairf ? 1 : 0) +
                (c.rsq_n ? (c.rsq_com ? 5 : 2) : 0);
     }
     uint64_t chain_len() const {
-        if (c.prec == PREC_FP64) return 11;
+        if (c.prec == PREC_FP64) return c.pairf ? 12 : 11;
         return (!c.staged && c.ntile && c.tiled) ? 11 : 10;
     }
 
@@ -1153,6 +1197,11 @@ int parm_create(parm_system** out, int ndim, uint32_t nsys, const uint32_t* nato
     A(S->alloc(c.chains, 1));
     A(S->alloc(c.params, 1));
     A(S->alloc(c.sysout, (size_t)nsys * 16));
+    if (precision == PARM_FP64) {
+        A(S->alloc(c.half_n, n));
+        A(S->alloc(c.half_base, n));
+        A(S->alloc(c.half_cnt, nsys));
+    }
     if (precision == PARM_MIXED) {
         A(S->alloc(c.bandn, 1));
         A(S->alloc(c.bandq, n));
@@ -1527,6 +1576,10 @@ int parm_set_interaction(parm_system* S, int kind, const double* params, const u
     TRY(S->setup_cells());
     uint32_t need = S->estimate_capacity();
     if (need > S->c.maxnb) TRY(S->set_capacity(need));
+    else if ((S->c.pairf != nullptr) != S->slots_pay()) {
+        TRY(S->plan_slots());
+        S->clear_graphs();
+    }
     // every list is rebuilt next (ignorechanged), in the preferred format
     const uint32_t was = S->c.staged;
     S->c.staged = (S->stg_ok && S->want_staged) ? 1u : 0u;
@@ -2055,6 +2108,16 @@ int parm_debug_stage_cap(parm_system* S, uint32_t cap) {
     TRY(S->flush());
     S->stage_cap_override = cap;
     TRY(S->plan_blocks());
+    S->clear_graphs();
+    return PARM_OK;
+}
+
+int parm_debug_pair_slots(parm_system* S, int keep) {
+    if (!S) return fail(PARM_ERR_ARG, "NULL handle");
+    if (S->prec != PREC_FP64) return PARM_OK;
+    TRY(S->flush());
+    S->want_slots = keep < 0 ? -1 : (keep != 0 ? 1 : 0);
+    TRY(S->plan_slots());
     S->clear_graphs();
     return PARM_OK;
 }

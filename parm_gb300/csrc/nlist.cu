@@ -75,6 +75,7 @@ __global__ void k_arm(DevCtx c, int count_step, int use_cond, cudaGraphCondition
 __global__ void k_zero_cells(DevCtx c) {
     uint32_t s = blockIdx.x;
     if (!c.flag[s]) return;
+    if (threadIdx.x == 0 && c.half_cnt) c.half_cnt[s] = 0u;
     uint32_t b0 = c.bucket_off[s], nb = c.sys[s].ncell + 1;
     for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) c.cell_count[b0 + b] = 0u;
 }
@@ -752,49 +753,112 @@ __global__ void __launch_bounds__(TILE_ATOMS) k_tile(DevCtx c, int all) {
 // list kept both arrays in local memory and moved ~n^2/4 entries there:
 // 268 -> 7.5 us at 1000 LJ atoms, 427 -> 31 us at 29,667, 7.57 -> 0.89 ms at
 // 1,048,576 (~72 entries; one GB300).
+// Entries of smaller rank than the atom's come first; with pair slots
+// (c.pairf), the CTA hands each list as many consecutive slots of its system.
 constexpr uint32_t SORT_CAP = 256;   // longer lists are reported, not sorted
-constexpr uint32_t SORT_WARPS = 4, SORT_SLOTS = 3;
-__global__ void __launch_bounds__(SORT_WARPS * 32) k_sort_lists(DevCtx c) {
+constexpr uint32_t SORT_WARPS = 8, SORT_SLOTS = 3;
+__global__ void __launch_bounds__(SORT_WARPS * 32) k_sort_lists(DevCtx c, int all) {
     __shared__ __align__(16) uint32_t rk[SORT_WARPS][SORT_CAP], jv[SORT_WARPS][SORT_CAP];
+    __shared__ uint32_t low[SORT_WARPS], sysw[SORT_WARPS];
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const uint32_t i = blockIdx.x * SORT_WARPS + w;   // uniform in the warp from here
-    if (i >= c.n || !c.flag[c.atom_sys[i]]) return;
-    const uint32_t cnt = c.nnb[i];
-    if (cnt < 2) return;
+    const uint32_t s = i < c.n ? c.atom_sys[i] : 0u;
+    const bool go = i < c.n && (all || c.flag[s]);
+    uint32_t cnt = go ? min(c.nnb[i], c.maxnb) : 0u;
     if (cnt > SORT_CAP) {
         if (lane == 0) atomicOr(c.status, ST_SORT_CAP);
-        return;
+        cnt = 0u;
     }
-    uint32_t* row = c.nbr + (size_t)i * c.maxnb;
-    const uint32_t padded = (cnt + 3u) & ~3u;   // <= SORT_CAP
-    for (uint32_t q = lane; q < padded; q += 32u) {
-        const uint32_t j = q < cnt ? row[q] : 0u;
-        jv[w][q] = j;
-        rk[w][q] = q < cnt ? c.rank[j] : 0xFFFFFFFFu;
-    }
-    __syncwarp();
-    for (uint32_t q0 = 0; q0 < cnt; q0 += 32u * SORT_SLOTS) {
-        uint32_t mine[SORT_SLOTS], pos[SORT_SLOTS];
-#pragma unroll
-        for (uint32_t u = 0; u < SORT_SLOTS; u++) {
-            const uint32_t q = q0 + lane + 32u * u;
-            mine[u] = q < cnt ? rk[w][q] : 0u;
-            pos[u] = 0u;
+    uint32_t below = 0u;
+    if (cnt) {
+        uint32_t* row = c.nbr + (size_t)i * c.maxnb;
+        const uint32_t ri = c.rank[i];
+        const uint32_t padded = (cnt + 3u) & ~3u;   // <= SORT_CAP
+        for (uint32_t q = lane; q < padded; q += 32u) {
+            const uint32_t j = q < cnt ? row[q] : 0u;
+            const uint32_t r = q < cnt ? c.rank[j] : 0xFFFFFFFFu;
+            jv[w][q] = j;
+            rk[w][q] = r;
+            below += r < ri ? 1u : 0u;
         }
+        below = __reduce_add_sync(0xFFFFFFFFu, below);
+        __syncwarp();
+        for (uint32_t q0 = 0; q0 < cnt; q0 += 32u * SORT_SLOTS) {
+            uint32_t mine[SORT_SLOTS], pos[SORT_SLOTS];
+#pragma unroll
+            for (uint32_t u = 0; u < SORT_SLOTS; u++) {
+                const uint32_t q = q0 + lane + 32u * u;
+                mine[u] = q < cnt ? rk[w][q] : 0u;
+                pos[u] = 0u;
+            }
 #pragma unroll 2
-        for (uint32_t t = 0; t < padded; t += 4u) {
-            const uint4 K = *reinterpret_cast<const uint4*>(&rk[w][t]);
+            for (uint32_t t = 0; t < padded; t += 4u) {
+                const uint4 K = *reinterpret_cast<const uint4*>(&rk[w][t]);
 #pragma unroll
-            for (uint32_t u = 0; u < SORT_SLOTS; u++)
-                pos[u] += (K.x < mine[u] ? 1u : 0u) + (K.y < mine[u] ? 1u : 0u) + (K.z < mine[u] ? 1u : 0u) +
-                          (K.w < mine[u] ? 1u : 0u);
-        }
+                for (uint32_t u = 0; u < SORT_SLOTS; u++)
+                    pos[u] += (K.x < mine[u] ? 1u : 0u) + (K.y < mine[u] ? 1u : 0u) + (K.z < mine[u] ? 1u : 0u) +
+                              (K.w < mine[u] ? 1u : 0u);
+            }
 #pragma unroll
-        for (uint32_t u = 0; u < SORT_SLOTS; u++) {
-            const uint32_t q = q0 + lane + 32u * u;
-            if (q < cnt) row[pos[u]] = jv[w][q];
+            for (uint32_t u = 0; u < SORT_SLOTS; u++) {
+                const uint32_t q = q0 + lane + 32u * u;
+                if (q < cnt) row[pos[u]] = jv[w][q];
+            }
         }
     }
+    if (!c.pairf) return;
+    if (lane == 0) {
+        low[w] = below;
+        sysw[w] = go ? s : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    // warp 0: one atomic per run of lists of one system
+    if (w != 0 || lane >= SORT_WARPS) return;
+    const uint32_t my = sysw[lane];
+    if (my == 0xFFFFFFFFu) return;
+    uint32_t before = 0u, total = 0u, leader = lane;
+    for (uint32_t k = 0; k < SORT_WARPS; k++) {
+        if (sysw[k] != my) continue;
+        leader = min(leader, k);
+        total += low[k];
+        if (k < lane) before += low[k];
+    }
+    const uint32_t live = __activemask();
+    uint32_t first = 0u;
+    if (leader == lane) first = atomicAdd(&c.half_cnt[my], total);
+    first = __shfl_sync(live, first, leader);
+    const uint32_t me = blockIdx.x * SORT_WARPS + lane;
+    // lists cut at their capacity (reported) need not be symmetric: never past the system's slots
+    const bool fits = (size_t)first + before + low[lane] <= (size_t)c.sys[my].natoms * c.maxnb / 2;
+    c.half_n[me] = fits ? low[lane] : 0u;
+    c.half_base[me] = (uint32_t)((size_t)c.sys[my].atom_off * c.maxnb / 2) + first + before;
+}
+
+// slots of the pairs that an atom is second in: its place in the first atom's
+// list, by bisection of that (sorted) list
+__global__ void __launch_bounds__(BLOCK) k_slots(DevCtx c, int all) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t i = blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5);
+    if (i >= c.n || !(all || c.flag[c.atom_sys[i]])) return;
+    const uint32_t cnt = min(c.nnb[i], c.maxnb), ri = c.rank[i];
+    for (uint32_t k = c.half_n[i] + lane; k < cnt; k += 32u) {
+        const uint32_t j = c.nbr[(size_t)i * c.maxnb + k];
+        const uint32_t* row = c.nbr + (size_t)j * c.maxnb;
+        uint32_t lo = 0, hi = c.half_n[j];   // first entry whose rank is not below ri
+        const uint32_t nj = hi;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (c.rank[row[mid]] < ri) lo = mid + 1; else hi = mid;
+        }
+        // not found only in lists that are about to be rebuilt (a capacity cut)
+        c.slots[(size_t)i * c.maxnb + k] = (lo < nj && row[lo] == i) ? c.half_base[j] + lo : NO_SLOT;
+    }
+}
+
+void launch_half(const DevCtx& c, cudaStream_t s, int all) {
+    if (all && c.pairf) cudaMemsetAsync(c.half_cnt, 0, 4 * (size_t)c.nsys, s);
+    k_sort_lists<<<grid_for(c.n, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(c, all);
+    if (c.pairf) k_slots<<<grid_for(c.n, BLOCK / 32), BLOCK, 0, s>>>(c, all);
 }
 
 // ---------------------------------------------------------------------------
@@ -910,7 +974,7 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
             k_copyback<2><<<ga, BLOCK, 0, s>>>(c);
             k_build_lees<2><<<ga, BLOCK, 0, s>>>(c);
         }
-        k_sort_lists<<<grid_for(c.n, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(c);
+        launch_half(c, s, 0);
         return;
     }
     if (c.nd == 3) {
@@ -925,7 +989,7 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
         else k_build<2, false><<<(c.nbucket + BUILD_WARPS - 1) / BUILD_WARPS, BUILD_WARPS * 32, 0, s>>>(c);
     }
     if (c.prec == PREC_FP64) {
-        k_sort_lists<<<grid_for(c.n, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(c);
+        launch_half(c, s, 0);
     } else if (c.ntile && c.tiled) {
         launch_tiles(c, s, 0);
     }

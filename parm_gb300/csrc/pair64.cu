@@ -452,9 +452,10 @@ __device__ __forceinline__ void store3(void* p, uint32_t i, const double* o) {
     static_cast<V*>(p)[i] = t;
 }
 
-// FP32 squared distance of the minimum image (0 when the image is in doubt:
+// FP32 squared distance of the minimum image, 0 when the image is in doubt:
 // disp32 picks it from the coarse parts, which can be off by 1/8, so near half
-// a box length it may take the farther one); `wrap` tells whether the FP64
+// a box length it may take the farther one, and beyond 2^20 the coarse parts
+// and their difference are no longer exact.  `wrap` tells whether the FP64
 // displacement needs the remainder.  It does not when every component is well
 // below half a box length without a shift: |x_i - x_j| < L/2 is its own
 // remainder (the FP32 components are within an ulp or so of the FP64 ones).
@@ -470,55 +471,144 @@ __device__ __forceinline__ float image32(const SysConst& S, const float4& Ai, co
     for (int d = 0; d < ND; d++) {
         const float r = disp32(Xi[d], Xj[d], Fi[d], Fj[d], S.Lhi[d], S.Llo[d], S.invLf[d]);
         d2 += r * r;
-        doubt = doubt || fabsf(r) > 0.499f * S.Lhi[d] - 0.13f;
+        doubt = doubt || fabsf(r) > 0.499f * S.Lhi[d] - 0.13f || !(fabsf(Xi[d]) < 1048576.0f) ||
+                !(fabsf(Xj[d]) < 1048576.0f);
         wrap = wrap || !(fabsf((Xi[d] - Xj[d]) + (Fi[d] - Fj[d])) < 0.49f * S.Lhi[d]);
     }
+    wrap = wrap || doubt;
     return doubt ? 0.f : d2;
 }
 
 // ---------------------------------------------------------------------------
-// Forces, one CTA of F64_THREADS threads per F64_ATOMS consecutive atoms.
-// What bounds it: the FP64 pipe (2 lanes per clock and SM), about 40 FP64
-// operations per interacting LJ pair.  A thread that walked one atom's list
-// kept a third of its lanes idle in the FP64 part (the listed pairs beyond the
-// cut-off) and left small systems with one warp per scheduler in a serial
-// chain over the whole list.  So, in rounds of F64_CHUNK list entries:
-//   1. a warp per atom screens the entries in FP32, 32 at a time, and appends
-//      the survivors to the atom's segment in list order;
-//   2. the CTA's survivors are numbered consecutively and evaluated one per
-//      thread, so that the FP64 warps are full; each pair's force goes to its
-//      place in the segment;
-//   3. one lane per (atom, component) adds the segment in order: the sums are
-//      the reference's, bit for bit (a pair that turns out not to interact
-//      adds +0, which changes no sum that starts at +0).
-// Measured (one GB300, LJ, ~72 listed pairs per atom, thread-per-atom kernel
-// -> this one): 379 -> 23.4 us at 1000 atoms, 385 -> 161 us at 29,667,
-// 8.03 -> 4.39 ms at 1,048,576; FP64 pipe 72 % busy at 29,667.
+// Forces.  What bounds them: the FP64 pipe (2 lanes per clock and SM), about
+// 40 FP64 operations per interacting LJ pair; so the FP64 part runs on full
+// warps of pairs that pass an FP32 screen, each pair once where memory allows.
+//
+// Pair forces kept (launch_force64 with c.pairf set): k_pair64 evaluates every
+// listed pair once, for its first atom (the one of higher rank: its list
+// entries below half_n), and writes the force to the pair's slot; k_sum64 adds
+// each atom's slots in list order, its own pairs and then, negated, those of
+// the atoms ranked after it: the reference's order and its f_last -= F.
+//
+// Without (handles whose slots would take too much memory): k_force64
+// evaluates every pair for both of its atoms, so it needs no slots.
+//
+// A CTA takes F64_ATOMS consecutive atoms in rounds of F64_CHUNK list entries:
+// a warp per atom screens the entries, 32 at a time, and appends the survivors
+// to the atom's segment in list order; the CTA's survivors are then numbered
+// consecutively and evaluated one per thread.  A pair that turns out not to
+// interact adds +0, which changes no sum that starts at +0.
+// Measured, LJ, ~72 listed pairs per atom (one GB300): a thread per atom that
+// walked its list 379 us at 1000 atoms, 385 us at 29,667, 8.03 ms at 1,048,576
+// (a third of its lanes idle in the FP64 part, a serial chain over the list);
+// k_force64 23.4 us, 161 us, 4.39 ms; k_pair64 + k_sum64 115 us at 29,667 and
+// 3.35 ms at 1,048,576.
 // ---------------------------------------------------------------------------
 constexpr int F64_THREADS = 128;
-constexpr uint32_t F64_ATOMS = 8;    // x 3 components: the lanes of the summing warp
+constexpr uint32_t F64_ATOMS = 8;    // x 3 components: the lanes of k_force64's summing warp
 constexpr uint32_t F64_CHUNK = 96;   // list entries per atom and round (whole LJ lists in one round)
 constexpr uint32_t F64_SEG = F64_CHUNK + 1;   // odd: the summing lanes read different banks
 
-template <int ND, int KIND, int MODE>
-__global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
-    __shared__ double pf[ND][F64_ATOMS * F64_SEG];      // pair forces
+// FP32 screen of entry (i, j): false when the pair is certainly beyond the cut-off
+template <int ND, int KIND>
+__device__ __forceinline__ bool screen64(const DevCtx& c, const SysConst& S, const float4& Ai, const float4& Bi,
+                                         const float4& Qi, uint32_t j, bool& wrap) {
+    float4 Aj, Bj;
+    ld_pos(c.pos, j, Aj, Bj);
+    float4 Qj = Qi;
+    if ((c.uniform & UNI_ALL) != UNI_ALL) Qj = c.prm32[j];
+    // (the screen is per-axis periodic: not for a sheared box)
+    const float d2 = image32<ND>(S, Ai, Bi, Aj, Bj, wrap);
+    return S.lees || !beyond32<KIND>(d2, Qi, Qj, c.uniform);
+}
+
+// pair constants of (i, j); `first` tells that i is the pair's first atom
+template <int KIND>
+__device__ __forceinline__ PairC pair_constants(const DevCtx& c, uint32_t i, uint32_t j, bool first) {
+    const uint32_t uni = c.uniform;
+    const AtomPrm Pi = c.prm[i];
+    PairC pc;
+    if constexpr (idx_kind<KIND>()) {
+        const uint32_t ti = __float_as_uint(c.prm32[i].x), tj = __float_as_uint(c.prm32[j].x);
+        pc = first ? combine_idx<KIND>(c, Pi, c.prm[j], ti, tj, uni) : combine_idx<KIND>(c, c.prm[j], Pi, tj, ti, uni);
+    } else {
+        pc = combine<KIND>(Pi, (uni & UNI_ALL) == UNI_ALL ? Pi : c.prm[j], uni);
+    }
+    pc.set_derived();
+    return pc;
+}
+
+// FP64 force of j on i (0 beyond the cut-off); `wrap`: the minimum image needs the remainder
+template <int ND, int KIND>
+__device__ __forceinline__ void force_of_pair(const DevCtx& c, const SysConst& S, uint32_t i, uint32_t j,
+                                              const double* xi, bool wrap, const PairC& pc, double* fo) {
+    double xj[3] = {0, 0, 0}, r[3] = {0, 0, 0};
+    load3<ND>(c.x, j, xj);
+    if (S.lees) {
+        lees_diff<ND>(S, xi, xj, r);
+    } else {
+#pragma unroll
+        for (int d = 0; d < ND; d++) r[d] = xi[d] - xj[d];
+        if (wrap) {
+#pragma unroll
+            for (int d = 0; d < ND; d++) r[d] = remainder_exact(r[d], S.L[d], S.invL[d], S.halfL[d]);
+        }
+    }
+    double dsq = r[0] * r[0] + r[1] * r[1];
+    if constexpr (ND == 3) dsq = dsq + r[2] * r[2];
+    fo[0] = fo[1] = fo[2] = 0.0;
+    if constexpr (KIND == KIND_REPULSIONDRAG) {
+        double vi[3] = {0, 0, 0}, vj[3] = {0, 0, 0};
+        load3<ND>(c.v, i, vi);
+        load3<ND>(c.v, j, vj);
+        if (!drag_force<ND>(pc, r, dsq, vi, vj, fo)) fo[0] = fo[1] = fo[2] = 0.0;
+    } else {
+        double sc;
+        if (force_scale<KIND>(pc, dsq, c.uniform, sc)) {
+#pragma unroll
+            for (int d = 0; d < ND; d++) fo[d] = r[d] * sc;
+        }
+    }
+}
+
+// f of internal atom i and, with MODE FM_FORCES_A, a = f/m (Collection::
+// set_forces(true): zero for m <= 0 or inf)
+template <int ND, int MODE>
+__device__ __forceinline__ void store_force(const DevCtx& c, uint32_t i, const double* f) {
+    store3<ND>(c.f, i, f);
+    if constexpr (MODE == FM_FORCES_A) {
+        const double m = c.m[i];
+        double a[3] = {0, 0, 0};
+        if (mobile64(m)) {
+#pragma unroll
+            for (int d = 0; d < ND; d++) a[d] = f[d] / m;
+        }
+        store3<ND>(c.a, i, a);
+    }
+}
+
+// The work of k_pair64 (HALF) and k_force64.
+template <int ND, int KIND, int MODE, bool HALF>
+__device__ __forceinline__ void forces64(const DevCtx& c) {
+    __shared__ double pf[HALF ? 1 : ND][HALF ? 1 : F64_ATOMS * F64_SEG];   // pair forces
     __shared__ uint32_t pj[F64_ATOMS * F64_CHUNK];      // surviving neighbours
     __shared__ uint8_t pw[F64_ATOMS * F64_CHUNK];       // 1: the minimum image needs the remainder
-    __shared__ double xs[ND][F64_ATOMS];
-    __shared__ uint32_t nn_s[F64_ATOMS], cnt[F64_ATOMS];
+    __shared__ uint16_t pk[HALF ? F64_ATOMS * F64_CHUNK : 1];   // their list entries
+    __shared__ double xs[F64_ATOMS][4];
+    __shared__ uint32_t nn_s[F64_ATOMS], cnt[F64_ATOMS], slot0[F64_ATOMS];
+    using V = typename DVec<ND>::T;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t i0 = blockIdx.x * F64_ATOMS;
-    const uint32_t uni = c.uniform;
-    const bool all_uni = (uni & UNI_ALL) == UNI_ALL;
+    const bool all_uni = (c.uniform & UNI_ALL) == UNI_ALL;
     if (tid < F64_ATOMS) {
         const uint32_t i = i0 + tid;
         const bool go = i < c.n && c.active[c.atom_sys[i]] && c.rank[i] != NOT_MEMBER;
-        nn_s[tid] = go ? c.nnb[i] : 0u;
+        nn_s[tid] = !go ? 0u : (HALF ? c.half_n[i] : c.nnb[i]);
+        slot0[tid] = HALF && go ? c.half_base[i] : 0u;
         double xi[3] = {0, 0, 0};
         if (go) load3<ND>(c.x, i, xi);
 #pragma unroll
-        for (int d = 0; d < ND; d++) xs[d][tid] = xi[d];
+        for (int d = 0; d < 3; d++) xs[tid][d] = xi[d];
     }
     __syncthreads();
     uint32_t nmax = 0;
@@ -545,19 +635,15 @@ __global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
                     uint32_t j = 0;
                     if (k < hi) {
                         j = __ldg(nb + k);
-                        float4 Aj, Bj;
-                        ld_pos(c.pos, j, Aj, Bj);
-                        float4 Qj = Qi;
-                        if (!all_uni) Qj = c.prm32[j];
-                        // (the FP32 screen is per-axis periodic: not for a sheared box)
-                        const float d2 = image32<ND>(S, Ai, Bi, Aj, Bj, wrap);
-                        keep = S.lees || !beyond32<KIND>(d2, Qi, Qj, uni);
+                        keep = screen64<ND, KIND>(c, S, Ai, Bi, Qi, j, wrap);
+                        if (HALF && !keep) static_cast<V*>(c.pairf)[slot0[a] + k] = V{};
                     }
                     const uint32_t mask = __ballot_sync(0xFFFFFFFFu, keep);
                     if (keep) {
                         const uint32_t q = a * F64_CHUNK + m + __popc(mask & ((1u << lane) - 1u));
                         pj[q] = j;
                         pw[q] = wrap ? 1 : 0;
+                        if (HALF) pk[q] = (uint16_t)k;
                     }
                     m += __popc(mask);
                 }
@@ -571,80 +657,143 @@ __global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
         for (uint32_t t = tid; t < total; t += F64_THREADS) {
             uint32_t a = 0, m = t;
             while (m >= cnt[a]) m -= cnt[a++];
-            const uint32_t i = i0 + a, j = pj[a * F64_CHUNK + m];
-            const SysConst& S = c.sys[c.atom_sys[i]];
-            double xj[3] = {0, 0, 0}, r[3] = {0, 0, 0}, fo[3] = {0, 0, 0};
-            load3<ND>(c.x, j, xj);
-            if (S.lees) {
-                const double xi[3] = {xs[0][a], xs[1][a], ND == 3 ? xs[ND - 1][a] : 0.0};
-                lees_diff<ND>(S, xi, xj, r);
-            } else {
-#pragma unroll
-                for (int d = 0; d < ND; d++) r[d] = xs[d][a] - xj[d];
-                if (pw[a * F64_CHUNK + m]) {
-#pragma unroll
-                    for (int d = 0; d < ND; d++) r[d] = remainder_exact(r[d], S.L[d], S.invL[d], S.halfL[d]);
-                }
-            }
-            double dsq = r[0] * r[0] + r[1] * r[1];
-            if constexpr (ND == 3) dsq = dsq + r[2] * r[2];
+            const uint32_t q = a * F64_CHUNK + m, i = i0 + a, j = pj[q];
             if (!all_uni || !have) {
-                const AtomPrm Pi = c.prm[i];
-                if constexpr (idx_kind<KIND>()) {
-                    // the pair's first atom is the one of higher neighbour-list rank
-                    const uint32_t ti = __float_as_uint(c.prm32[i].x), tj = __float_as_uint(c.prm32[j].x);
-                    pc = (c.rank[i] > c.rank[j]) ? combine_idx<KIND>(c, Pi, c.prm[j], ti, tj, uni)
-                                                 : combine_idx<KIND>(c, c.prm[j], Pi, tj, ti, uni);
-                } else {
-                    pc = combine<KIND>(Pi, all_uni ? Pi : c.prm[j], uni);
-                }
-                pc.set_derived();
+                pc = pair_constants<KIND>(c, i, j, HALF || c.rank[i] > c.rank[j]);
                 have = true;
             }
-            if constexpr (KIND == KIND_REPULSIONDRAG) {
-                double vi[3] = {0, 0, 0}, vj[3] = {0, 0, 0};
-                load3<ND>(c.v, i, vi);
-                load3<ND>(c.v, j, vj);
-                if (!drag_force<ND>(pc, r, dsq, vi, vj, fo)) fo[0] = fo[1] = fo[2] = 0.0;
-            } else {
-                double sc;
-                if (force_scale<KIND>(pc, dsq, uni, sc)) {
+            double fo[3];
+            force_of_pair<ND, KIND>(c, c.sys[c.atom_sys[i]], i, j, xs[a], pw[q] != 0, pc, fo);
+            if constexpr (HALF) {
+                V v;
+                double* vp = reinterpret_cast<double*>(&v);
 #pragma unroll
-                    for (int d = 0; d < ND; d++) fo[d] = r[d] * sc;
+                for (int d = 0; d < (int)(sizeof(V) / 8); d++) vp[d] = d < ND ? fo[d] : 0.0;
+                static_cast<V*>(c.pairf)[slot0[a] + pk[q]] = v;
+            } else {
+#pragma unroll
+                for (int d = 0; d < ND; d++) pf[HALF ? 0 : d][a * F64_SEG + m] = fo[d];
+            }
+        }
+        __syncthreads();
+        if constexpr (!HALF) {
+            if (sd < ND) {
+                const double* p = &pf[sd][sa * F64_SEG];
+                const uint32_t m = cnt[sa];
+#pragma unroll 4
+                for (uint32_t k = 0; k < m; k++) fsum = fsum + p[k];
+            }
+            __syncthreads();
+        }
+    }
+    if constexpr (!HALF) {
+        // the components of an atom meet in its segment
+        if (sd < ND) pf[sd][sa * F64_SEG] = fsum;
+        __syncthreads();
+        const uint32_t i = i0 + tid;
+        if (tid >= F64_ATOMS || i >= c.n || !c.active[c.atom_sys[i]]) return;
+        double f[3] = {0, 0, 0};
+#pragma unroll
+        for (int d = 0; d < ND; d++) f[d] = pf[d][tid * F64_SEG];
+        store_force<ND, MODE>(c, i, f);
+    }
+}
+
+template <int ND, int KIND, int MODE>
+__global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
+    forces64<ND, KIND, MODE, false>(c);
+}
+template <int ND, int KIND>
+__global__ void __launch_bounds__(F64_THREADS) k_pair64(DevCtx c) {
+    forces64<ND, KIND, FM_FORCES, true>(c);
+}
+
+// Per-atom sums of the pair forces, one warp per sum64_atoms() atoms on its
+// own: in rounds of 32 list entries it gathers the slots of each atom (its own
+// pairs are consecutive; another atom's pair is one 32-byte sector), drops the
+// zeros and stages the rest in list order, then one lane per (atom, component)
+// adds them.  Bound by those FP64 adds and the 32 B per entry from L2 and
+// memory: ~30 us of the 115 at 29,667 LJ atoms, 1.2 ms of 3.35 at 1,048,576.
+constexpr int SUM64_WARPS = 4;
+template <int ND>
+constexpr uint32_t sum64_atoms() { return ND == 3 ? 10u : 16u; }   // x ND components: one warp
+template <int ND, int MODE>
+__global__ void __launch_bounds__(32 * SUM64_WARPS) k_sum64(DevCtx c) {
+    constexpr uint32_t ATOMS = sum64_atoms<ND>(), GROUP = ATOMS / 2;
+    __shared__ double pf_s[SUM64_WARPS][ND][ATOMS * 33];
+    using V = typename DVec<ND>::T;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t i0 = (blockIdx.x * SUM64_WARPS + warp) * ATOMS;   // uniform in the warp from here
+    if (i0 >= c.n) return;
+    double (*pf)[ATOMS * 33] = pf_s[warp];
+    // lane a < ATOMS holds atom a's list
+    uint32_t nn = 0u, lower = 0u, b0 = 0u;
+    bool live = false;
+    if (lane < ATOMS && i0 + lane < c.n) {
+        const uint32_t i = i0 + lane;
+        live = c.active[c.atom_sys[i]] != 0u;
+        if (live && c.rank[i] != NOT_MEMBER) {
+            nn = c.nnb[i];
+            lower = c.half_n[i];
+            b0 = c.half_base[i];
+        }
+    }
+    const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, nn);
+    const uint32_t sa = lane % ATOMS, sd = lane / ATOMS;   // summing lane: atom, component
+    double fsum = 0.0;
+    for (uint32_t base = 0; base < nmax; base += 32u) {
+        const uint32_t k = base + lane;
+        uint32_t cnt = 0u;   // lane a: entries staged for atom a
+#pragma unroll
+        for (uint32_t g = 0; g < 2; g++) {
+            V w[GROUP];
+            uint32_t second = 0u;   // bit u: the atom is second in the pair
+#pragma unroll
+            for (uint32_t u = 0; u < GROUP; u++) {   // all loads before any use
+                const uint32_t a = g * GROUP + u;
+                const uint32_t na = __shfl_sync(0xFFFFFFFFu, nn, a), la = __shfl_sync(0xFFFFFFFFu, lower, a);
+                const uint32_t ba = __shfl_sync(0xFFFFFFFFu, b0, a);
+                w[u] = V{};
+                if (k < na) {
+                    const uint32_t sl = k < la ? ba + k : __ldg(c.slots + (size_t)(i0 + a) * c.maxnb + k);
+                    if (sl != NO_SLOT) w[u] = static_cast<const V*>(c.pairf)[sl];
+                    second |= (k < la ? 0u : 1u) << u;
                 }
             }
 #pragma unroll
-            for (int d = 0; d < ND; d++) pf[d][a * F64_SEG + m] = fo[d];
+            for (uint32_t u = 0; u < GROUP; u++) {
+                const uint32_t a = g * GROUP + u;
+                const unsigned long long* wb = reinterpret_cast<const unsigned long long*>(&w[u]);
+                unsigned long long any = 0;
+#pragma unroll
+                for (int d = 0; d < ND; d++) any |= wb[d];
+                const uint32_t mask = __ballot_sync(0xFFFFFFFFu, any != 0ull);
+                if (any) {
+                    const uint32_t q = a * 33u + __popc(mask & ((1u << lane) - 1u));
+                    const unsigned long long neg = (unsigned long long)((second >> u) & 1u) << 63;
+#pragma unroll
+                    for (int d = 0; d < ND; d++) pf[d][q] = __longlong_as_double((long long)(wb[d] ^ neg));
+                }
+                if (lane == a) cnt = (uint32_t)__popc(mask);
+            }
         }
-        __syncthreads();
+        __syncwarp();
+        const uint32_t m = __shfl_sync(0xFFFFFFFFu, cnt, sa);
         if (sd < ND) {
-            const double* p = &pf[sd][sa * F64_SEG];
-            const uint32_t m = cnt[sa];
+            const double* p = &pf[sd][sa * 33u];
 #pragma unroll 4
-            for (uint32_t k = 0; k < m; k++) fsum = fsum + p[k];
+            for (uint32_t q = 0; q < m; q++) fsum = fsum + p[q];
         }
-        __syncthreads();
+        __syncwarp();
     }
-    // the components of an atom meet in its segment
-    if (sd < ND) pf[sd][sa * F64_SEG] = fsum;
-    __syncthreads();
-    if (tid >= F64_ATOMS) return;
-    const uint32_t i = i0 + tid;
-    if (i >= c.n || !c.active[c.atom_sys[i]]) return;
+    // the components of an atom meet in its first staged place
+    if (sd < ND) pf[sd][sa * 33u] = fsum;
+    __syncwarp();
+    if (!live) return;
     double f[3] = {0, 0, 0};
 #pragma unroll
-    for (int d = 0; d < ND; d++) f[d] = pf[d][tid * F64_SEG];
-    store3<ND>(c.f, i, f);
-    if constexpr (MODE == FM_FORCES_A) {
-        // Collection::set_forces(true): a = f/m, zero for m <= 0 or inf
-        const double m = c.m[i];
-        double a[3] = {0, 0, 0};
-        if (mobile64(m)) {
-#pragma unroll
-            for (int d = 0; d < ND; d++) a[d] = f[d] / m;
-        }
-        store3<ND>(c.a, i, a);
-    }
+    for (int d = 0; d < ND; d++) f[d] = pf[d][lane * 33u];
+    store_force<ND, MODE>(c, i0 + lane, f);
 }
 
 // per-atom partial sums over the half list (neighbours of smaller rank), i.e.
@@ -722,6 +871,13 @@ __global__ void __launch_bounds__(BLOCK) k_eval64(DevCtx c, int what) {
 template <int ND, int KIND>
 static void force64_nd_kind(const DevCtx& c, cudaStream_t s, int mode) {
     const unsigned g = grid_for(c.n, F64_ATOMS);
+    if (c.pairf) {
+        k_pair64<ND, KIND><<<g, F64_THREADS, 0, s>>>(c);
+        const unsigned gs = grid_for(c.n, (int)(SUM64_WARPS * sum64_atoms<ND>()));
+        if (mode == FM_FORCES_A) k_sum64<ND, FM_FORCES_A><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
+        else k_sum64<ND, FM_FORCES><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
+        return;
+    }
     if (mode == FM_FORCES_A) k_force64<ND, KIND, FM_FORCES_A><<<g, F64_THREADS, 0, s>>>(c);
     else k_force64<ND, KIND, FM_FORCES><<<g, F64_THREADS, 0, s>>>(c);
 }

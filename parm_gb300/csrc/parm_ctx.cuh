@@ -110,6 +110,14 @@ struct DevCtx {
     // neighbour list
     uint32_t* nbr;
     uint32_t* nnb;
+    // FP64 path: each listed pair's force, computed once for its first atom (the
+    // one of higher rank) in slot half_base[first] + entry; null: not kept
+    // (pair64.cu).  A system's slots start at atom_off * maxnb / 2.
+    void* pairf;
+    uint32_t* half_n;     // entries of each list with smaller ranks (the pairs of the atom as first)
+    uint32_t* half_base;  // slot of the first of them
+    uint32_t* half_cnt;   // per system: slots handed out at its last build
+    uint32_t* slots;      // [i * maxnb + k]: slot of entry k's pair where k >= half_n[i], or NO_SLOT
 
     // shared-memory tiles of the mixed-precision pair kernel: TILE_ATOMS
     // consecutive atoms of one system; entries are the tile's distinct
@@ -192,6 +200,7 @@ void launch_arm(const DevCtx& c, cudaStream_t s, int count_step, int use_cond,
 void launch_rebuild(const DevCtx& c, cudaStream_t s);
 void launch_check(const DevCtx& c, cudaStream_t s);
 void launch_tiles(const DevCtx& c, cudaStream_t s, int all);   // tiles of every system when all != 0
+void launch_half(const DevCtx& c, cudaStream_t s, int all);   // list sort and pair slots (every system when all != 0)
 void launch_numpairs(const DevCtx& c, cudaStream_t s);   // -> sysout[s] (as double)
 void launch_posq(const DevCtx& c, cudaStream_t s);
 void launch_reframe(const DevCtx& c, cudaStream_t s);
@@ -327,6 +336,7 @@ __device__ __forceinline__ void cell_coords(const SysConst& S, uint32_t b, uint3
 }
 
 constexpr int BLOCK = 256;
+constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
 constexpr uint32_t RED_CHUNK = 4096;   // atoms per reduction chunk
 constexpr int TILE_ATOMS = 64;
 constexpr int TILE_ECAP = 1024;

@@ -305,6 +305,9 @@ class System:
     def debug_stage_cap(self, cap: int) -> None:
         check(self.lib.parm_debug_stage_cap(self.h, int(cap)))
 
+    def debug_pair_slots(self, keep: int) -> None:
+        check(self.lib.parm_debug_pair_slots(self.h, int(keep)))
+
     def autotune(self) -> int:
         v = C.c_uint32()
         check(self.lib.parm_autotune(self.h, C.byref(v)))

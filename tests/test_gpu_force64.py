@@ -43,3 +43,33 @@ def test_repulsion_exponents(ndim, exponent, rel):
     o.set_forces(False)
     f, ref = g.get_atoms()["f"], o.get_state()["f"]
     assert np.abs(f - ref).max() <= rel * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("kind,ndim", [(0, 3), (1, 2), (2, 3), (3, 2)])
+def test_slots_and_both_sides_agree(kind, ndim):
+    """Pair forces kept once per pair, or evaluated for both atoms: the same bits, through rebuilds, on a ragged
+    batch whose systems rebuild at different steps (one of them frozen for a while)."""
+    ws = [W.small_random(n=n, ndim=ndim, kind=kind, seed=n, phi=0.3, skin=0.3) for n in (5, 61, 130, 311)]
+    w = W.Workload("b", ndim, [k.n for k in ws], np.concatenate([k.L for k in ws]), np.concatenate([k.x for k in ws]),
+                   np.concatenate([k.v for k in ws]), np.concatenate([k.m for k in ws]), kind,
+                   np.concatenate([k.params for k in ws]), 0.3)
+    rng = np.random.default_rng(kind)
+    rank = np.concatenate([rng.permutation(k.n) for k in ws]).astype(np.uint32)
+    out = []
+    for keep in (True, False):
+        g = make_gpu(w, rank=rank)
+        g.debug_pair_slots(keep)
+        g.nlist_update(False)
+        g.set_forces(True)
+        g.damped(1e-4, 5.0, 20)
+        g.set_active([1, 1, 0, 1])
+        g.damped(1e-4, 5.0, 40)
+        g.set_active([1, 1, 1, 1])
+        g.set_capacity(g.capacity() + 24)   # lists re-pitched between rebuilds
+        g.damped(1e-4, 5.0, 40)
+        g.nlist_update(True)
+        g.damped(1e-4, 5.0, 4)
+        out.append((g.get_atoms(), g.which()))
+    for k in ("x", "v", "a", "f"):
+        assert np.array_equal(out[0][0][k], out[1][0][k])
+    assert np.array_equal(out[0][1], out[1][1]) and out[0][1].min() > 1
