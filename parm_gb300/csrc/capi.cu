@@ -19,6 +19,7 @@
 #include <string>
 #include <vector>
 
+#include "noise.cuh"
 #include "parm_ctx.cuh"
 #include "parm_gb300.h"
 
@@ -1854,10 +1855,19 @@ int parm_sol(parm_system* S, double dt, double damping, double T, uint64_t seed,
     p.dtc12 = dt * (c1 - c2);
     p.dtc2 = dt * c2;
     p.T = T;
+    p.sqrt_T = std::sqrt(T);
     p.x11 = sigmar;
     p.x21 = sigmav * corr;
     p.x22 = sigmav * std::sqrt(1 - corr * corr);
     p.noise = damping > 0 ? 1 : 0;
+    if (!S->c.noise) {
+        NoiseTable* d = nullptr;
+        TRY(S->alloc(d, 1));
+        const NoiseTable t = noise_table();
+        CUDA_TRY(cudaMemcpyAsync(d, &t, sizeof(t), cudaMemcpyHostToDevice, S->st));
+        CUDA_TRY(cudaStreamSynchronize(S->st));
+        S->c.noise = d;
+    }
     std::vector<unsigned long long> seeds(S->nsys);
     for (uint32_t s = 0; s < S->nsys; s++) seeds[s] = splitmix64(seed + s);
     CUDA_TRY(cudaMemcpyAsync(S->c.seed, seeds.data(), 8 * S->nsys, cudaMemcpyHostToDevice, S->st));
@@ -2471,10 +2481,16 @@ int parm_debug_normals(uint64_t seed, uint32_t sys, uint64_t step, uint32_t nato
     if (!out) return fail(PARM_ERR_ARG, "NULL argument");
     if (natoms == 0) return PARM_OK;
     double* buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, 48 * (size_t)natoms));
-    launch_normals_test(splitmix64(seed + sys), step, natoms, buf, 0);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpy(out, buf, 48 * (size_t)natoms, cudaMemcpyDeviceToHost);
+    CUDA_TRY(cudaMalloc(&buf, sizeof(NoiseTable) + 48 * (size_t)natoms));
+    NoiseTable* dt = reinterpret_cast<NoiseTable*>(buf);
+    double* res = reinterpret_cast<double*>(dt + 1);
+    const NoiseTable t = noise_table();
+    cudaError_t e = cudaMemcpy(dt, &t, sizeof(t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        launch_normals_test(dt, splitmix64(seed + sys), step, natoms, res, 0);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, res, 48 * (size_t)natoms, cudaMemcpyDeviceToHost);
     cudaFree(buf);
     if (e != cudaSuccess) return fail(PARM_ERR_CUDA, cudaGetErrorString(e));
     return PARM_OK;

@@ -9,7 +9,7 @@
 //   CollectionSol::timestep     265-322  (first loop, BivariateGauss noise)
 // The second half of step k (a = f/m and the final velocity update) is fused
 // with the first half of step k+1 in k_kickdrift; a call ends with k_kick.
-#include "fpbits.cuh"
+#include "noise.cuh"
 #include "parm_check.cuh"
 
 namespace parm {
@@ -28,44 +28,6 @@ __device__ __forceinline__ void posq_split2(double x, float& X, float& xf) {
     double t = trunc(x * 8.0) * 0.125;
     X = (float)t;
     xf = (float)(x - t);
-}
-
-// ---- counter-based Gaussian noise (Philox4x32-10 + Box-Muller) ----
-__device__ __forceinline__ void philox10(uint32_t c[4], uint32_t k0, uint32_t k1) {
-#pragma unroll
-    for (int r = 0; r < 10; r++) {
-        uint32_t hi0 = __umulhi(0xD2511F53u, c[0]), lo0 = 0xD2511F53u * c[0];
-        uint32_t hi1 = __umulhi(0xCD9E8D57u, c[2]), lo1 = 0xCD9E8D57u * c[2];
-        uint32_t n0 = hi1 ^ c[1] ^ k0;
-        uint32_t n2 = hi0 ^ c[3] ^ k1;
-        c[0] = n0;
-        c[1] = lo1;
-        c[2] = n2;
-        c[3] = lo0;
-        k0 += 0x9E3779B9u;
-        k1 += 0xBB67AE85u;
-    }
-}
-
-__device__ __forceinline__ double u53(uint32_t a, uint32_t b) {
-    unsigned long long v = ((unsigned long long)(a >> 5) << 26) | (unsigned long long)(b >> 6);
-    return ((double)v + 0.5) * (1.0 / 9007199254740992.0);
-}
-
-__device__ __forceinline__ void normals6(unsigned long long seed, unsigned long long step,
-                                         uint32_t atom, double out[6]) {
-#pragma unroll
-    for (uint32_t blk = 0; blk < 3; blk++) {
-        uint32_t c[4] = {atom, (uint32_t)step, (uint32_t)(step >> 32), blk};
-        philox10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-        double u1 = u53(c[0], c[1]);
-        double u2 = u53(c[2], c[3]);
-        double r = sqrt(-2.0 * log(u1));
-        double sn, cs;
-        sincos(6.283185307179586 * u2, &sn, &cs);
-        out[2 * blk] = r * cs;
-        out[2 * blk + 1] = r * sn;
-    }
 }
 
 template <int ND>
@@ -210,16 +172,27 @@ __global__ void __launch_bounds__(BLOCK) k_kickdrift(DevCtx c) {
         } else {
             // CollectionSol: x += v*(c1*dt) + a*(c2*dt*dt) + drG*r0;
             //                v  = v*c0 + a*(dt*(c1-c2)) + dvG*v0
-            double v0 = sqrt(P.T / m);
-            double r0 = P.dt * v0;
+            // (sqrt(T / 1) == sqrt(T): formed once on the host)
+            const double v0 = __double_as_longlong(m) == 0x3FF0000000000000ll ? P.sqrt_T : sqrt(P.T / m);
+            const double r0 = P.dt * v0;
             double g[6] = {0, 0, 0, 0, 0, 0};
-            if (P.noise) normals6(c.seed[s], P.step, c.orig[i] - c.sys[s].atom_off, g);
+            if (P.noise) normals<ND>(c.noise, c.seed[s], P.step, c.orig[i] - c.sys[s].atom_off, g);
+            if constexpr (MIXED) {
+                // the same updates contracted into fused multiply-adds
+                const double gr = P.x11 * r0, gv1 = P.x21 * v0, gv2 = P.x22 * v0;
 #pragma unroll
-            for (int d = 0; d < ND; d++) {
-                double drG = g[d] * P.x11;
-                double dvG = g[d] * P.x21 + g[ND + d] * P.x22;
-                x[d] = x[d] + ((v[d] * P.c1dt + a[d] * P.c2dtdt) + drG * r0);
-                v[d] = (v[d] * P.c0 + a[d] * P.dtc12) + dvG * v0;
+                for (int d = 0; d < ND; d++) {
+                    x[d] = __fma_rn(v[d], P.c1dt, __fma_rn(a[d], P.c2dtdt, __fma_rn(g[d], gr, x[d])));
+                    v[d] = __fma_rn(v[d], P.c0, __fma_rn(a[d], P.dtc12, __fma_rn(g[d], gv1, g[ND + d] * gv2)));
+                }
+            } else {
+#pragma unroll
+                for (int d = 0; d < ND; d++) {
+                    double drG = g[d] * P.x11;
+                    double dvG = g[d] * P.x21 + g[ND + d] * P.x22;
+                    x[d] = x[d] + ((v[d] * P.c1dt + a[d] * P.c2dtdt) + drG * r0);
+                    v[d] = (v[d] * P.c0 + a[d] * P.dtc12) + dvG * v0;
+                }
             }
         }
         }
@@ -653,11 +626,12 @@ __global__ void k_philox_test(const uint32_t* in, uint32_t* out, uint32_t n) {
 }
 
 // the six normals the Langevin step draws for atoms 0..n-1 of a system keyed `key` at counter `step`
-__global__ void k_normals_test(unsigned long long key, unsigned long long step, uint32_t n, double* out) {
+__global__ void k_normals_test(const NoiseTable* t, unsigned long long key, unsigned long long step, uint32_t n,
+                               double* out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double g[6];
-    normals6(key, step, i, g);
+    normals<3>(t, key, step, i, g);
 #pragma unroll
     for (int q = 0; q < 6; q++) out[6 * (size_t)i + q] = g[q];
 }
@@ -678,9 +652,9 @@ void launch_philox_test(const uint32_t* in, uint32_t* out, uint32_t n, cudaStrea
     if (n) k_philox_test<<<grid_for(n), BLOCK, 0, s>>>(in, out, n);
 }
 
-void launch_normals_test(unsigned long long key, unsigned long long step, uint32_t n, double* out,
-                         cudaStream_t s) {
-    if (n) k_normals_test<<<grid_for(n), BLOCK, 0, s>>>(key, step, n, out);
+void launch_normals_test(const NoiseTable* t, unsigned long long key, unsigned long long step, uint32_t n,
+                         double* out, cudaStream_t s) {
+    if (n) k_normals_test<<<grid_for(n), BLOCK, 0, s>>>(t, key, step, n, out);
 }
 
 }  // namespace parm

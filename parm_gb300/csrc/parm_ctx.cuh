@@ -5,6 +5,8 @@
 
 namespace parm {
 
+struct NoiseTable;   // noise.cuh
+
 // integrator / evaluation modes of the pair-force kernels (the epilogue that
 // runs once an atom's force is complete)
 enum ForceMode : int {
@@ -27,6 +29,7 @@ struct StepParams {
     double dtc12;        // dt * (c1 - c2)
     double dtc2;         // dt * c2
     double T;            // desired temperature (CollectionSol)
+    double sqrt_T;
     double x11, x21, x22;// BivariateGauss::set outputs
     int noise;           // damping > 0 in CollectionSol
     int pad;
@@ -159,6 +162,7 @@ struct DevCtx {
     unsigned long long* top;  // [2*s] largest, [2*s+1] second largest squared displacement (bits)
     uint32_t* which;      // NeighborList::which()
     unsigned long long* seed;  // per-system Langevin key
+    const NoiseTable* noise;   // tables of the Langevin normals (null before the first parm_sol)
     uint32_t* status;
     uint32_t* any_flag;
     uint32_t* chains;     // rebuild-chain executions (for launch accounting)
@@ -258,8 +262,8 @@ void launch_remainder_test(const double* d, const double* L, double* out, uint32
 // test hooks of the Langevin generator (integrate.cu)
 void launch_philox_test(const uint32_t* in, uint32_t* out, uint32_t n, cudaStream_t s);
 void launch_fpbits_test(const double* d, const float* f, uint32_t n, float* d2f, double* f2d, cudaStream_t s);
-void launch_normals_test(unsigned long long key, unsigned long long step, uint32_t n, double* out,
-                         cudaStream_t s);
+void launch_normals_test(const NoiseTable* t, unsigned long long key, unsigned long long step, uint32_t n,
+                         double* out, cudaStream_t s);
 
 // what for launch_eval*: writes per-atom partials into c.red, ncomp per atom
 enum EvalWhat : int {
