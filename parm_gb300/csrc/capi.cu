@@ -128,7 +128,7 @@ struct parm_system {
     std::vector<uint32_t> rank_in;   // global order
     std::vector<std::set<uint32_t>> excl;
     bool have_excl = false, excl_dirty = false;
-    cudaStream_t st = nullptr, st2 = nullptr;
+    cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;   // st2, st3: captures of conditional bodies
     std::vector<void*> allocs;
     void* cell_mem = nullptr;
     void* nbr_mem = nullptr;
@@ -186,6 +186,7 @@ struct parm_system {
         if (hst) cudaFreeHost(hst);
         if (st) cudaStreamDestroy(st);
         if (st2) cudaStreamDestroy(st2);
+        if (st3) cudaStreamDestroy(st3);
     }
 
     void clear_graphs() {
@@ -615,31 +616,14 @@ struct parm_system {
     // pending by the last time step)
     int build_flush_graph(GraphEntry& ge) {
         CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        cudaStreamCaptureStatus cs;
-        cudaGraph_t g = nullptr;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t ndeps = 0;
-        CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &ndeps));
         cudaGraphConditionalHandle h;
-        CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+        TRY(cond_handle(st, h));
         launch_arm(c, st, 0, 1, (unsigned long long)h);
         CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &ndeps));
-        alignas(cudaGraphNodeParams) unsigned char cpbuf[sizeof(cudaGraphNodeParams)];
-        std::memset(cpbuf, 0, sizeof(cpbuf));
-        cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cpbuf);
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = h;
-        cp.conditional.type = cudaGraphCondTypeIf;
-        cp.conditional.size = 1;
-        cudaGraphNode_t node;
-        CUDA_TRY(cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &cp));
-        CUDA_TRY(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(st2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        launch_rebuild(c, st2);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamEndCapture(st2, &body));
+        TRY(cond_node(st, st2, h, cudaGraphCondTypeIf, [&](cudaStream_t q) {
+            launch_rebuild(c, q);
+            return PARM_OK;
+        }));
         CUDA_TRY(cudaStreamEndCapture(st, &ge.graph));
         CUDA_TRY(cudaGraphInstantiate(&ge.exec, ge.graph, 0));
         return PARM_OK;
@@ -695,35 +679,14 @@ struct parm_system {
         const int fmode = FM_FORCES;
         CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         for (uint32_t step = 0; step < k; step++) {
-            cudaStreamCaptureStatus cs;
-            cudaGraph_t g = nullptr;
-            const cudaGraphNode_t* deps = nullptr;
-            size_t ndeps = 0;
-            CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &ndeps));
             cudaGraphConditionalHandle h;
-            CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+            TRY(cond_handle(st, h));
             launch_arm(c, st, 1, 1, (unsigned long long)h);
             CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &ndeps));
-            // the struct's union has members without default constructors:
-            // build it in zeroed storage
-            alignas(cudaGraphNodeParams) unsigned char cpbuf[sizeof(cudaGraphNodeParams)];
-            std::memset(cpbuf, 0, sizeof(cpbuf));
-            cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cpbuf);
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = h;
-            cp.conditional.type = cudaGraphCondTypeIf;
-            cp.conditional.size = 1;
-            cudaGraphNode_t node;
-            CUDA_TRY(cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &cp));
-            CUDA_TRY(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1,
-                                                         cudaStreamSetCaptureDependencies));
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            CUDA_TRY(cudaStreamBeginCaptureToGraph(st2, body, nullptr, nullptr, 0,
-                                                   cudaStreamCaptureModeThreadLocal));
-            launch_rebuild(c, st2);
-            CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaStreamEndCapture(st2, &body));
+            TRY(cond_node(st, st2, h, cudaGraphCondTypeIf, [&](cudaStream_t q) {
+                launch_rebuild(c, q);
+                return PARM_OK;
+            }));
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step], st, cudaEventRecordExternal));
             launch_drift(c, st, dmode, step > 0);
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step + 1], st, cudaEventRecordExternal));
@@ -848,18 +811,21 @@ struct parm_system {
         if (prec == PREC_FP64) launch_eval64(cs, q, EV_VIRIAL);
         else launch_eval32(cs, q, EV_VIRIAL);
         launch_sys_reduce(cb, q, 1);
-        launch_nlcg_ctl(cb, q, NP_FL, 0, 0);
+        launch_nlcg_ctl(cb, q, NP_FL);
     }
 
-    // a conditional node (IF or WHILE on handle h) after the captured work
-    // of `q`; `emit` fills its body, captured on st2
+    // a conditional node (IF or WHILE on handle h) after the captured work of
+    // stream `q`; `emit` fills its body, captured on stream `inner`
     template <class F>
-    int nlcg_cond_node(cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, F&& emit) {
+    int cond_node(cudaStream_t q, cudaStream_t inner, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
+                  F&& emit) {
         cudaStreamCaptureStatus cs;
         cudaGraph_t g = nullptr;
         const cudaGraphNode_t* deps = nullptr;
         size_t ndeps = 0;
-        CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &ndeps));
+        CUDA_TRY(cudaStreamGetCaptureInfo(q, &cs, nullptr, &g, &deps, nullptr, &ndeps));
+        // the struct's union has members without default constructors: build
+        // it in zeroed storage
         alignas(cudaGraphNodeParams) unsigned char cpbuf[sizeof(cudaGraphNodeParams)];
         std::memset(cpbuf, 0, sizeof(cpbuf));
         cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cpbuf);
@@ -869,96 +835,95 @@ struct parm_system {
         cp.conditional.size = 1;
         cudaGraphNode_t node;
         CUDA_TRY(cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &cp));
-        CUDA_TRY(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
+        CUDA_TRY(cudaStreamUpdateCaptureDependencies(q, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
         cudaGraph_t body = cp.conditional.phGraph_out[0];
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(st2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        emit(st2);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(cudaStreamEndCapture(st2, &body));
+        CUDA_TRY(cudaStreamBeginCaptureToGraph(inner, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+        const int r = emit(inner);
+        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e2 = cudaStreamEndCapture(inner, &body);
+        if (r != PARM_OK) return r;
+        CUDA_TRY(e);
+        CUDA_TRY(e2);
         return PARM_OK;
     }
 
-    int nlcg_new_handle(cudaGraphConditionalHandle& h) {
+    int cond_handle(cudaStream_t q, cudaGraphConditionalHandle& h) {
         cudaStreamCaptureStatus cs;
         cudaGraph_t g = nullptr;
         const cudaGraphNode_t* deps = nullptr;
         size_t ndeps = 0;
-        CUDA_TRY(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, nullptr, &ndeps));
+        CUDA_TRY(cudaStreamGetCaptureInfo(q, &cs, nullptr, &g, &deps, nullptr, &ndeps));
         CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
         return PARM_OK;
     }
 
-    // the displacement test and, where it fires, the rebuild (update_trackers)
-    int nlcg_update_trackers(const DevCtx& cb, bool graph) {
-        launch_check(cb, st);
+    // stepx and, after it, the displacement test and, where it fires, the
+    // rebuild (update_trackers); on stream q, a rebuild's body captured on `inner`
+    int nlcg_step_track(const DevCtx& cb, cudaStream_t q, cudaStream_t inner, bool graph) {
         if (!graph) {
-            launch_arm(cb, st, 0, 0, 0);
-            launch_rebuild(cb, st);
+            launch_nlcg_stepx(cb, q, true, 0, 0);
+            launch_nlcg_box(cb, q);
+            launch_rebuild(cb, q);
             CUDA_TRY(cudaGetLastError());
             return PARM_OK;
         }
         cudaGraphConditionalHandle h;
-        TRY(nlcg_new_handle(h));
-        launch_arm(cb, st, 0, 1, (unsigned long long)h);
+        TRY(cond_handle(q, h));
+        launch_nlcg_stepx(cb, q, true, 1, (unsigned long long)h);
+        launch_nlcg_box(cb, q);
         CUDA_TRY(cudaGetLastError());
-        return nlcg_cond_node(h, cudaGraphCondTypeIf, [&](cudaStream_t q) { launch_rebuild(cb, q); });
+        return cond_node(q, inner, h, cudaGraphCondTypeIf, [&](cudaStream_t z) {
+            launch_rebuild(cb, z);
+            return PARM_OK;
+        });
     }
 
     // one secant iteration (collection.cpp:716-790, 1075-1131) on stream q
-    void nlcg_secant(const DevCtx& cb, const DevCtx& cs, cudaStream_t q, int use_cond, unsigned long long h) {
-        launch_nlcg_terms(cb, q, NT_FV, c.nlcg_loop);
-        launch_sys_reduce(cb, q, 1);
-        launch_nlcg_ctl(cb, q, NP_PRE, 0, 0);
-        launch_nlcg_stepx(cb, q);
-        launch_nlcg_box(cb, q);
-        if (!nlcg_boxed) {
+    int nlcg_secant(const DevCtx& cb, const DevCtx& cs, cudaStream_t q, cudaStream_t inner, bool graph,
+                    unsigned long long h) {
+        launch_nlcg_dot(cb, q, NT_FV, c.nlcg_loop, NP_SECANT, graph ? 1 : 0, h);
+        if (nlcg_boxed) {
+            launch_nlcg_stepx(cb, q, false, 0, 0);
+            launch_nlcg_box(cb, q);
+        } else {
             // CollectionNLCGV updates its trackers after every secant step
-            launch_check(cb, q);
-            launch_arm(cb, q, 0, 0, 0);
-            launch_rebuild(cb, q);
+            TRY(nlcg_step_track(cb, q, inner, graph));
         }
         nlcg_forces(cb, cs, q);
-        launch_nlcg_ctl(cb, q, NP_POST, use_cond, h);
+        return PARM_OK;
     }
 
     // CollectionNLCG::timestep / CollectionNLCGV::timestep for every active system
     int nlcg_emit_step(bool graph, uint32_t max_sec) {
         DevCtx cb, cs;
         nlcg_ctx(cb, cs);
-        launch_nlcg_ctl(cb, st, NP_BEGIN, 0, 0);
-        launch_nlcg_stepx(cb, st);
+        launch_nlcg_ctl(cb, st, NP_BEGIN);
+        launch_nlcg_stepx(cb, st, false, 0, 0);
         launch_nlcg_box(cb, st);
         nlcg_forces(cb, cs, st);
-        launch_nlcg_terms(cb, st, NT_FV, c.nlcg_step);
-        launch_sys_reduce(cb, st, 1);
-        launch_nlcg_ctl(cb, st, NP_ETA0, 0, 0);
-        launch_nlcg_stepx(cb, st);
-        launch_nlcg_box(cb, st);
-        TRY(nlcg_update_trackers(cb, graph));
+        launch_nlcg_dot(cb, st, NT_FV, c.nlcg_step, NP_ETA0, 0, 0);
+        TRY(nlcg_step_track(cb, st, st2, graph));
         nlcg_forces(cb, cs, st);
-        launch_nlcg_terms(cb, st, NT_VV, c.nlcg_step);
-        launch_sys_reduce(cb, st, 1);
         CUDA_TRY(cudaGetLastError());
         if (graph) {
             cudaGraphConditionalHandle h;
-            TRY(nlcg_new_handle(h));
-            launch_nlcg_ctl(cb, st, NP_LOOPINIT, 1, (unsigned long long)h);
+            TRY(cond_handle(st, h));
+            launch_nlcg_dot(cb, st, NT_VV, c.nlcg_step, NP_LOOPINIT, 1, (unsigned long long)h);
             CUDA_TRY(cudaGetLastError());
-            TRY(nlcg_cond_node(h, cudaGraphCondTypeWhile,
-                               [&](cudaStream_t q) { nlcg_secant(cb, cs, q, 1, (unsigned long long)h); }));
+            TRY(cond_node(st, st2, h, cudaGraphCondTypeWhile, [&](cudaStream_t q) {
+                return nlcg_secant(cb, cs, q, st3, true, (unsigned long long)h);
+            }));
         } else {
-            launch_nlcg_ctl(cb, st, NP_LOOPINIT, 0, 0);
+            launch_nlcg_dot(cb, st, NT_VV, c.nlcg_step, NP_LOOPINIT, 0, 0);
             for (uint32_t it = 0; it <= 2 * max_sec + 2; it++) {
                 CUDA_TRY(cudaMemcpyAsync(hst, c.nlcg_any, 4, cudaMemcpyDeviceToHost, st));
                 CUDA_TRY(cudaStreamSynchronize(st));
                 if (!hst[0]) break;
-                nlcg_secant(cb, cs, st, 0, 0);
+                TRY(nlcg_secant(cb, cs, st, nullptr, false, 0));
                 CUDA_TRY(cudaGetLastError());
             }
         }
-        launch_nlcg_terms(cb, st, NT_FA_FF, c.active);
-        launch_sys_reduce(cb, st, 2);
-        launch_nlcg_ctl(cb, st, NP_FINISH, 0, 0);
+        launch_nlcg_dot(cb, st, NT_FA_FF, c.active, NP_FINISH, 0, 0);
         launch_nlcg_atoms(cb, st, NA_FINISH);
         CUDA_TRY(cudaGetLastError());
         return PARM_OK;
@@ -1126,7 +1091,8 @@ int parm_create(parm_system** out, int ndim, uint32_t nsys, const uint32_t* nato
         return r;
     };
     if (cudaStreamCreateWithFlags(&S->st, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&S->st2, cudaStreamNonBlocking) != cudaSuccess)
+        cudaStreamCreateWithFlags(&S->st2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&S->st3, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(PARM_ERR_CUDA, "cudaStreamCreate failed"));
     DevCtx& c = S->c;
     c.nd = ndim;
@@ -1196,6 +1162,7 @@ int parm_create(parm_system** out, int ndim, uint32_t nsys, const uint32_t* nato
     A(S->alloc(c.m_mixed, 1));
     A(S->alloc(c.any_flag, 1));
     A(S->alloc(c.chains, 1));
+    A(S->alloc(c.done, 2 + (size_t)nsys));
     A(S->alloc(c.params, 1));
     A(S->alloc(c.sysout, (size_t)nsys * 16));
     if (precision == PARM_FP64) {
@@ -2302,7 +2269,7 @@ int parm_nlcg_init(parm_system* S, int boxed, const double* params) {
     TRY(S->flush());
     CUDA_TRY(cudaStreamSynchronize(S->st));
     if (!S->nlcg_mem) {
-        const size_t bytes = sizeof(NlcgSys) * (size_t)S->nsys + 8 * (size_t)S->nsys + 16;
+        const size_t bytes = sizeof(NlcgSys) * (size_t)S->nsys + 8 * (size_t)S->nsys + 16;   // nlcg_any: two words
         CUDA_TRY(cudaMalloc(&S->nlcg_mem, bytes));
         CUDA_TRY(cudaMemset(S->nlcg_mem, 0, bytes));
         char* b = static_cast<char*>(S->nlcg_mem);
@@ -2376,9 +2343,7 @@ static int nlcg_set_forces_impl(parm_system* S, bool c_and_a) {
     launch_nlcg_atoms(cb, S->st, NA_IMMOBILE_A);
     if (c_and_a) {
         launch_nlcg_atoms(cb, S->st, NA_SETF);
-        launch_nlcg_terms(cb, S->st, NT_FA_FF, S->c.active);
-        launch_sys_reduce(cb, S->st, 2);
-        launch_nlcg_ctl(cb, S->st, NP_SETF, 0, 0);
+        launch_nlcg_dot(cb, S->st, NT_FA_FF, S->c.active, NP_SETF, 0, 0);
     }
     CUDA_TRY(cudaGetLastError());
     return PARM_OK;
@@ -2400,10 +2365,10 @@ int parm_nlcg_reset(parm_system* S) {
         // CollectionNLCG::reset (collection.cpp:525-532)
         TRY(nlcg_set_forces_impl(S, true));
         launch_nlcg_atoms(cb, S->st, NA_RESET);
-        launch_nlcg_ctl(cb, S->st, NP_RESET, 0, 0);
+        launch_nlcg_ctl(cb, S->st, NP_RESET);
     } else {
         // CollectionNLCGV::reset (collection.cpp:977-988)
-        launch_nlcg_ctl(cb, S->st, NP_RESET, 0, 0);
+        launch_nlcg_ctl(cb, S->st, NP_RESET);
         TRY(nlcg_set_forces_impl(S, false));
         launch_nlcg_atoms(cb, S->st, NA_DESCEND);
     }
@@ -2419,10 +2384,8 @@ int parm_nlcg_descend(parm_system* S) {
     // descend (collection.cpp:811-829, 990-1005): forces, v = a = f, stepx(dt), trackers
     TRY(nlcg_set_forces_impl(S, false));
     launch_nlcg_atoms(cb, S->st, NA_DESCEND);
-    launch_nlcg_ctl(cb, S->st, NP_DESCEND, 0, 0);
-    launch_nlcg_stepx(cb, S->st);
-    launch_nlcg_box(cb, S->st);
-    TRY(S->nlcg_update_trackers(cb, false));
+    launch_nlcg_ctl(cb, S->st, NP_DESCEND);
+    TRY(S->nlcg_step_track(cb, S->st, nullptr, false));
     TRY(S->sync_status());
     return S->nlcg_sync_boxes();
 }

@@ -11,6 +11,7 @@
 // with the first half of step k+1 in k_kickdrift; a call ends with k_kick.
 #include "noise.cuh"
 #include "parm_check.cuh"
+#include "reduce.cuh"
 
 namespace parm {
 
@@ -466,30 +467,6 @@ void launch_reduce_atoms(const DevCtx& c, cudaStream_t s, int what, const double
 // consecutive atoms of one system is reduced by one CTA (fixed striding and
 // tree), then one CTA per system reduces its chunks in chunk order.  ncomp < 0
 // means a single-component maximum.
-template <int NT>
-__device__ __forceinline__ double block_reduce(double acc, bool is_max, double* sh) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const double o = __shfl_down_sync(0xFFFFFFFFu, acc, off);
-        acc = is_max ? fmax(acc, o) : acc + o;
-    }
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    double v = 0.0;
-    if (threadIdx.x < 32) {
-        v = threadIdx.x < NT / 32 ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const double o = __shfl_down_sync(0xFFFFFFFFu, v, off);
-            v = is_max ? fmax(v, o) : v + o;
-        }
-    }
-    __syncthreads();
-    return v;   // valid in thread 0
-}
-
-constexpr int RED_THREADS = 256;
-
 __global__ void __launch_bounds__(RED_THREADS) k_red_chunks(DevCtx c, int ncomp) {
     __shared__ double sh[32];
     const uint4 ch = c.chunk[blockIdx.x];   // (system, first atom, atoms, -)

@@ -6,18 +6,21 @@
 //     positions only, fixed box.
 // Every system keeps its own minimiser state (NlcgSys) in device memory and
 // runs its own secant line search; one launch of each kernel serves all
-// systems.  Per-system scalar decisions are taken by k_nlcg_ctl (one thread
-// per system); per-atom work by k_nlcg_stepx / k_nlcg_atoms / k_nlcg_terms;
-// the sums (fdotv, vdotv, fdota, the virial) by the deterministic two-pass
-// per-system reductions of integrate.cu.  The secant loop runs inside a CUDA
-// graph as a conditional WHILE node whose condition k_nlcg_ctl sets while any
-// system is still searching, so a time step needs no host round trip.
+// systems.  Per-atom work is done by k_nlcg_stepx / k_nlcg_atoms; the sums
+// fdotv, vdotv and fdota by k_nlcg_dot in fixed order, whose last block per
+// system takes that system's decisions with them (k_nlcg_ctl takes those that
+// need no such sum); the virial by the reductions of integrate.cu.  The secant
+// loop runs inside a CUDA graph as a conditional WHILE node whose condition
+// k_nlcg_dot sets while any system is still searching, and list rebuilds are
+// conditional IF nodes that k_nlcg_stepx arms, so a time step needs no host
+// round trip and an iteration without a rebuild is three kernels.
 //
 // Compiled with -fmad=false: the update formulas round like the reference's
 // unfused FP64 code.  The sums are parallel, so the scalars (and the
 // trajectories through them) agree with the reference to rounding, not bit
 // for bit.
-#include "parm_ctx.cuh"
+#include "parm_check.cuh"
+#include "reduce.cuh"
 
 namespace parm {
 
@@ -106,36 +109,59 @@ __device__ __forceinline__ double length_sq(const SysConst& S) {
 // set_forces_get_pressure, collection.cpp:181-208) zeroes the acceleration of
 // immobile atoms; that is done here as well.
 // ---------------------------------------------------------------------------
-template <int ND, bool BOXED>
-__global__ void __launch_bounds__(BLOCK) k_nlcg_stepx(DevCtx c) {
+// With TRACK, the displacement test of every member atom follows (update_list
+// after the step), and the last block arms the rebuild: with separate kernels
+// a minimiser step spent as much on their launches as on its forces.
+template <int ND, bool BOXED, bool TRACK>
+__global__ void __launch_bounds__(BLOCK) k_nlcg_stepx(DevCtx c, int use_cond, cudaGraphConditionalHandle handle) {
+    using V = typename DVec<ND>::T;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    const uint32_t s = c.atom_sys[i];
-    if (!c.nlcg_step[s]) return;
-    const NlcgSys& G = c.nlcg[s];
-    const double m = c.m[i];
-    double x[3] = {0, 0, 0}, v[3] = {0, 0, 0};
-    ld3<ND>(c.x, i, x);
-    ld3<ND>(c.v, i, v);
-    if (BOXED) {
-        const double lf = G.lfac, dx = G.dx;
+    const uint32_t s = i < c.n ? c.atom_sys[i] : 0u;
+    bool valid = false;
+    double dsq = 0.0;
+    if (i < c.n) {
+        const bool step = c.nlcg_step[s] != 0u;
+        double x[3] = {0, 0, 0};
+        if (step || TRACK) ld3<ND>(c.x, i, x);
+        if (step) {
+            const NlcgSys& G = c.nlcg[s];
+            const bool mob = mobile_cg(c.m[i]);
+            double v[3] = {0, 0, 0};
+            ld3<ND>(c.v, i, v);
+            if (BOXED) {
+                const double lf = G.lfac, dx = G.dx;
 #pragma unroll
-        for (int d = 0; d < ND; d++) {
-            x[d] = x[d] * lf;
-            x[d] = x[d] + v[d] * dx;
-        }
-        if (!mobile_cg(m)) {
-            const double z[3] = {0, 0, 0};
-            st3<ND>(c.a, i, z);
-        }
-    } else {
-        if (!mobile_cg(m)) return;
-        const double dx = G.dx;
+                for (int d = 0; d < ND; d++) {
+                    x[d] = x[d] * lf;
+                    x[d] = x[d] + v[d] * dx;
+                }
+                if (!mob) {
+                    const double z[3] = {0, 0, 0};
+                    st3<ND>(c.a, i, z);
+                }
+            } else if (mob) {
+                const double dx = G.dx;
 #pragma unroll
-        for (int d = 0; d < ND; d++) x[d] = x[d] + v[d] * dx;
+                for (int d = 0; d < ND; d++) x[d] = x[d] + v[d] * dx;
+            }
+            if (BOXED || mob) {
+                st3<ND>(c.x, i, x);
+                posq_store<ND>(c, i, x);
+            }
+        }
+        if (TRACK && c.rank[i] != NOT_MEMBER) {
+            V xv;
+            double* xp = reinterpret_cast<double*>(&xv);
+#pragma unroll
+            for (int d = 0; d < (int)(sizeof(V) / 8); d++) xp[d] = d < ND ? x[d] : 0.0;
+            dsq = disp_sq<ND>(xv, static_cast<const V*>(c.lastloc)[i]);
+            valid = !(dsq != dsq);
+        }
     }
-    st3<ND>(c.x, i, x);
-    posq_store<ND>(c, i, x);
+    if constexpr (TRACK) {
+        check_accumulate(c, s, valid, dsq);
+        if (last_block(&c.done[0], gridDim.x)) arm_systems(c, 0, use_cond, handle);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -184,40 +210,6 @@ __global__ void k_nlcg_box(DevCtx c) {
         // the current lists index atoms, not cells: they stay valid, and the
         // next rebuild (when the displacement test asks for one) bins on this grid
     }
-}
-
-// ---------------------------------------------------------------------------
-// per-atom inputs of the per-system sums (component-major in red), mobile
-// atoms of systems flagged in `mask` only:
-//   NT_FV    f . v       (fdotv)
-//   NT_VV    v . v       (vdotv)
-//   NT_FA_FF f . a, f . f (fdota before and after a = f)
-// ---------------------------------------------------------------------------
-template <int ND>
-__global__ void __launch_bounds__(BLOCK) k_nlcg_terms(DevCtx c, int what, const uint32_t* mask) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    const uint32_t s = c.atom_sys[i];
-    double t0 = 0.0, t1 = 0.0;
-    if (mask[s] && mobile_cg(c.m[i])) {
-        double f[3] = {0, 0, 0}, q[3] = {0, 0, 0};
-        if (what == NT_VV) {
-            ld3<ND>(c.v, i, q);
-            t0 = dot<ND>(q, q);
-        } else {
-            ldf<ND>(c, i, f);
-            if (what == NT_FV) {
-                ld3<ND>(c.v, i, q);
-                t0 = dot<ND>(f, q);
-            } else {
-                ld3<ND>(c.a, i, q);
-                t0 = dot<ND>(f, q);
-                t1 = dot<ND>(f, f);
-            }
-        }
-    }
-    c.red[i] = t0;
-    if (what == NT_FA_FF) c.red[(size_t)c.n + i] = t1;
 }
 
 // ---------------------------------------------------------------------------
@@ -276,182 +268,246 @@ __global__ void __launch_bounds__(BLOCK) k_nlcg_atoms(DevCtx c, int what) {
 }
 
 // ---------------------------------------------------------------------------
-// per-system decisions (one thread per system); sysout holds the sums of the
-// preceding reduction
+// decisions of one system (one thread); S0, S1: the sums they need.  Returns
+// whether the system goes on searching.
 // ---------------------------------------------------------------------------
 template <int ND, bool BOXED>
-__global__ void k_nlcg_ctl(DevCtx c, int phase, int use_cond, cudaGraphConditionalHandle handle) {
-    __shared__ int sany;
-    if (threadIdx.x == 0) sany = 0;
-    __syncthreads();
-    int any = 0;
+__device__ bool nlcg_decide(const DevCtx& c, uint32_t s, int phase, double S0, double S1) {
     const double kd = (double)ND;
-    for (uint32_t s = threadIdx.x; s < c.nsys; s += blockDim.x) {
-        NlcgSys& G = c.nlcg[s];
-        const SysConst& S = c.sys[s];
-        const bool act = c.active[s] != 0;
-        const double lsq = BOXED ? length_sq<ND>(S) : 1.0;
-        switch (phase) {
-            case NP_BEGIN:   // stepx(dt)
-                if (act) {
-                    G.dx = G.dt;
-                    G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
-                }
-                c.nlcg_step[s] = act ? 1u : 0u;
-                break;
-            case NP_FL:      // CollectionNLCG::set_forces(.., true), collection.cpp:536-541
-                if (BOXED && c.nlcg_step[s]) {
-                    const double interacP = c.sysout[s];
-                    G.fl = ((interacP / kd) - (G.P0 * box_volume<ND>(S))) / G.kappa;
-                }
-                break;
-            case NP_ETA0:    // eta0 = -fdotv() (collection.cpp:701); stepx(-dt) next
-                if (act) {
-                    const double fv = BOXED ? c.sysout[s] / lsq + G.fl * G.vl : c.sysout[s];
-                    G.eta0 = -fv;
-                    G.dx = -G.dt;
-                    G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
-                }
-                c.nlcg_step[s] = act ? 1u : 0u;
-                break;
-            case NP_LOOPINIT:   // collection.cpp:703-711
-                if (act) {
-                    G.vdv = BOXED ? c.sysout[s] / lsq + G.vl * G.vl : c.sysout[s];
-                    G.alpha = -G.dt;
-                    G.dxsum = 0.0;
-                    G.sec = 0.0;
-                    G.iters = 0.0;
-                }
-                c.nlcg_loop[s] = (act && G.secmax > 0.0) ? 1u : 0u;
-                c.nlcg_step[s] = 0u;
-                any |= c.nlcg_loop[s] ? 1 : 0;
-                break;
-            case NP_PRE: {   // collection.cpp:716-773 up to stepx(alpha)
-                c.nlcg_step[s] = 0u;
-                if (!c.nlcg_loop[s]) break;
-                const double fv = BOXED ? c.sysout[s] / lsq + G.fl * G.vl : c.sysout[s];
-                const double eta = -fv;
-                G.eta = eta;
-                double alphafac = -eta / fabs(G.eta0 - eta);
-                if (fabs(G.eta0 - eta) <= 1e-12 * fabs(eta)) {
-                    alphafac = G.alphamax > 0 ? G.alphamax : 1.1;
-                    G.sec = G.sec > 0 ? G.sec * 2 - 1 : 1;
-                }
-                if (G.alphamax > 0 && alphafac > G.alphamax) alphafac = G.alphamax;
-                if (G.alphamax > 0 && alphafac < -G.alphamax) alphafac = -G.alphamax;
-                G.alpha = fabs(G.alpha) * alphafac;
-                const double newdxsum = fabs(G.dxsum + G.alpha);
-                if (G.dxmax > 0 && newdxsum > G.dxmax) {
+    NlcgSys& G = c.nlcg[s];
+    const SysConst& S = c.sys[s];
+    const bool act = c.active[s] != 0;
+    const double lsq = BOXED ? length_sq<ND>(S) : 1.0;
+    switch (phase) {
+        case NP_BEGIN:   // stepx(dt)
+            if (act) {
+                G.dx = G.dt;
+                G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
+            }
+            c.nlcg_step[s] = act ? 1u : 0u;
+            break;
+        case NP_FL:      // CollectionNLCG::set_forces(.., true), collection.cpp:536-541
+            if (BOXED && c.nlcg_step[s]) {
+                const double interacP = S0;
+                G.fl = ((interacP / kd) - (G.P0 * box_volume<ND>(S))) / G.kappa;
+            }
+            break;
+        case NP_ETA0:    // eta0 = -fdotv() (collection.cpp:701); stepx(-dt) next
+            if (act) {
+                const double fv = BOXED ? S0 / lsq + G.fl * G.vl : S0;
+                G.eta0 = -fv;
+                G.dx = -G.dt;
+                G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
+            }
+            c.nlcg_step[s] = act ? 1u : 0u;
+            break;
+        case NP_LOOPINIT:   // collection.cpp:703-711
+            if (act) {
+                G.vdv = BOXED ? S0 / lsq + G.vl * G.vl : S0;
+                G.alpha = -G.dt;
+                G.dxsum = 0.0;
+                G.sec = 0.0;
+                G.iters = 0.0;
+            }
+            c.nlcg_loop[s] = (act && G.secmax > 0.0) ? 1u : 0u;
+            c.nlcg_step[s] = 0u;
+            return c.nlcg_loop[s] != 0u;
+        case NP_SECANT: {   // collection.cpp:716-790
+            c.nlcg_step[s] = 0u;
+            if (!c.nlcg_loop[s]) return false;
+            const double fv = BOXED ? S0 / lsq + G.fl * G.vl : S0;
+            const double eta = -fv;
+            G.eta = eta;
+            double alphafac = -eta / fabs(G.eta0 - eta);
+            if (fabs(G.eta0 - eta) <= 1e-12 * fabs(eta)) {
+                alphafac = G.alphamax > 0 ? G.alphamax : 1.1;
+                G.sec = G.sec > 0 ? G.sec * 2 - 1 : 1;
+            }
+            if (G.alphamax > 0 && alphafac > G.alphamax) alphafac = G.alphamax;
+            if (G.alphamax > 0 && alphafac < -G.alphamax) alphafac = -G.alphamax;
+            G.alpha = fabs(G.alpha) * alphafac;
+            const double newdxsum = fabs(G.dxsum + G.alpha);
+            if (G.dxmax > 0 && newdxsum > G.dxmax) {
+                G.k = 0;
+                c.nlcg_loop[s] = 0u;
+                return false;
+            }
+            if (BOXED) {
+                const double dVoverV = expm1(fabs(G.dxsum + G.alpha) * G.vl / (G.kappa * kd));
+                if (G.maxdV > 0 && dVoverV > G.maxdV) {
                     G.k = 0;
                     c.nlcg_loop[s] = 0u;
-                    break;
+                    return false;
                 }
-                if (BOXED) {
-                    const double dVoverV = expm1(fabs(G.dxsum + G.alpha) * G.vl / (G.kappa * kd));
-                    if (G.maxdV > 0 && dVoverV > G.maxdV) {
-                        G.k = 0;
-                        c.nlcg_loop[s] = 0u;
-                        break;
-                    }
-                }
-                G.dxsum += G.alpha;
-                G.dx = G.alpha;
-                G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
-                c.nlcg_step[s] = 1u;
-                break;
             }
-            case NP_POST:    // collection.cpp:774-790 and the loop increment
-                if (c.nlcg_step[s]) {
-                    G.eta0 = G.eta;
-                    bool brk = false;
-                    if (G.alpha * G.alpha * G.vdv < G.seceps * G.seceps) brk = true;
-                    else if ((G.sec > 1) && (G.afrac > 0) && (fabs(G.alpha) < fabs(G.dxsum)) &&
-                             (fabs(G.alpha) / fabs(G.dxsum) < G.afrac))
-                        brk = true;
-                    else if (G.stepmax > 0 && G.dxsum * G.dxsum * G.vdv > G.stepmax * G.stepmax) {
-                        G.k = 0;
-                        brk = true;
-                    }
-                    if (brk) {
-                        c.nlcg_loop[s] = 0u;
-                    } else {
-                        G.sec += 1;
-                        if (!(G.sec < G.secmax)) c.nlcg_loop[s] = 0u;
-                    }
-                    // sec grows by at least one per iteration, so the loop ends
-                    // within secmax iterations; the count bounds it regardless
-                    G.iters += 1;
-                    if (!(G.iters < G.secmax)) c.nlcg_loop[s] = 0u;
-                }
-                c.nlcg_step[s] = 0u;
-                any |= c.nlcg_loop[s] ? 1 : 0;
-                break;
-            case NP_FINISH:  // collection.cpp:792-809 (sysout: fdota before, after a = f)
-                if (act) {
-                    G.alphavmax = sqrt(G.alpha * G.alpha * G.vdv);
-                    const double Kold = G.Knew;
-                    const double Kmid = BOXED ? c.sysout[2 * s] / lsq + G.fl * G.al : c.sysout[2 * s];
-                    G.al = G.fl;
-                    G.Knew = BOXED ? c.sysout[2 * s + 1] / lsq + G.fl * G.al : c.sysout[2 * s + 1];
-                    G.beta = (G.Knew - Kmid) / Kold;
-                    G.betaused = G.beta;
-                    G.k += 1;
-                    if (G.k >= G.kmax || isinf(G.betaused) || isnan(G.betaused) || G.betaused <= 0) {
-                        G.k = 0;
-                        G.betaused = 0;
-                    } else if (G.betaused > 1) {
-                        G.betaused = 1;
-                    }
-                    if (BOXED) G.vl = G.al + G.betaused * G.vl;
-                }
-                break;
-            case NP_SETF:    // set_forces(true, true): al = vl = fl; Knew = fdota() with a = f
-                if (act) {
-                    if (BOXED) {
-                        G.al = G.fl;
-                        G.vl = G.fl;
-                    }
-                    G.Knew = BOXED ? c.sysout[2 * s + 1] / lsq + G.fl * G.al : c.sysout[2 * s + 1];
-                }
-                break;
-            case NP_RESET:   // reset(): k = 0 (and vl = al)
-                if (act) {
+            G.dxsum += G.alpha;
+            G.dx = G.alpha;
+            G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
+            c.nlcg_step[s] = 1u;
+            // the tests that follow the step and its forces need neither
+            // (collection.cpp:774-790 and the loop increment)
+            G.eta0 = G.eta;
+            bool brk = false;
+            if (G.alpha * G.alpha * G.vdv < G.seceps * G.seceps) brk = true;
+            else if ((G.sec > 1) && (G.afrac > 0) && (fabs(G.alpha) < fabs(G.dxsum)) &&
+                     (fabs(G.alpha) / fabs(G.dxsum) < G.afrac))
+                brk = true;
+            else if (G.stepmax > 0 && G.dxsum * G.dxsum * G.vdv > G.stepmax * G.stepmax) {
+                G.k = 0;
+                brk = true;
+            }
+            if (brk) {
+                c.nlcg_loop[s] = 0u;
+            } else {
+                G.sec += 1;
+                if (!(G.sec < G.secmax)) c.nlcg_loop[s] = 0u;
+            }
+            // sec grows by at least one per iteration, so the loop ends
+            // within secmax iterations; the count bounds it regardless
+            G.iters += 1;
+            if (!(G.iters < G.secmax)) c.nlcg_loop[s] = 0u;
+            return c.nlcg_loop[s] != 0u;
+        }
+        case NP_FINISH:  // collection.cpp:792-809 (the sums: fdota before, after a = f)
+            c.nlcg_step[s] = 0u;
+            if (act) {
+                G.alphavmax = sqrt(G.alpha * G.alpha * G.vdv);
+                const double Kold = G.Knew;
+                const double Kmid = BOXED ? S0 / lsq + G.fl * G.al : S0;
+                G.al = G.fl;
+                G.Knew = BOXED ? S1 / lsq + G.fl * G.al : S1;
+                G.beta = (G.Knew - Kmid) / Kold;
+                G.betaused = G.beta;
+                G.k += 1;
+                if (G.k >= G.kmax || isinf(G.betaused) || isnan(G.betaused) || G.betaused <= 0) {
                     G.k = 0;
-                    if (BOXED) G.vl = G.al;
+                    G.betaused = 0;
+                } else if (G.betaused > 1) {
+                    G.betaused = 1;
                 }
-                break;
-            case NP_DESCEND:  // descend(): al = vl = fl, then stepx(dt)
-                if (act) {
-                    if (BOXED) {
-                        G.al = G.fl;
-                        G.vl = G.fl;
-                    }
-                    G.dx = G.dt;
-                    G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
+                if (BOXED) G.vl = G.al + G.betaused * G.vl;
+            }
+            break;
+        case NP_SETF:    // set_forces(true, true): al = vl = fl; Knew = fdota() with a = f
+            if (act) {
+                if (BOXED) {
+                    G.al = G.fl;
+                    G.vl = G.fl;
                 }
-                c.nlcg_step[s] = act ? 1u : 0u;
-                break;
-            default:
-                break;
+                G.Knew = BOXED ? S1 / lsq + G.fl * G.al : S1;
+            }
+            break;
+        case NP_RESET:   // reset(): k = 0 (and vl = al)
+            if (act) {
+                G.k = 0;
+                if (BOXED) G.vl = G.al;
+            }
+            break;
+        case NP_DESCEND:  // descend(): al = vl = fl, then stepx(dt)
+            if (act) {
+                if (BOXED) {
+                    G.al = G.fl;
+                    G.vl = G.fl;
+                }
+                G.dx = G.dt;
+                G.lfac = BOXED ? exp(G.dx * G.vl / (G.kappa * kd)) : 1.0;
+            }
+            c.nlcg_step[s] = act ? 1u : 0u;
+            break;
+        default:
+            break;
+    }
+    return false;
+}
+
+// decisions that need no sum, or the virial's in sysout (NP_FL): one block
+template <int ND, bool BOXED>
+__global__ void k_nlcg_ctl(DevCtx c, int phase) {
+    for (uint32_t s = threadIdx.x; s < c.nsys; s += blockDim.x)
+        nlcg_decide<ND, BOXED>(c, s, phase, phase == NP_FL ? c.sysout[s] : 0.0, 0.0);
+}
+
+// ---------------------------------------------------------------------------
+// per-system sums over the mobile atoms of the systems flagged in `mask`:
+//   NT_FV    f . v       (fdotv)
+//   NT_VV    v . v       (vdotv)
+//   NT_FA_FF f . a, f . f (fdota before and after a = f)
+// One block per chunk of atoms, in the fixed order of the reductions of
+// integrate.cu; the last block of a system adds its chunks and takes its
+// decisions, and the last of all sets the secant loop's condition.  (Terms,
+// chunk sums, system sums and decisions as four kernels: 19 us a sum on 65,536
+// atoms, most of it launches.)
+// ---------------------------------------------------------------------------
+template <int ND, bool BOXED, int WHAT>
+__global__ void __launch_bounds__(RED_THREADS) k_nlcg_dot(DevCtx c, const uint32_t* mask, int phase, int use_cond,
+                                                          cudaGraphConditionalHandle handle) {
+    constexpr int NC = WHAT == NT_FA_FF ? 2 : 1;
+    __shared__ double sh[32];
+    const uint4 ch = c.chunk[blockIdx.x];   // (system, first atom, atoms, -)
+    const uint32_t s = ch.x;
+    double acc[2] = {0.0, 0.0};
+    if (mask[s]) {
+#pragma unroll 4
+        for (uint32_t k = threadIdx.x; k < ch.z; k += RED_THREADS) {
+            const uint32_t i = ch.y + k;
+            double t[2] = {0.0, 0.0}, f[3] = {0, 0, 0}, q[3] = {0, 0, 0};
+            if (mobile_cg(c.m[i])) {
+                if (WHAT == NT_VV) {
+                    ld3<ND>(c.v, i, q);
+                    t[0] = dot<ND>(q, q);
+                } else {
+                    ldf<ND>(c, i, f);
+                    ld3<ND>(WHAT == NT_FV ? c.v : c.a, i, q);
+                    t[0] = dot<ND>(f, q);
+                    if (WHAT == NT_FA_FF) t[1] = dot<ND>(f, f);
+                }
+            }
+#pragma unroll
+            for (int q2 = 0; q2 < NC; q2++) acc[q2] = acc[q2] + t[q2];
         }
     }
-    if (any) atomicOr(&sany, 1);
-    __syncthreads();
-    if (threadIdx.x == 0 && (phase == NP_LOOPINIT || phase == NP_POST)) {
-        *c.nlcg_any = (uint32_t)sany;
-        if (use_cond) cudaGraphSetConditional(handle, sany ? 1u : 0u);
+#pragma unroll
+    for (int q = 0; q < NC; q++) {
+        acc[q] = block_reduce<RED_THREADS>(acc[q], false, sh);
+        if (threadIdx.x == 0) c.part[(size_t)blockIdx.x * NC + q] = acc[q];
+    }
+    const uint32_t k0 = c.sys_chunk[s], k1 = c.sys_chunk[s + 1];
+    if (!last_block(&c.done[2 + s], k1 - k0)) return;
+    double sum[2] = {0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < NC; q++) {
+        double a = 0.0;
+        for (uint32_t k = k0 + threadIdx.x; k < k1; k += RED_THREADS) a = a + __ldcg(&c.part[(size_t)k * NC + q]);
+        sum[q] = block_reduce<RED_THREADS>(a, false, sh);
+    }
+    if (threadIdx.x != 0) return;
+    if (nlcg_decide<ND, BOXED>(c, s, phase, sum[0], sum[1])) atomicOr(&c.nlcg_any[1], 1u);
+    if (phase != NP_LOOPINIT && phase != NP_SECANT) return;
+    __threadfence();
+    if (atomicAdd(&c.done[1], 1u) + 1u == c.nsys) {   // every system has decided
+        atomicExch(&c.done[1], 0u);
+        const uint32_t any = atomicExch(&c.nlcg_any[1], 0u);
+        c.nlcg_any[0] = any;
+        if (use_cond) cudaGraphSetConditional(handle, any);
     }
 }
 
 // ---------------------------------------------------------------------------
-void launch_nlcg_stepx(const DevCtx& c, cudaStream_t s) {
+template <int ND, bool BOXED>
+static void stepx_nd(const DevCtx& c, cudaStream_t s, bool track, int use_cond, unsigned long long handle) {
     const unsigned g = grid_for(c.n);
+    const auto h = (cudaGraphConditionalHandle)handle;
+    if (track) k_nlcg_stepx<ND, BOXED, true><<<g, BLOCK, 0, s>>>(c, use_cond, h);
+    else k_nlcg_stepx<ND, BOXED, false><<<g, BLOCK, 0, s>>>(c, use_cond, h);
+}
+
+void launch_nlcg_stepx(const DevCtx& c, cudaStream_t s, bool track, int use_cond, unsigned long long handle) {
     if (c.nd == 3) {
-        if (c.nlcg_boxed) k_nlcg_stepx<3, true><<<g, BLOCK, 0, s>>>(c);
-        else k_nlcg_stepx<3, false><<<g, BLOCK, 0, s>>>(c);
+        if (c.nlcg_boxed) stepx_nd<3, true>(c, s, track, use_cond, handle);
+        else stepx_nd<3, false>(c, s, track, use_cond, handle);
     } else {
-        if (c.nlcg_boxed) k_nlcg_stepx<2, true><<<g, BLOCK, 0, s>>>(c);
-        else k_nlcg_stepx<2, false><<<g, BLOCK, 0, s>>>(c);
+        if (c.nlcg_boxed) stepx_nd<2, true>(c, s, track, use_cond, handle);
+        else stepx_nd<2, false>(c, s, track, use_cond, handle);
     }
 }
 
@@ -462,22 +518,35 @@ void launch_nlcg_box(const DevCtx& c, cudaStream_t s) {
     else k_nlcg_box<2><<<g, 128, 0, s>>>(c);
 }
 
-void launch_nlcg_ctl(const DevCtx& c, cudaStream_t s, int phase, int use_cond, unsigned long long handle) {
+void launch_nlcg_ctl(const DevCtx& c, cudaStream_t s, int phase) {
     const unsigned t = c.nsys >= 1024 ? 1024u : ((c.nsys + 31) / 32) * 32;
-    const auto h = (cudaGraphConditionalHandle)handle;
     if (c.nd == 3) {
-        if (c.nlcg_boxed) k_nlcg_ctl<3, true><<<1, t, 0, s>>>(c, phase, use_cond, h);
-        else k_nlcg_ctl<3, false><<<1, t, 0, s>>>(c, phase, use_cond, h);
+        if (c.nlcg_boxed) k_nlcg_ctl<3, true><<<1, t, 0, s>>>(c, phase);
+        else k_nlcg_ctl<3, false><<<1, t, 0, s>>>(c, phase);
     } else {
-        if (c.nlcg_boxed) k_nlcg_ctl<2, true><<<1, t, 0, s>>>(c, phase, use_cond, h);
-        else k_nlcg_ctl<2, false><<<1, t, 0, s>>>(c, phase, use_cond, h);
+        if (c.nlcg_boxed) k_nlcg_ctl<2, true><<<1, t, 0, s>>>(c, phase);
+        else k_nlcg_ctl<2, false><<<1, t, 0, s>>>(c, phase);
     }
 }
 
-void launch_nlcg_terms(const DevCtx& c, cudaStream_t s, int what, const uint32_t* mask) {
-    const unsigned g = grid_for(c.n);
-    if (c.nd == 3) k_nlcg_terms<3><<<g, BLOCK, 0, s>>>(c, what, mask);
-    else k_nlcg_terms<2><<<g, BLOCK, 0, s>>>(c, what, mask);
+template <int ND, bool BOXED>
+static void dot_nd(const DevCtx& c, cudaStream_t s, int what, const uint32_t* mask, int phase, int use_cond,
+                   cudaGraphConditionalHandle h) {
+    if (what == NT_FV) k_nlcg_dot<ND, BOXED, NT_FV><<<c.nchunk, RED_THREADS, 0, s>>>(c, mask, phase, use_cond, h);
+    else if (what == NT_VV) k_nlcg_dot<ND, BOXED, NT_VV><<<c.nchunk, RED_THREADS, 0, s>>>(c, mask, phase, use_cond, h);
+    else k_nlcg_dot<ND, BOXED, NT_FA_FF><<<c.nchunk, RED_THREADS, 0, s>>>(c, mask, phase, use_cond, h);
+}
+
+void launch_nlcg_dot(const DevCtx& c, cudaStream_t s, int what, const uint32_t* mask, int phase, int use_cond,
+                     unsigned long long handle) {
+    const auto h = (cudaGraphConditionalHandle)handle;
+    if (c.nd == 3) {
+        if (c.nlcg_boxed) dot_nd<3, true>(c, s, what, mask, phase, use_cond, h);
+        else dot_nd<3, false>(c, s, what, mask, phase, use_cond, h);
+    } else {
+        if (c.nlcg_boxed) dot_nd<2, true>(c, s, what, mask, phase, use_cond, h);
+        else dot_nd<2, false>(c, s, what, mask, phase, use_cond, h);
+    }
 }
 
 void launch_nlcg_atoms(const DevCtx& c, cudaStream_t s, int what) {

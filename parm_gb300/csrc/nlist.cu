@@ -34,39 +34,7 @@ __device__ __forceinline__ void posq_split(double x, float& X, float& xf) {
 // arm: decide, per system, whether this step starts with a rebuild
 // ---------------------------------------------------------------------------
 __global__ void k_arm(DevCtx c, int count_step, int use_cond, cudaGraphConditionalHandle handle) {
-    __shared__ int sany;
-    if (threadIdx.x == 0) sany = 0;
-    __syncthreads();
-    int any = 0;
-    for (uint32_t s = threadIdx.x; s < c.nsys; s += blockDim.x) {
-        if (count_step && !c.active[s]) {
-            // frozen system: no rebuild in time steps; its pending test
-            // (displacements, forced rebuild) waits until it is stepped again
-            c.flag[s] = 0u;
-            continue;
-        }
-        double t1 = __longlong_as_double((long long)c.top[2 * (size_t)s]);
-        double t2 = __longlong_as_double((long long)c.top[2 * (size_t)s + 1]);
-        // reference: bigdist + biggestdist >= skin, evaluated only once some atom moved
-        bool rb = c.force_rb[s] != 0u;
-        if (!rb && t1 > 0.0) rb = __dadd_rn(__dsqrt_rn(t2), __dsqrt_rn(t1)) >= c.sys[s].skin;
-        c.flag[s] = rb ? 1u : 0u;
-        if (rb) {
-            c.which[s] += 1u;
-            c.force_rb[s] = 0u;
-        }
-        c.top[2 * (size_t)s] = 0ull;
-        c.top[2 * (size_t)s + 1] = 0ull;
-        any |= rb ? 1 : 0;
-    }
-    if (any) atomicOr(&sany, 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *c.any_flag = (uint32_t)sany;
-        if (sany) *c.chains += 1u;
-        if (count_step) c.params->step += 1ull;
-        if (use_cond) cudaGraphSetConditional(handle, sany ? 1u : 0u);
-    }
+    arm_systems(c, count_step, use_cond, handle);
 }
 
 // ---------------------------------------------------------------------------

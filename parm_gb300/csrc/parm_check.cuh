@@ -92,6 +92,63 @@ __device__ __forceinline__ void check_accumulate(const DevCtx& c, uint32_t sys_i
     }
 }
 
+// Whether this block is the last of its grid to arrive at `counter` (every
+// thread of every block calls it, with its own writes done); the last block
+// sees the others' writes (through L2: __ldcg, atomics) and leaves the counter
+// at 0 for the next launch.
+__device__ __forceinline__ bool last_block(uint32_t* counter, uint32_t blocks) {
+    __shared__ uint32_t last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t k = atomicAdd(counter, 1u);
+        last = k + 1u == blocks ? 1u : 0u;
+        if (last) atomicExch(counter, 0u);
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0u;
+}
+
+// Arm (one block): decide, per system, whether a rebuild is due, from the
+// forced requests and the two largest displacements; counts the build and
+// clears what it consumed, and sets the conditional node's value.
+__device__ __forceinline__ void arm_systems(const DevCtx& c, int count_step, int use_cond,
+                                            cudaGraphConditionalHandle handle) {
+    __shared__ int sany;
+    if (threadIdx.x == 0) sany = 0;
+    __syncthreads();
+    int any = 0;
+    for (uint32_t s = threadIdx.x; s < c.nsys; s += blockDim.x) {
+        if (count_step && !c.active[s]) {
+            // frozen system: no rebuild in time steps; its pending test
+            // (displacements, forced rebuild) waits until it is stepped again
+            c.flag[s] = 0u;
+            continue;
+        }
+        const ulonglong2 top = __ldcg(reinterpret_cast<const ulonglong2*>(c.top) + s);
+        const double t1 = __longlong_as_double((long long)top.x), t2 = __longlong_as_double((long long)top.y);
+        // reference: bigdist + biggestdist >= skin, evaluated only once some atom moved
+        bool rb = c.force_rb[s] != 0u;
+        if (!rb && t1 > 0.0) rb = __dadd_rn(__dsqrt_rn(t2), __dsqrt_rn(t1)) >= c.sys[s].skin;
+        c.flag[s] = rb ? 1u : 0u;
+        if (rb) {
+            c.which[s] += 1u;
+            c.force_rb[s] = 0u;
+        }
+        reinterpret_cast<ulonglong2*>(c.top)[s] = make_ulonglong2(0ull, 0ull);
+        any |= rb ? 1 : 0;
+    }
+    if (any) atomicOr(&sany, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *c.any_flag = (uint32_t)sany;
+        if (sany) *c.chains += 1u;
+        if (count_step) c.params->step += 1ull;
+        if (use_cond) cudaGraphSetConditional(handle, sany ? 1u : 0u);
+    }
+}
+
 // squared displacement |x - lastloc|^2 in the reference's order
 // ((dx*dx + dy*dy) + dz*dz); FP64 without contraction (callers compile with
 // -fmad=false or use this routine, which uses explicit round-to-nearest ops)

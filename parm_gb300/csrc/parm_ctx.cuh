@@ -172,7 +172,8 @@ struct DevCtx {
     NlcgSys* nlcg;        // per system, or null before parm_nlcg_init
     uint32_t* nlcg_step;  // per system: moves in the current stepx (and is evaluated after it)
     uint32_t* nlcg_loop;  // per system: still in its secant loop
-    uint32_t* nlcg_any;   // [0]: some system is still in its secant loop
+    uint32_t* nlcg_any;   // [0]: some system is still in its secant loop; [1]: gathered while they decide
+    uint32_t* done;       // arrival counters, 0 between kernels: [0] blocks of a grid, [1] systems, [2 + s] chunks of system s
     uint32_t nlcg_boxed;  // CollectionNLCG (box scaled with kappa) rather than CollectionNLCGV
 
     // reduction scratch
@@ -230,8 +231,7 @@ enum NlcgPhase : int {
     NP_FL = 1,        // fl from the virial in sysout (boxed)
     NP_ETA0 = 2,      // eta0 = -fdotv; stepx(-dt) next
     NP_LOOPINIT = 3,  // vdv = vdotv; secant loop starts
-    NP_PRE = 4,       // secant iteration before its step
-    NP_POST = 5,      // secant iteration after its step
+    NP_SECANT = 4,    // secant iteration: the step to take, and whether another follows
     NP_FINISH = 6,    // Polak-Ribiere update of the direction's scalars
     NP_SETF = 7,      // end of set_forces(true, true): al = vl = fl, Knew
     NP_RESET = 8,     // end of reset(): vl = al, k = 0
@@ -245,10 +245,15 @@ enum NlcgAtoms : int {
     NA_DESCEND = 3,   // descend(): v = a = f (mobile)
     NA_IMMOBILE_A = 4 // immobile atoms: a = 0 (Collection::set_forces_get_pressure)
 };
-void launch_nlcg_stepx(const DevCtx& c, cudaStream_t s);
+// stepx; with `track`, NeighborList::update_list's displacement test and the arm
+// step after it (which sets the conditional node `handle` when use_cond)
+void launch_nlcg_stepx(const DevCtx& c, cudaStream_t s, bool track, int use_cond, unsigned long long handle);
 void launch_nlcg_box(const DevCtx& c, cudaStream_t s);
-void launch_nlcg_ctl(const DevCtx& c, cudaStream_t s, int phase, int use_cond, unsigned long long handle);
-void launch_nlcg_terms(const DevCtx& c, cudaStream_t s, int what, const uint32_t* mask);
+void launch_nlcg_ctl(const DevCtx& c, cudaStream_t s, int phase);
+// per-system sums of per-atom dot products over the systems flagged in `mask`,
+// then the decisions of `phase` with them
+void launch_nlcg_dot(const DevCtx& c, cudaStream_t s, int what, const uint32_t* mask, int phase, int use_cond,
+                     unsigned long long handle);
 void launch_nlcg_atoms(const DevCtx& c, cudaStream_t s, int what);
 // staged.cu (mixed path, cell blocks)
 void launch_build_stg(const DevCtx& c, cudaStream_t s);
@@ -341,7 +346,9 @@ __device__ __forceinline__ void cell_coords(const SysConst& S, uint32_t b, uint3
 
 constexpr int BLOCK = 256;
 constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
-constexpr uint32_t RED_CHUNK = 4096;   // atoms per reduction chunk
+// atoms per reduction chunk: four per thread of a reducing block (16 of them left
+// 65,536 atoms on 16 blocks: 10.5 us a sum)
+constexpr uint32_t RED_CHUNK = 1024;
 constexpr int TILE_ATOMS = 64;
 constexpr int TILE_ECAP = 1024;
 constexpr int TILE_HASH = 4096;
