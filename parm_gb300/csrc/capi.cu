@@ -307,6 +307,11 @@ struct parm_system {
         for (uint32_t s2 = 0; s2 < nsys; s2++)
             for (int d = 0; d < nd; d++)
                 if (sys[s2].nc[d] < 3) c.any_wrap = 1;
+        // k_force64s (a thread per entry) for lists that leave a warp per list idle,
+        // from where its CTAs of 16 atoms fill the SMs (force kernel, a warp per
+        // list / a thread per entry: 16.4 / 17.4 us on 5003 spheres, 34.5 / 30.1 on
+        // 20,000, 54.8 / 42.9 on 65,536 disks, 290 / 179 on 48 WCA replicas)
+        c.short_lists = n >= 8192 && mean_list() <= 32.0 ? 1u : 0u;
         std::vector<int> newnc;
         for (uint32_t s2 = 0; s2 < nsys; s2++)
             for (int d = 0; d < 3; d++) newnc.push_back(sys[s2].nc[d]);
@@ -571,8 +576,9 @@ struct parm_system {
         return PARM_OK;
     }
 
-    uint32_t estimate_capacity(double density_factor = 1.0) const {
-        double worst = 8.0;
+    // list entries per atom at the current boxes, in the densest system
+    double mean_list(double density_factor = 1.0) const {
+        double worst = 0.0;
         for (uint32_t s = 0; s < nsys; s++) {
             const SysConst& S = sys[s];
             double V = S.L[0] * S.L[1] * (nd == 3 ? S.L[2] : 1.0);
@@ -581,7 +587,10 @@ struct parm_system {
             double vol = (nd == 3) ? 4.18879020478639 * rl * rl * rl : 3.14159265358979 * rl * rl;
             worst = std::max(worst, rho * vol);
         }
-        double est = 1.6 * worst + 24.0;
+        return worst;
+    }
+    uint32_t estimate_capacity(double density_factor = 1.0) const {
+        double est = 1.6 * std::max(8.0, mean_list(density_factor)) + 24.0;
         if (est > 4096.0) est = 4096.0;
         return (uint32_t)std::ceil(est);
     }

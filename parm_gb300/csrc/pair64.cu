@@ -703,6 +703,121 @@ template <int ND, int KIND, int MODE>
 __global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
     forces64<ND, KIND, MODE, false>(c);
 }
+
+// k_force64 for short lists (a warp per atom would leave most lanes idle in
+// the screen, and eight atoms too few survivors for a warp): F64S_ATOMS atoms
+// a CTA, their entries numbered consecutively and screened one per thread, the
+// survivors evaluated one per thread in any order, each force stored at its
+// entry's place, and every entry added in order, zeros included.
+// FP64-bound from there (a soft-sphere pair takes ~55 FP64 operations): 54.8 ->
+// 42.9 us on 65,536 harmonic disks, 290 -> 179 us on 48 WCA replicas (~330,000
+// atoms).
+constexpr int F64S_THREADS = 128;
+constexpr uint32_t F64S_ATOMS = 16, F64S_CHUNK = 32;   // entries per atom and round
+constexpr uint32_t F64S_CAP = F64S_ATOMS * F64S_CHUNK;
+template <int ND, int KIND, int MODE>
+__global__ void __launch_bounds__(F64S_THREADS) k_force64s(DevCtx c) {
+    __shared__ double pf[ND][F64S_CAP];                 // pair forces by entry
+    __shared__ uint32_t pj[F64S_CAP];                   // survivors: neighbour,
+    __shared__ uint16_t pe[F64S_CAP];                   // entry,
+    __shared__ uint8_t pa[F64S_CAP];                    // atom | 128 when the image needs the remainder
+    __shared__ double xs[F64S_ATOMS][4];
+    __shared__ uint32_t off[F64S_ATOMS + 1], nsurv;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    const uint32_t i0 = blockIdx.x * F64S_ATOMS;
+    const bool all_uni = (c.uniform & UNI_ALL) == UNI_ALL;
+    uint32_t nn = 0u, nmax = 0u;   // of atom i0 + lane, in every warp
+    {
+        const uint32_t i = i0 + lane;
+        const bool go = lane < F64S_ATOMS && i < c.n && c.active[c.atom_sys[i]] && c.rank[i] != NOT_MEMBER;
+        if (go) nn = c.nnb[i];
+        nmax = __reduce_max_sync(0xFFFFFFFFu, nn);
+        if (tid < F64S_ATOMS) {
+            double xi[3] = {0, 0, 0};
+            if (go) load3<ND>(c.x, i, xi);
+#pragma unroll
+            for (int d = 0; d < 3; d++) xs[lane][d] = xi[d];
+        }
+    }
+    constexpr uint32_t SUMS = F64S_ATOMS * ND;   // (atom, component) pairs, one per thread
+    const uint32_t sa = tid % F64S_ATOMS, sd = tid / F64S_ATOMS;
+    double fsum = 0.0;
+    PairC pc;
+    bool have = false;
+    for (uint32_t base = 0; base < nmax; base += F64S_CHUNK) {
+        if (tid < 32u) {
+            const uint32_t m = nn > base ? min(nn - base, F64S_CHUNK) : 0u;
+            uint32_t incl = m;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (uint32_t)o) incl += u;
+            }
+            if (lane < F64S_ATOMS) off[lane + 1] = incl;
+            if (lane == 0) off[0] = nsurv = 0u;
+        }
+        __syncthreads();
+        const uint32_t total = off[F64S_ATOMS];
+        for (uint32_t t0 = tid - lane; t0 < total; t0 += F64S_THREADS) {   // uniform in the warp
+            const uint32_t t = t0 + lane;
+            bool keep = false, wrap = true;
+            uint32_t a = 0u, j = 0u;
+            if (t < total) {
+#pragma unroll
+                for (uint32_t h = F64S_ATOMS / 2; h; h >>= 1)
+                    if (off[a + h] <= t) a += h;
+                const uint32_t i = i0 + a;
+                j = __ldg(c.nbr + (size_t)i * c.maxnb + base + (t - off[a]));
+                float4 Ai, Bi;
+                ld_pos(c.pos, i, Ai, Bi);
+                keep = screen64<ND, KIND>(c, c.sys[c.atom_sys[i]], Ai, Bi, c.prm32[i], j, wrap);
+                if (!keep) {
+#pragma unroll
+                    for (int d = 0; d < ND; d++) pf[d][t] = 0.0;
+                }
+            }
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, keep);
+            uint32_t q = 0u;
+            if (lane == 0 && mask) q = atomicAdd(&nsurv, (uint32_t)__popc(mask));
+            q = __shfl_sync(0xFFFFFFFFu, q, 0) + __popc(mask & ((1u << lane) - 1u));
+            if (keep) {
+                pj[q] = j;
+                pe[q] = (uint16_t)t;
+                pa[q] = (uint8_t)(a | (wrap ? 128u : 0u));
+            }
+        }
+        __syncthreads();
+        const uint32_t ns = nsurv;
+        for (uint32_t q = tid; q < ns; q += F64S_THREADS) {
+            const uint32_t a = pa[q] & 127u, i = i0 + a, j = pj[q];
+            if (!all_uni || !have) {
+                pc = pair_constants<KIND>(c, i, j, c.rank[i] > c.rank[j]);
+                have = true;
+            }
+            double fo[3];
+            force_of_pair<ND, KIND>(c, c.sys[c.atom_sys[i]], i, j, xs[a], (pa[q] & 128u) != 0u, pc, fo);
+#pragma unroll
+            for (int d = 0; d < ND; d++) pf[d][pe[q]] = fo[d];
+        }
+        __syncthreads();
+        if (tid < SUMS) {
+            const uint32_t hi = off[sa + 1];
+#pragma unroll 4
+            for (uint32_t t = off[sa]; t < hi; t++) fsum = fsum + pf[sd][t];
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+    // the components of an atom meet in shared memory
+    if (tid < SUMS) pf[sd][sa] = fsum;
+    __syncthreads();
+    const uint32_t i = i0 + tid;
+    if (tid >= F64S_ATOMS || i >= c.n || !c.active[c.atom_sys[i]]) return;
+    double f[3] = {0, 0, 0};
+#pragma unroll
+    for (int d = 0; d < ND; d++) f[d] = pf[d][tid];
+    store_force<ND, MODE>(c, i, f);
+}
 template <int ND, int KIND>
 __global__ void __launch_bounds__(F64_THREADS) k_pair64(DevCtx c) {
     forces64<ND, KIND, FM_FORCES, true>(c);
@@ -876,6 +991,12 @@ static void force64_nd_kind(const DevCtx& c, cudaStream_t s, int mode) {
         const unsigned gs = grid_for(c.n, (int)(SUM64_WARPS * sum64_atoms<ND>()));
         if (mode == FM_FORCES_A) k_sum64<ND, FM_FORCES_A><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
         else k_sum64<ND, FM_FORCES><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
+        return;
+    }
+    if (c.short_lists) {
+        const unsigned gs = grid_for(c.n, F64S_ATOMS);
+        if (mode == FM_FORCES_A) k_force64s<ND, KIND, FM_FORCES_A><<<gs, F64S_THREADS, 0, s>>>(c);
+        else k_force64s<ND, KIND, FM_FORCES><<<gs, F64S_THREADS, 0, s>>>(c);
         return;
     }
     if (mode == FM_FORCES_A) k_force64<ND, KIND, FM_FORCES_A><<<g, F64_THREADS, 0, s>>>(c);

@@ -73,3 +73,30 @@ def test_slots_and_both_sides_agree(kind, ndim):
     for k in ("x", "v", "a", "f"):
         assert np.array_equal(out[0][0][k], out[1][0][k])
     assert np.array_equal(out[0][1], out[1][1]) and out[0][1].min() > 1
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 34, 64, 65, 66, 97, 130])
+def test_cluster_in_a_large_box(n, ndim):
+    """The kernel for short lists (chosen by the mean list and the atom count) on lists that are not: every atom of a
+    small cluster in each list, one round of the kernel and more; a second system of lone atoms makes up the count."""
+    w = W.small_random(n=n, ndim=ndim, kind=1, seed=n, phi=0.6, skin=30.0)
+    w.L[:] = 400.0
+    o = make_oracle(w)
+    lone = 8192
+    gap = 40.0   # beyond every list
+    k = 21 if ndim == 3 else 91
+    x = (np.stack(np.meshgrid(*[np.arange(k)] * ndim, indexing="ij"), -1).reshape(-1, ndim)[:lone] + 0.5) * gap
+    g = make_gpu(W.Workload("c", ndim, [n, lone], np.array([[400.0] * ndim, [k * gap] * ndim]),
+                            np.concatenate([w.x, x]), np.zeros((n + lone, ndim)),
+                            np.concatenate([w.m, np.ones(lone)]), 1,
+                            np.concatenate([w.params, np.tile(w.params[:1], (lone, 1))]), 30.0))
+    g.set_capacity(n)
+    g.nlist_update(True)
+    o.nl_update(True)
+    assert g.numpairs()[0] == n * (n - 1) // 2
+    g.set_forces(True)
+    o.set_forces(True)
+    st, ref = g.get_atoms(), o.get_state()
+    assert np.array_equal(st["f"][:n], ref["f"]) and not st["f"][n:].any()
+    assert np.array_equal(st["a"][:n], ref["a"])
