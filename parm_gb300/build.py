@@ -39,6 +39,7 @@ CUDA_UNITS = {
     "pair64.cu": ["-fmad=false"],
     "pair32.cu": [],
     "staged.cu": [],
+    "staged_eval.cu": [],
     "capi.cu": ["-fmad=false"],
     "noalloc.cu": ["-fmad=false"],
     "nlcg.cu": ["-fmad=false"],

@@ -384,6 +384,7 @@ struct parm_system {
             return PARM_OK;
         }
         std::vector<uint4> bl;
+        std::vector<uint32_t> first(1, 0u);   // first block of each system
         double worst = 0.0;
         bool ok = true;
         const double margin = 2.0 * skin + 1.0;
@@ -415,6 +416,7 @@ struct parm_system {
                         const uint32_t y0 = (uint32_t)(by * S.nc[1] / nby), y1 = (uint32_t)((by + 1) * S.nc[1] / nby);
                         bl.push_back(make_uint4(s, x0 | (x1 << 16), y0 | (y1 << 16), (uint32_t)z));
                     }
+            first.push_back((uint32_t)bl.size());
         }
         if (!ok || worst > 20000.0 || bl.empty()) {
             c.staged = 0;
@@ -424,14 +426,26 @@ struct parm_system {
         blk_mem = nullptr;
         if (tab_mem) cudaFree(tab_mem);
         tab_mem = nullptr;
-        CUDA_TRY(cudaMalloc(&blk_mem, sizeof(uint4) * bl.size()));
-        CUDA_TRY(cudaMemcpy(blk_mem, bl.data(), sizeof(uint4) * bl.size(), cudaMemcpyHostToDevice));
+        // blocks, their partial sums (9 doubles each), the systems' first blocks
+        const size_t nb = bl.size();
+        CUDA_TRY(cudaMalloc(&blk_mem, (sizeof(uint4) + 72) * nb + 4 * first.size()));
+        CUDA_TRY(cudaMemcpy(blk_mem, bl.data(), sizeof(uint4) * nb, cudaMemcpyHostToDevice));
+        c.blk_part = reinterpret_cast<double*>(static_cast<uint4*>(blk_mem) + nb);
+        uint32_t* dfirst = reinterpret_cast<uint32_t*>(c.blk_part + 9 * nb);
+        CUDA_TRY(cudaMemcpy(dfirst, first.data(), 4 * first.size(), cudaMemcpyHostToDevice));
+        c.sys_blk = dfirst;
         CUDA_TRY(cudaMalloc(&tab_mem, (size_t)16 * STG_TAB_WORDS * bl.size()));
         c.blk = static_cast<const uint4*>(blk_mem);
         c.stg_tab = static_cast<float4*>(tab_mem);
         c.nblk = (uint32_t)bl.size();
+        // staged atoms per block: half above the mean neighbourhood (a lattice's
+        // planes can fall unevenly into the cells); the evaluation stages a fifth
+        // above it and reads the rest of a larger one from global memory, so that
+        // four of its blocks share an SM
         c.stg_cap = (uint32_t)std::min(4096.0, std::ceil((1.5 * worst + 64.0) / 32.0) * 32.0);
-        if (stage_cap_override) c.stg_cap = stage_cap_override;
+        c.stg_cap_eval = (uint32_t)std::min(4096.0, std::ceil((1.2 * worst + 96.0) / 32.0) * 32.0);
+        c.stg_cap_eval = std::min(c.stg_cap, c.stg_cap_eval);
+        if (stage_cap_override) c.stg_cap = c.stg_cap_eval = stage_cap_override;
         const bool uni_eps = c.uniform & UNI_EPS, uni_sig = c.uniform & UNI_SIG, uni_th = c.uniform & UNI_THIRD;
         c.stg_prm = (uni_eps && uni_sig && uni_th) ? 0u : ((uni_eps && uni_th) ? 1u : 2u);
         c.stg_dia = (uni_sig && (kind != PARM_LJCUT || uni_th)) ? 0u : 1u;
@@ -1025,8 +1039,11 @@ struct parm_system {
         return (!c.staged && c.ntile && c.tiled) ? 11 : 10;
     }
 
-    int reduce_sys(int ncomp, std::vector<double>& out) {
-        launch_sys_reduce(c, st, ncomp);
+    // sums of what was launched last: per-atom values in red (or, with
+    // `blocks`, the cell blocks' partial sums)
+    int reduce_sys(int ncomp, std::vector<double>& out, bool blocks = false) {
+        if (blocks) launch_blk_reduce(c, st, ncomp);
+        else launch_sys_reduce(c, st, ncomp);
         CUDA_TRY(cudaGetLastError());
         int nc = ncomp < 0 ? 1 : ncomp;
         out.resize((size_t)nsys * nc);
@@ -1677,10 +1694,11 @@ int parm_nlist_which(parm_system* S, uint32_t* which) {
 int parm_nlist_numpairs(parm_system* S, uint64_t* numpairs) {
     if (!S || !numpairs) return fail(PARM_ERR_ARG, "NULL argument");
     TRY(S->flush());
-    TRY(S->rowmajor());
-    launch_numpairs(S->c, S->st);
+    const bool blocks = S->c.staged != 0;
+    if (blocks) launch_eval_stg(S->c, S->st, EV_PAIRS);
+    else launch_numpairs(S->c, S->st);
     std::vector<double> out;
-    TRY(S->reduce_sys(1, out));
+    TRY(S->reduce_sys(1, out, blocks));
     for (uint32_t s = 0; s < S->nsys; s++) numpairs[s] = (uint64_t)(out[s] + 0.5);
     return PARM_OK;
 }
@@ -1744,14 +1762,13 @@ int parm_evaluate(parm_system* S, int what, double* out) {
         std::fill(out, out + (size_t)S->nsys * ncomp, 0.0);
         return PARM_OK;
     }
+    const bool blocks = S->prec == PREC_MIXED && S->c.staged;
     if (S->prec == PREC_FP64) launch_eval64(S->c, S->st, what);
-    else {
-        TRY(S->rowmajor());
-        launch_eval32(S->c, S->st, what);
-    }
+    else if (blocks) launch_eval_stg(S->c, S->st, what);
+    else launch_eval32(S->c, S->st, what);
     CUDA_TRY(cudaGetLastError());
     std::vector<double> v;
-    TRY(S->reduce_sys(ncomp, v));
+    TRY(S->reduce_sys(ncomp, v, blocks));
     std::copy(v.begin(), v.end(), out);
     return PARM_OK;
 }

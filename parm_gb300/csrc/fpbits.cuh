@@ -76,6 +76,16 @@ PARM_FPB_HD double f2d_bits(float f) {
     return (double)f;
 }
 
+// (double)f without a branch (a compiler that turns f2d_bits' rare case into a
+// predicated conversion pays its FP64 slot every time): subnormals, below
+// 1.2e-38, become zero; infinities and NaN stay
+PARM_FPB_HD double f2d_flush(float f) {
+    const uint32_t b = fpb_f2u(f);
+    const uint32_t e = (b >> 23) & 0xFFu;
+    const uint32_t hi = ((e == 255u ? 2047u : e + 896u) << 20) | ((b & 0x7FFFFFu) >> 3);
+    return fpb_hilo2d((b & 0x80000000u) | (e ? hi : 0u), e ? b << 29 : 0u);
+}
+
 // (float)d: a double whose float result is normal keeps its top 23 fraction
 // bits, rounded to nearest (ties to even) on the 29 dropped ones; a carry out
 // of the fraction moves into the exponent, as the rounding requires

@@ -484,16 +484,18 @@ __global__ void __launch_bounds__(RED_THREADS) k_red_chunks(DevCtx c, int ncomp)
     }
 }
 
-__global__ void __launch_bounds__(RED_THREADS) k_sys_reduce(DevCtx c, int ncomp) {
+// part: ncomp values per chunk, system s's chunks from first[s] to first[s + 1]
+__global__ void __launch_bounds__(RED_THREADS) k_sys_reduce(DevCtx c, int ncomp, const double* part,
+                                                            const uint32_t* first) {
     __shared__ double sh[32];
     const uint32_t s = blockIdx.x;
     const bool is_max = ncomp < 0;
     const int nc = is_max ? 1 : ncomp;
-    const uint32_t k0 = c.sys_chunk[s], k1 = c.sys_chunk[s + 1];
+    const uint32_t k0 = first[s], k1 = first[s + 1];
     for (int comp = 0; comp < nc; comp++) {
         double acc = 0.0;
         for (uint32_t k = k0 + threadIdx.x; k < k1; k += RED_THREADS) {
-            const double v = c.part[(size_t)k * nc + comp];
+            const double v = part[(size_t)k * nc + comp];
             acc = is_max ? fmax(acc, v) : acc + v;
         }
         acc = block_reduce<RED_THREADS>(acc, is_max, sh);
@@ -503,7 +505,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_sys_reduce(DevCtx c, int ncomp)
 
 void launch_sys_reduce(const DevCtx& c, cudaStream_t s, int ncomp) {
     k_red_chunks<<<c.nchunk, RED_THREADS, 0, s>>>(c, ncomp);
-    k_sys_reduce<<<c.nsys, RED_THREADS, 0, s>>>(c, ncomp);
+    k_sys_reduce<<<c.nsys, RED_THREADS, 0, s>>>(c, ncomp, c.part, c.sys_chunk);
+}
+
+void launch_blk_reduce(const DevCtx& c, cudaStream_t s, int ncomp) {
+    k_sys_reduce<<<c.nsys, RED_THREADS, 0, s>>>(c, ncomp, c.blk_part, c.sys_blk);
 }
 
 // ---------------------------------------------------------------------------

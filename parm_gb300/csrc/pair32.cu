@@ -38,15 +38,6 @@ __device__ __noinline__ bool lj_beyond_exact(const DevCtx& c, const SysConst& S,
     return rsq > __dmul_rn(cut, cut);
 }
 
-template <int ND>
-__device__ __forceinline__ void disp3(const SysConst& S, const float4& Ai, const float4& Bi,
-                                      const float4& Aj, const float4& Bj, float* r) {
-    r[0] = disp32(Ai.x, Aj.x, Bi.x, Bj.x, S.Lhi[0], S.Llo[0], S.invLf[0]);
-    r[1] = disp32(Ai.y, Aj.y, Bi.y, Bj.y, S.Lhi[1], S.Llo[1], S.invLf[1]);
-    r[2] = 0.0f;
-    if constexpr (ND == 3) r[2] = disp32(Ai.z, Aj.z, Bi.z, Bj.z, S.Lhi[2], S.Llo[2], S.invLf[2]);
-}
-
 // TPA threads share one atom: lane `sub` of the group takes neighbours
 // sub, sub + TPA, ...; the partial forces are summed with shuffles.  The lists
 // are row-major and in cell order, so the TPA lanes of a group read one

@@ -141,9 +141,12 @@ struct DevCtx {
     uint32_t staged;      // use them (every system has >= 3 cells per axis)
     uint32_t nblk;        // blocks over all systems
     uint32_t stg_cap;     // atoms staged in shared memory per block
+    uint32_t stg_cap_eval;   // the same for the evaluation kernel
     uint32_t stg_prm;     // force kernel: 0 uniform parameters, 1 per-atom sigma, 2 all per atom
     uint32_t stg_dia;     // list build: per-atom list diameters
     const uint4* blk;     // per block: (system, x0 | x1 << 16, y0 | y1 << 16, z)
+    const uint32_t* sys_blk;   // first block of each system (nsys + 1)
+    double* blk_part;     // per block: partial sums of an evaluation (up to 9)
     float4* stg_tab;      // per block: its table (STG_TAB_WORDS 16-byte words), set by the list build
     uint16_t* nbr16;      // staged lists (layout in staged.cu)
     // per-atom cell-block records (mixed path): see make_record below
@@ -221,6 +224,7 @@ void launch_gather_out(const DevCtx& c, cudaStream_t s, double* staging, uint64_
 void launch_reduce_atoms(const DevCtx& c, cudaStream_t s, int what, const double* origin);
 void launch_rsq(const DevCtx& c, cudaStream_t s, int init);   // tracker start (init) or update
 void launch_sys_reduce(const DevCtx& c, cudaStream_t s, int ncomp);
+void launch_blk_reduce(const DevCtx& c, cudaStream_t s, int ncomp);   // blk_part -> sysout
 // pair64.cu / pair32.cu
 void launch_force64(const DevCtx& c, cudaStream_t s, int mode);
 void launch_force32(const DevCtx& c, cudaStream_t s, int mode);
@@ -259,8 +263,10 @@ void launch_nlcg_atoms(const DevCtx& c, cudaStream_t s, int what);
 // staged.cu (mixed path, cell blocks)
 void launch_build_stg(const DevCtx& c, cudaStream_t s);
 void launch_force_stg(const DevCtx& c, cudaStream_t s, int mode);
+void launch_eval_stg(const DevCtx& c, cudaStream_t s, int what);   // -> blk_part (EvalWhat)
 void launch_expand_stg(const DevCtx& c, cudaStream_t s);     // staged lists -> nbr (row-major)
 void launch_compress_stg(const DevCtx& c, cudaStream_t s);   // nbr (row-major) -> staged lists
+void eval_stg_set_smem_limits(size_t most);
 int stg_set_smem_limits();   // cudaError_t of raising the kernels' shared-memory limits
 // debug entry used by the tests of the minimum-image routine
 void launch_remainder_test(const double* d, const double* L, double* out, uint32_t n,
@@ -278,6 +284,7 @@ enum EvalWhat : int {
     EV_STRESS = 2,     // nd*nd comps
     EV_CONTACTS = 3,   // 1 comp (count E != 0)
     EV_OVERLAPS = 4,   // 1 comp (count E > 0)
+    EV_PAIRS = 5,      // 1 comp (listed pairs; cell-block kernels)
 };
 
 // what for launch_reduce_atoms

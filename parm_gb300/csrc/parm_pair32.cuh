@@ -15,6 +15,16 @@ namespace parm {
 // LJRepulsive forces vanish continuously at their cut-offs.)
 constexpr float CUT_BAND = 4e-6f;
 
+// minimum-image displacement from two position views
+template <int ND>
+__device__ __forceinline__ void disp3(const SysConst& S, const float4& Ai, const float4& Bi,
+                                      const float4& Aj, const float4& Bj, float* r) {
+    r[0] = disp32(Ai.x, Aj.x, Bi.x, Bj.x, S.Lhi[0], S.Llo[0], S.invLf[0]);
+    r[1] = disp32(Ai.y, Aj.y, Bi.y, Bj.y, S.Lhi[1], S.Llo[1], S.invLf[1]);
+    r[2] = 0.0f;
+    if constexpr (ND == 3) r[2] = disp32(Ai.z, Aj.z, Bi.z, Bj.z, S.Lhi[2], S.Llo[2], S.invLf[2]);
+}
+
 // FP32 pair law; returns the force scale s (F = r * s), 0 beyond the cut-off.
 // isig2 = 1/sigma_ij^2; e12 = 12*eps_ij (LJ kinds) or eps_ij (repulsion).
 template <int KIND>
