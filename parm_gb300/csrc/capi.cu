@@ -129,6 +129,7 @@ struct parm_system {
     std::vector<std::set<uint32_t>> excl;
     bool have_excl = false, excl_dirty = false;
     cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;   // st2, st3: captures of conditional bodies
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;   // branches of captured graphs
     std::vector<void*> allocs;
     void* cell_mem = nullptr;
     void* nbr_mem = nullptr;
@@ -187,6 +188,8 @@ struct parm_system {
         if (st) cudaStreamDestroy(st);
         if (st2) cudaStreamDestroy(st2);
         if (st3) cudaStreamDestroy(st3);
+        if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_join) cudaEventDestroy(ev_join);
     }
 
     void clear_graphs() {
@@ -388,35 +391,50 @@ struct parm_system {
         double worst = 0.0;
         bool ok = true;
         const double margin = 2.0 * skin + 1.0;
-        for (uint32_t s = 0; s < nsys && ok; s++) {
-            const SysConst& S = sys[s];
-            for (int d = 0; d < nd; d++)
-                if (S.nc[d] < 3) ok = false;
-            if (!ok) break;
-            const double a = std::max(1e-3, (double)natoms[s] / S.ncell);
-            // about 0.85 home atoms per thread: nearly every block still fits one
-            // pass of its threads, and few threads idle in the pair loop
-            const int cells = std::max(1, (int)std::lround(0.85 * STG_THREADS_HOST / a));
-            const int ky = std::max(1, std::min({(int)std::lround(std::sqrt(cells / 2.0)), STG_KY_MAX, S.nc[1] - 2}));
-            const int kx = std::max(1, std::min({(int)std::lround((double)cells / ky), STG_KX_MAX, S.nc[0] - 2}));
-            const int nbx = (S.nc[0] + kx - 1) / kx, nby = (S.nc[1] + ky - 1) / ky;
-            const double wx = std::ceil((double)S.nc[0] / nbx), wy = std::ceil((double)S.nc[1] / nby);
-            // extents in the block frames (length units): staged fields stay
-            // in [0, 3840) / [0, 768) (units of 1/8, bias 256 for the margin)
-            const double ex = S.L[0] + 2.0 * S.cellw[0] + margin;
-            const double ey = (wy + 2.0) * S.cellw[1] + margin;
-            const double ez = nd == 3 ? 3.0 * S.cellw[2] + margin : 0.0;
-            if (margin >= 30.0 || ex >= 440.0 || ey >= 60.0 || ez >= 60.0) ok = false;
-            worst = std::max(worst, a * (wx + 2) * (wy + 2) * (nd == 3 ? 3 : 1));
-            const int nzl = nd == 3 ? S.nc[2] : 1;
-            for (int z = 0; z < nzl; z++)
-                for (int by = 0; by < nby; by++)
-                    for (int bx = 0; bx < nbx; bx++) {
-                        const uint32_t x0 = (uint32_t)(bx * S.nc[0] / nbx), x1 = (uint32_t)((bx + 1) * S.nc[0] / nbx);
-                        const uint32_t y0 = (uint32_t)(by * S.nc[1] / nby), y1 = (uint32_t)((by + 1) * S.nc[1] / nby);
-                        bl.push_back(make_uint4(s, x0 | (x1 << 16), y0 | (y1 << 16), (uint32_t)z));
-                    }
-            first.push_back((uint32_t)bl.size());
+        // One thread per home atom, or (blocks of a quarter of the atoms, four
+        // threads each) where that leaves SMs without a block: in-graph forces
+        // with one / four threads 17.6 / 14.2 us at 4080 LJ atoms, 28.2 / 25.2 at
+        // 29,667 (137 blocks), 30.3 / 34.9 at 64,000; 14.6 / 12.5 us on 20,011
+        // disks.
+        int sms = 0, dev = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        for (uint32_t lg = 0; lg <= 2u && ok; lg += 2u) {
+            if (lg && bl.size() >= (size_t)sms) break;
+            c.stg_lg = lg;
+            bl.clear();
+            first.assign(1, 0u);
+            worst = 0.0;
+            for (uint32_t s = 0; s < nsys && ok; s++) {
+                const SysConst& S = sys[s];
+                for (int d = 0; d < nd; d++)
+                    if (S.nc[d] < 3) ok = false;
+                if (!ok) break;
+                const double a = std::max(1e-3, (double)natoms[s] / S.ncell);
+                // about 0.85 home atoms per thread: nearly every block still fits one
+                // pass of its threads, and few threads idle in the pair loop
+                const int cells = std::max(1, (int)std::lround(0.85 * (STG_THREADS_HOST >> c.stg_lg) / a));
+                const int ky = std::max(1, std::min({(int)std::lround(std::sqrt(cells / 2.0)), STG_KY_MAX, S.nc[1] - 2}));
+                const int kx = std::max(1, std::min({(int)std::lround((double)cells / ky), STG_KX_MAX, S.nc[0] - 2}));
+                const int nbx = (S.nc[0] + kx - 1) / kx, nby = (S.nc[1] + ky - 1) / ky;
+                const double wx = std::ceil((double)S.nc[0] / nbx), wy = std::ceil((double)S.nc[1] / nby);
+                // extents in the block frames (length units): staged fields stay
+                // in [0, 3840) / [0, 768) (units of 1/8, bias 256 for the margin)
+                const double ex = S.L[0] + 2.0 * S.cellw[0] + margin;
+                const double ey = (wy + 2.0) * S.cellw[1] + margin;
+                const double ez = nd == 3 ? 3.0 * S.cellw[2] + margin : 0.0;
+                if (margin >= 30.0 || ex >= 440.0 || ey >= 60.0 || ez >= 60.0) ok = false;
+                worst = std::max(worst, a * (wx + 2) * (wy + 2) * (nd == 3 ? 3 : 1));
+                const int nzl = nd == 3 ? S.nc[2] : 1;
+                for (int z = 0; z < nzl; z++)
+                    for (int by = 0; by < nby; by++)
+                        for (int bx = 0; bx < nbx; bx++) {
+                            const uint32_t x0 = (uint32_t)(bx * S.nc[0] / nbx), x1 = (uint32_t)((bx + 1) * S.nc[0] / nbx);
+                            const uint32_t y0 = (uint32_t)(by * S.nc[1] / nby), y1 = (uint32_t)((by + 1) * S.nc[1] / nby);
+                            bl.push_back(make_uint4(s, x0 | (x1 << 16), y0 | (y1 << 16), (uint32_t)z));
+                        }
+                first.push_back((uint32_t)bl.size());
+            }
         }
         if (!ok || worst > 20000.0 || bl.empty()) {
             c.staged = 0;
@@ -450,8 +468,6 @@ struct parm_system {
         c.stg_prm = (uni_eps && uni_sig && uni_th) ? 0u : ((uni_eps && uni_th) ? 1u : 2u);
         c.stg_dia = (uni_sig && (kind != PARM_LJCUT || uni_th)) ? 0u : 1u;
         static bool limits_set[256] = {};
-        int dev = 0;
-        CUDA_TRY(cudaGetDevice(&dev));
         if (dev >= 0 && dev < 256 && !limits_set[dev]) {
             const int e = stg_set_smem_limits();
             if (e != 0) return fail(PARM_ERR_CUDA, "raising the shared-memory limit of the cell-block kernels failed");
@@ -701,23 +717,36 @@ struct parm_system {
         const int dmode = mode == SM_VERLET ? DM_VERLET : (mode == SM_DAMPED ? DM_DAMPED : DM_SOL);
         const int fmode = FM_FORCES;
         CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        // Every step opens with its rebuild (IF node).  The first one is armed
+        // before it, the others beside the forces of the step before (they read
+        // nothing that the arm kernel writes), off the steps' critical path.
+        cudaGraphConditionalHandle h;
+        TRY(cond_handle(st, h));
+        launch_arm(c, st, 1, 1, (unsigned long long)h);
+        CUDA_TRY(cudaGetLastError());
         for (uint32_t step = 0; step < k; step++) {
-            cudaGraphConditionalHandle h;
-            TRY(cond_handle(st, h));
-            launch_arm(c, st, 1, 1, (unsigned long long)h);
-            CUDA_TRY(cudaGetLastError());
             TRY(cond_node(st, st2, h, cudaGraphCondTypeIf, [&](cudaStream_t q) {
                 launch_rebuild(c, q);
                 return PARM_OK;
             }));
+            const bool more = step + 1 < k;
+            if (more) TRY(cond_handle(st, h));
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step], st, cudaEventRecordExternal));
             launch_drift(c, st, dmode, step > 0);
+            if (more) {
+                CUDA_TRY(cudaEventRecord(ev_fork, st));
+                CUDA_TRY(cudaStreamWaitEvent(st3, ev_fork, 0));
+                launch_arm(c, st3, 1, 1, (unsigned long long)h);
+                CUDA_TRY(cudaGetLastError());
+                CUDA_TRY(cudaEventRecord(ev_join, st3));
+            }
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step + 1], st, cudaEventRecordExternal));
             if (prec == PREC_FP64) launch_force64(c, st, fmode);
             else launch_force32(c, st, fmode);
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step + 2], st, cudaEventRecordExternal));
             launch_rsq(c, st, 0);   // trackers, at the end of the step (positions final)
             CUDA_TRY(cudaGetLastError());
+            if (more) CUDA_TRY(cudaStreamWaitEvent(st, ev_join, 0));
         }
         launch_kick(c, st, dmode);   // second half of the chunk's last step
         CUDA_TRY(cudaGetLastError());
@@ -1118,7 +1147,9 @@ int parm_create(parm_system** out, int ndim, uint32_t nsys, const uint32_t* nato
     };
     if (cudaStreamCreateWithFlags(&S->st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&S->st2, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&S->st3, cudaStreamNonBlocking) != cudaSuccess)
+        cudaStreamCreateWithFlags(&S->st3, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&S->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&S->ev_join, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(PARM_ERR_CUDA, "cudaStreamCreate failed"));
     DevCtx& c = S->c;
     c.nd = ndim;

@@ -17,6 +17,12 @@ namespace parm {
 
 __device__ __forceinline__ bool mobile(double m) { return !(m <= 0.0 || isinf(m)); }
 
+// m == 0 or inf, on the bit pattern
+__device__ __forceinline__ bool zero_or_inf_bits(double m) {
+    const unsigned long long mag = (unsigned long long)__double_as_longlong(m) & 0x7FFFFFFFFFFFFFFFull;
+    return mag == 0ull || mag == 0x7FF0000000000000ull;
+}
+
 // the same test on the bit pattern (integer instructions, not the FP64 pipe):
 // NaN -> mobile; +-0, negative, +-inf -> not
 __device__ __forceinline__ bool mobile_bits(double m) {
@@ -44,28 +50,25 @@ __device__ __forceinline__ void store_posq(const DevCtx& c, uint32_t i, const do
 }
 
 // Second half of the previous step (the reference's loop after set_forces):
-// a = f/m and the final velocity update.  Mobility tests as in the reference:
-// Verlet and Damped skip m <= 0 or inf; Sol tests m == 0 or inf.
+// a = f/m and the final velocity update.  Mobility tests as in the reference: Verlet and Damped skip m <= 0
+// or inf; Sol tests m == 0 or inf.
 template <int ND, int MODE, bool MIXED>
 __device__ __forceinline__ void kick(const DevCtx& c, uint32_t i, double m, double* a, double* v) {
     const StepParams& P = *c.params;
     double f[3] = {0.0, 0.0, 0.0};
-    float fm[3] = {0.f, 0.f, 0.f};
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (MIXED) {
-        const float4 q = c.f32[i];
-        fm[0] = q.x;
-        fm[1] = q.y;
-        fm[2] = q.z;
+        q = c.f32[i];
     } else {
         using V = typename DVec<ND>::T;
-        V fv = static_cast<const V*>(c.f)[i];
+        const V fv = static_cast<const V*>(c.f)[i];
         const double* fp = reinterpret_cast<const double*>(&fv);
 #pragma unroll
         for (int d = 0; d < ND; d++) f[d] = fp[d];
     }
     const bool sol = (MODE == DM_SOL);
-    const bool has_a = sol ? !(m == 0.0 || isinf(m)) : mobile(m);
-    if (!has_a) {
+    const bool mob = mobile_bits(m);
+    if (sol ? zero_or_inf_bits(m) : !mob) {
 #pragma unroll
         for (int d = 0; d < ND; d++) {
             a[d] = 0.0;
@@ -74,9 +77,14 @@ __device__ __forceinline__ void kick(const DevCtx& c, uint32_t i, double m, doub
         return;
     }
     if constexpr (MIXED) {
-        const float im = mobile(m) ? c.invm32[i] : (float)(1.0 / m);
+        const float im = mob ? c.invm32[i] : (float)(1.0 / m);   // (Sol, m < 0)
+        a[0] = f2d_bits(q.x * im);
+        a[1] = f2d_bits(q.y * im);
+        if constexpr (ND == 3) a[2] = f2d_bits(q.z * im);
+    } else if (__double_as_longlong(m) == 0x3FF0000000000000ll) {
+        // f / 1 == f: a third of the FP64 operations of the kernel for unit masses
 #pragma unroll
-        for (int d = 0; d < ND; d++) a[d] = f2d_bits(fm[d] * im);
+        for (int d = 0; d < ND; d++) a[d] = f[d];
     } else {
 #pragma unroll
         for (int d = 0; d < ND; d++) a[d] = f[d] / m;
@@ -88,32 +96,32 @@ __device__ __forceinline__ void kick(const DevCtx& c, uint32_t i, double m, doub
 
 // Fused time-step kernel: [kick of the previous step] + drift of this step +
 // FP32 position view + the neighbour-list displacement test (the reference
-// runs that test at the end of the step; positions do not change after the
-// drift, so testing here sees the same values).
+// drift, so testing here sees the same values).  Bound by the ~260 B per atom,
+// which takes every warp an SM holds: issuing all of an atom's loads before the
+// first use (58 registers), or arming the next rebuild in the last block (the
+// blocks wait for their arrival), made 1,048,576 LJ atoms 54 -> 63 and 70 us.
 template <int ND, int MODE, bool KICK, bool MIXED>
-__global__ void __launch_bounds__(BLOCK) k_kickdrift(DevCtx c) {
+__global__ void __launch_bounds__(BLOCK, MIXED && MODE == DM_VERLET ? 8 : 1) k_kickdrift(DevCtx c) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     using V = typename DVec<ND>::T;
     bool valid = false;
     double dsq = 0.0;
-    uint32_t s = i < c.n ? c.atom_sys[i] : 0u;
+    const uint32_t s = i < c.n ? c.atom_sys[i] : 0u;
     if (i < c.n && c.active[s]) {
-        const StepParams& P = *c.params;
         const double m = c.m[i];
-        V xv = static_cast<V*>(c.x)[i];
-        V vv = static_cast<V*>(c.v)[i];
-        V av;
+        V xv = static_cast<const V*>(c.x)[i];
+        V vv = static_cast<const V*>(c.v)[i];
+        V av{};
+        const StepParams& P = *c.params;
         double* x = reinterpret_cast<double*>(&xv);
         double* v = reinterpret_cast<double*>(&vv);
         double* a = reinterpret_cast<double*>(&av);
-        const bool mob = MIXED ? mobile_bits(m) : mobile(m);
+        const bool mob = mobile_bits(m);
         if constexpr (MIXED && MODE == DM_VERLET) {
             // leapfrog form of the same update: the previous step's closing
             // half kick and this step's opening one use the same force, so
             // v_half += a dt and x += v_half dt (two FP64 fused
             // multiply-adds per axis instead of four)
-#pragma unroll
-            for (int d = 0; d < (int)(sizeof(V) / 8); d++) a[d] = 0.0;
             if (mob) {
                 if constexpr (KICK) {
                     const float4 q = c.f32[i];
@@ -135,13 +143,8 @@ __global__ void __launch_bounds__(BLOCK) k_kickdrift(DevCtx c) {
                 for (int d = 0; d < ND; d++) v[d] = 0.0;
             }
         } else {
-        if constexpr (KICK) {
-#pragma unroll
-            for (int d = 0; d < (int)(sizeof(V) / 8); d++) a[d] = 0.0;
-            kick<ND, MODE, MIXED>(c, i, m, a, v);
-        } else {
-            av = static_cast<const V*>(c.a)[i];
-        }
+        if constexpr (KICK) kick<ND, MODE, MIXED>(c, i, m, a, v);
+        else av = static_cast<const V*>(c.a)[i];
         if (!mob) {
 #pragma unroll
             for (int d = 0; d < ND; d++) v[d] = 0.0;
@@ -202,22 +205,16 @@ __global__ void __launch_bounds__(BLOCK) k_kickdrift(DevCtx c) {
         if (KICK && !MIXED) static_cast<V*>(c.a)[i] = av;
         if (mob) {
             // fine part of the FP32 position view against the coarse part fixed
-            // at the last rebuild or upload (x - X is exact in FP64); an atom
-            // that has moved more than 1/4 from its coarse point is re-anchored
-            // (any multiple of 1/8 is a valid coarse point)
-            // (mixed path: on the bit patterns, integer and FP32 instructions
-            // only, within one ulp of (float)(x - X) and equal to it but for
-            // rare roundings; FP64 path: the FP64 subtraction, exact, with the
-            // conversions on the bit patterns)
-            float4 A = c.pos[2 * (size_t)i];
-            float4 B;
-            auto fine = [](double xd, float Xf) {
-                return MIXED ? fine_bits(xd, Xf) : d2f_bits(xd - f2d_bits(Xf));
-            };
-            B.x = fine(x[0], A.x);
-            B.y = fine(x[1], A.y);
+            // at the last rebuild or upload, on the bit patterns (integer and
+            // FP32 instructions only, within one ulp of (float)(x - X) and equal
+            // to it but for rare roundings); an atom that has moved more than
+            // 1/4 from its coarse point is re-anchored (any multiple of 1/8 is a
+            // valid coarse point)
+            float4 A = c.pos[2 * (size_t)i], B;
+            B.x = fine_bits(x[0], A.x);
+            B.y = fine_bits(x[1], A.y);
             B.z = 0.f;
-            if constexpr (ND == 3) B.z = fine(x[2], A.z);
+            if constexpr (ND == 3) B.z = fine_bits(x[2], A.z);
             B.w = 0.f;
             if (fabsf(B.x) > 0.25f || fabsf(B.y) > 0.25f || fabsf(B.z) > 0.25f) {
                 posq_split2(x[0], A.x, B.x);
@@ -230,9 +227,9 @@ __global__ void __launch_bounds__(BLOCK) k_kickdrift(DevCtx c) {
                 if (c.staged) c.rec[i] = make_record(A, B, c.rframe[i]);
         }
         if (c.rank[i] != NOT_MEMBER) {
-            const V l = static_cast<const V*>(c.lastloc)[i];
+            const V lv = static_cast<const V*>(c.lastloc)[i];
             if constexpr (MIXED) {
-                const double* lp = reinterpret_cast<const double*>(&l);
+                const double* lp = reinterpret_cast<const double*>(&lv);
                 const double d0 = x[0] - lp[0], d1 = x[1] - lp[1];
                 dsq = __fma_rn(d1, d1, d0 * d0);
                 if constexpr (ND == 3) {
@@ -240,7 +237,7 @@ __global__ void __launch_bounds__(BLOCK) k_kickdrift(DevCtx c) {
                     dsq = __fma_rn(d2, d2, dsq);
                 }
             } else {
-                dsq = disp_sq<ND>(xv, l);
+                dsq = disp_sq<ND>(xv, lv);
             }
             // dsq is a sum of squares: +0, positive, +inf or NaN, so the tests
             // compare bit patterns (integer instructions, not the FP64 pipe)

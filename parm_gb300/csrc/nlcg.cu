@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(BLOCK) k_nlcg_stepx(DevCtx c, int use_cond, cu
     }
     if constexpr (TRACK) {
         check_accumulate(c, s, valid, dsq);
-        if (last_block(&c.done[0], gridDim.x)) arm_systems(c, 0, use_cond, handle);
+        arm_by_last_block(c, 0, use_cond, handle);
     }
 }
 

@@ -34,7 +34,7 @@ __device__ __forceinline__ void posq_split(double x, float& X, float& xf) {
 // arm: decide, per system, whether this step starts with a rebuild
 // ---------------------------------------------------------------------------
 __global__ void k_arm(DevCtx c, int count_step, int use_cond, cudaGraphConditionalHandle handle) {
-    arm_systems(c, count_step, use_cond, handle);
+    arm_systems(c, blockDim.x, count_step, use_cond, handle);
 }
 
 // ---------------------------------------------------------------------------

@@ -92,34 +92,35 @@ __device__ __forceinline__ void check_accumulate(const DevCtx& c, uint32_t sys_i
     }
 }
 
-// Whether this block is the last of its grid to arrive at `counter` (every
-// thread of every block calls it, with its own writes done); the last block
-// sees the others' writes (through L2: __ldcg, atomics) and leaves the counter
-// at 0 for the next launch.
+// Thread 0 of a block: whether the block is the last of its grid to arrive at
+// `counter`.  The block's writes before its last barrier are seen by the last
+// block (the fence is cumulative over the barrier; read them through L2:
+// __ldcg, atomics), and the counter is left at 0 for the next launch.
+__device__ __forceinline__ bool arrive_last(uint32_t* counter, uint32_t blocks) {
+    __threadfence();
+    if (atomicAdd(counter, 1u) + 1u != blocks) return false;
+    atomicExch(counter, 0u);
+    __threadfence();
+    return true;
+}
+
+// the same, asked by every thread of the block
 __device__ __forceinline__ bool last_block(uint32_t* counter, uint32_t blocks) {
     __shared__ uint32_t last;
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t k = atomicAdd(counter, 1u);
-        last = k + 1u == blocks ? 1u : 0u;
-        if (last) atomicExch(counter, 0u);
-    }
+    if (threadIdx.x == 0) last = arrive_last(counter, blocks) ? 1u : 0u;
     __syncthreads();
-    if (last) __threadfence();
     return last != 0u;
 }
 
-// Arm (one block): decide, per system, whether a rebuild is due, from the
-// forced requests and the two largest displacements; counts the build and
-// clears what it consumed, and sets the conditional node's value.
-__device__ __forceinline__ void arm_systems(const DevCtx& c, int count_step, int use_cond,
+// Arm: decide, per system, whether a rebuild is due, from the forced requests
+// and the two largest displacements; counts the build and clears what it
+// consumed, and sets the conditional node's value.  Executed by the first
+// `threads` threads of a block (32: one warp, no block barrier; else all).
+__device__ __forceinline__ void arm_systems(const DevCtx& c, uint32_t threads, int count_step, int use_cond,
                                             cudaGraphConditionalHandle handle) {
-    __shared__ int sany;
-    if (threadIdx.x == 0) sany = 0;
-    __syncthreads();
     int any = 0;
-    for (uint32_t s = threadIdx.x; s < c.nsys; s += blockDim.x) {
+    for (uint32_t s = threadIdx.x; s < c.nsys; s += threads) {
         if (count_step && !c.active[s]) {
             // frozen system: no rebuild in time steps; its pending test
             // (displacements, forced rebuild) waits until it is stepped again
@@ -139,13 +140,28 @@ __device__ __forceinline__ void arm_systems(const DevCtx& c, int count_step, int
         reinterpret_cast<ulonglong2*>(c.top)[s] = make_ulonglong2(0ull, 0ull);
         any |= rb ? 1 : 0;
     }
-    if (any) atomicOr(&sany, 1);
-    __syncthreads();
+    if (threads == 32u) any = __any_sync(0xFFFFFFFFu, any);
+    else any = __syncthreads_or(any);
     if (threadIdx.x == 0) {
-        *c.any_flag = (uint32_t)sany;
-        if (sany) *c.chains += 1u;
+        *c.any_flag = (uint32_t)(any != 0);
+        if (any) *c.chains += 1u;
         if (count_step) c.params->step += 1ull;
-        if (use_cond) cudaGraphSetConditional(handle, sany ? 1u : 0u);
+        if (use_cond) cudaGraphSetConditional(handle, any ? 1u : 0u);
+    }
+}
+
+// Arm by the last block of a grid (after check_accumulate).  Up to 32 systems,
+// one warp of each block sees to it and the others leave at once: a block that
+// waits as a whole for its arrival costs large grids a sixth of their time.
+__device__ __forceinline__ void arm_by_last_block(const DevCtx& c, int count_step, int use_cond,
+                                                  cudaGraphConditionalHandle handle) {
+    if (c.nsys <= 32u) {
+        if (threadIdx.x >= 32u) return;
+        bool last = false;
+        if (threadIdx.x == 0) last = arrive_last(&c.done[0], gridDim.x);
+        if (__any_sync(0xFFFFFFFFu, last)) arm_systems(c, 32u, count_step, use_cond, handle);
+    } else if (last_block(&c.done[0], gridDim.x)) {
+        arm_systems(c, blockDim.x, count_step, use_cond, handle);
     }
 }
 

@@ -142,6 +142,7 @@ struct DevCtx {
     uint32_t nblk;        // blocks over all systems
     uint32_t stg_cap;     // atoms staged in shared memory per block
     uint32_t stg_cap_eval;   // the same for the evaluation kernel
+    uint32_t stg_lg;      // force kernel: 2^stg_lg threads per home atom
     uint32_t stg_prm;     // force kernel: 0 uniform parameters, 1 per-atom sigma, 2 all per atom
     uint32_t stg_dia;     // list build: per-atom list diameters
     const uint4* blk;     // per block: (system, x0 | x1 << 16, y0 | y1 << 16, z)

@@ -1,6 +1,8 @@
 // Mixed-precision cell-block kernels: list build, pair forces and list
 // expansion with the neighbourhood of a block of cells staged in shared memory
 // (blocks, staged records and lists: staged.cuh).
+#include <algorithm>
+
 #include "staged.cuh"
 
 namespace parm {
@@ -259,29 +261,46 @@ struct HomePre {
     const uint32_t* row;
 };
 
-__device__ __forceinline__ HomePre home_pre(const DevCtx& c, const HomeAtom& a) {
+// MULTI: thread `sub` of 2^lg takes the words sub, sub + 2^lg, ...
+template <bool MULTI = false>
+__device__ __forceinline__ HomePre home_pre(const DevCtx& c, const HomeAtom& a, uint32_t sub = 0u, uint32_t lg = 0u) {
     HomePre p;
     p.nn = c.nnb[a.i];
     p.Qi = c.prm32[a.i];
     p.row = reinterpret_cast<const uint32_t*>(c.nbr16) + ((size_t)a.s0 * c.maxnb >> 1) + a.hs;
+    if constexpr (MULTI) {
+        p.row += (size_t)sub * a.H;
+        const uint32_t nw = (p.nn + 1u) >> 1;   // words in use
+        p.w0 = sub < nw ? __ldg(p.row) : 0u;
+        p.w1 = sub + (1u << lg) < nw ? __ldg(p.row + ((size_t)a.H << lg)) : 0u;
+        return p;
+    }
     p.w0 = __ldg(p.row);       // entries of the first two words (read even when
     p.w1 = __ldg(p.row + a.H); // the list is shorter: they lie inside its region)
     return p;
 }
 
-template <int ND, int KIND, int PRM, bool FULL>
+template <int ND, int KIND, int PRM, bool FULL, bool MULTI>
 __device__ __forceinline__ void force_home(const DevCtx& c, const SysConst& S, const StgTable& T,
                                            const float4* srec, const void* sext, uint32_t cap,
                                            const HomeAtom& a, const HomePre& pre, const Law<KIND>& law0,
-                                           float* f, uint32_t hidx) {
+                                           float* f, uint32_t hidx, uint32_t sub, uint32_t lg) {
     float dmin = 1.0f;   // min over pairs of |rsq - cut^2| - band (LJCUT)
     const float4 ri = FULL ? srec[a.qi] : stg_get<ND>(c, S, T, srec, cap, a.qi);
     const uint32_t wi = stg_wi(ri);
     const float* ssig = static_cast<const float*>(sext);
     const float4* sprm = static_cast<const float4*>(sext);
     const float4 Qi = pre.Qi;
-    const uint32_t nn = pre.nn;
-    const uint32_t H = a.H;
+    // MULTI: this thread's words, as a list of its own (every word's entries but
+    // the high half of the list's last word when its length is odd)
+    uint32_t nn = pre.nn, H = a.H;
+    if constexpr (MULTI) {
+        const uint32_t nw = (nn + 1u) >> 1, split = 1u << lg;
+        const uint32_t mine = nw > sub ? (nw - sub + split - 1u) >> lg : 0u;
+        const bool last = mine && sub + ((mine - 1u) << lg) == nw - 1u;
+        nn = 2u * mine - ((last && (nn & 1u)) ? 1u : 0u);
+        H <<= lg;
+    }
     const uint32_t* row = pre.row;
     const uint32_t qmax = T.total - 1u;
     auto pair = [&](uint32_t q) {
@@ -409,6 +428,17 @@ __device__ __forceinline__ void force_home(const DevCtx& c, const SysConst& S, c
         pair(w >> 16);
     }
     if (nn & 1u) pair((nw == 0 ? pre.w0 : (nw == 1 ? pre.w1 : __ldg(row + (size_t)nw * H))) & 0xFFFFu);
+    if constexpr (MULTI) {
+        // the atom's threads are neighbouring lanes of one warp
+        const uint32_t lane = threadIdx.x & 31u, split = 1u << lg;
+        const uint32_t group = (split == 32u ? 0xFFFFFFFFu : (1u << split) - 1u) << (lane & ~(split - 1u));
+        for (uint32_t o = split >> 1; o; o >>= 1) {
+#pragma unroll
+            for (int d = 0; d < ND; d++) f[d] += __shfl_xor_sync(group, f[d], o);
+            if constexpr (KIND == KIND_LJCUT) dmin = fminf(dmin, __shfl_xor_sync(group, dmin, o));
+        }
+        if (sub) return;
+    }
     if constexpr (KIND == KIND_LJCUT) {
         // rare: a pair within the cut-off band; k_band_stg settles it by the
         // exact FP64 test after this kernel (kept out of this loop so that the
@@ -420,7 +450,9 @@ __device__ __forceinline__ void force_home(const DevCtx& c, const SysConst& S, c
     }
 }
 
-template <int ND, int KIND, int MODE, int PRM>
+// MULTI: 2^stg_lg threads per home atom (small systems: blocks with few home
+// atoms, so that there are blocks for every SM, and short serial lists)
+template <int ND, int KIND, int MODE, int PRM, bool MULTI>
 __global__ void __launch_bounds__(STG_THREADS, 5) k_force_stg(DevCtx c) {
     extern __shared__ float4 smem_f[];
     __shared__ StgTable T;
@@ -440,24 +472,27 @@ __global__ void __launch_bounds__(STG_THREADS, 5) k_force_stg(DevCtx c) {
     // wait, so its latency overlaps with the bulk copies
     HomeAtom a0{};
     HomePre p0{};
-    const bool has0 = threadIdx.x < T.nhome;
+    const uint32_t lg = MULTI ? c.stg_lg : 0u, sub = MULTI ? threadIdx.x & ((1u << lg) - 1u) : 0u;
+    const uint32_t hfirst = MULTI ? threadIdx.x >> lg : threadIdx.x;
+    const bool has0 = hfirst < T.nhome;
     if (has0) {
-        a0 = stg_home<ND, false>(c, T, threadIdx.x);
-        p0 = home_pre(c, a0);
+        a0 = stg_home<ND, false>(c, T, hfirst);
+        p0 = home_pre<MULTI>(c, a0, sub, lg);
     }
     __shared__ uint64_t bar;
     if (!stg_load_bulk<ND, PRM>(c, T, srec, sext, cap, &bar)) return;
     const bool full = T.total <= cap;
-    for (uint32_t h = threadIdx.x; h < T.nhome; h += blockDim.x) {
-        const HomeAtom a = h == threadIdx.x ? a0 : stg_home<ND, false>(c, T, h);
-        const HomePre pre = h == threadIdx.x ? p0 : home_pre(c, a);
+    for (uint32_t h = hfirst; h < T.nhome; h += MULTI ? blockDim.x >> lg : blockDim.x) {
+        const HomeAtom a = h == hfirst ? a0 : stg_home<ND, false>(c, T, h);
+        const HomePre pre = h == hfirst ? p0 : home_pre<MULTI>(c, a, sub, lg);
         const float4 Qi = pre.Qi;
         Law<KIND> law;
         law.set((KIND == KIND_REPULSION) ? Qi.x * Qi.x : 12.0f * Qi.x * Qi.x, Qi.y, rcp_approx(Qi.y * Qi.y),
                 Qi.z);
         float f[3] = {0.f, 0.f, 0.f};
-        if (full) force_home<ND, KIND, PRM, true>(c, S, T, srec, sext, cap, a, pre, law, f, h);
-        else force_home<ND, KIND, PRM, false>(c, S, T, srec, sext, cap, a, pre, law, f, h);
+        if (full) force_home<ND, KIND, PRM, true, MULTI>(c, S, T, srec, sext, cap, a, pre, law, f, h, sub, lg);
+        else force_home<ND, KIND, PRM, false, MULTI>(c, S, T, srec, sext, cap, a, pre, law, f, h, sub, lg);
+        if (MULTI && sub) continue;
         c.f32[a.i] = make_float4(f[0], f[1], f[2], 0.f);
         if constexpr (MODE == FM_FORCES_A) {
             using V = typename DVec<ND>::T;
@@ -591,6 +626,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS) k_band_stg(DevCtx c) {
         }
         __syncthreads();
     }
+    if (last_block(&c.done[0], gridDim.x) && threadIdx.x == 0) *c.bandn = 0u;   // for the next force launch
 }
 
 // ---------------------------------------------------------------------------
@@ -661,9 +697,12 @@ static void set_smem(K kern, size_t bytes) {
 
 template <int ND, int KIND, int MODE>
 static void limits_prm(size_t sm) {
-    set_smem(k_force_stg<ND, KIND, MODE, 0>, sm);
-    set_smem(k_force_stg<ND, KIND, MODE, 1>, sm);
-    set_smem(k_force_stg<ND, KIND, MODE, 2>, sm);
+    set_smem(k_force_stg<ND, KIND, MODE, 0, false>, sm);
+    set_smem(k_force_stg<ND, KIND, MODE, 1, false>, sm);
+    set_smem(k_force_stg<ND, KIND, MODE, 2, false>, sm);
+    set_smem(k_force_stg<ND, KIND, MODE, 0, true>, sm);
+    set_smem(k_force_stg<ND, KIND, MODE, 1, true>, sm);
+    set_smem(k_force_stg<ND, KIND, MODE, 2, true>, sm);
 }
 template <int ND, int KIND>
 static void limits_kind(size_t sm) {
@@ -722,21 +761,28 @@ void launch_build_stg(const DevCtx& c, cudaStream_t s) {
 
 constexpr unsigned BAND_CTAS = 2048;
 
+template <int ND, int KIND, int MODE, int PRM>
+static void force_stg_split(const DevCtx& c, cudaStream_t s, unsigned g, size_t sm) {
+    if (c.stg_lg) k_force_stg<ND, KIND, MODE, PRM, true><<<g, STG_THREADS, sm, s>>>(c);
+    else k_force_stg<ND, KIND, MODE, PRM, false><<<g, STG_THREADS, sm, s>>>(c);
+}
+
 template <int ND, int KIND, int MODE>
 static void force_stg_prm(const DevCtx& c, cudaStream_t s) {
     const size_t sm = stg_smem_force(c);
     const unsigned g = c.nblk + c.nsys;
-    if (KIND == KIND_LJCUT) cudaMemsetAsync(c.bandn, 0, sizeof(uint32_t), s);
     switch (c.stg_prm) {
-        case 0: k_force_stg<ND, KIND, MODE, 0><<<g, STG_THREADS, sm, s>>>(c); break;
-        case 1: k_force_stg<ND, KIND, MODE, 1><<<g, STG_THREADS, sm, s>>>(c); break;
-        default: k_force_stg<ND, KIND, MODE, 2><<<g, STG_THREADS, sm, s>>>(c); break;
+        case 0: force_stg_split<ND, KIND, MODE, 0>(c, s, g, sm); break;
+        case 1: force_stg_split<ND, KIND, MODE, 1>(c, s, g, sm); break;
+        default: force_stg_split<ND, KIND, MODE, 2>(c, s, g, sm); break;
     }
     if (KIND == KIND_LJCUT) {
+        // about one atom in 1500 of an LJ liquid has a pair in the band
+        const unsigned bg = std::max(16u, std::min(BAND_CTAS, c.n / 512u));
         switch (c.stg_prm) {
-            case 0: k_band_stg<ND, KIND, MODE, 0><<<BAND_CTAS, 32 * BAND_WARPS, 0, s>>>(c); break;
-            case 1: k_band_stg<ND, KIND, MODE, 1><<<BAND_CTAS, 32 * BAND_WARPS, 0, s>>>(c); break;
-            default: k_band_stg<ND, KIND, MODE, 2><<<BAND_CTAS, 32 * BAND_WARPS, 0, s>>>(c); break;
+            case 0: k_band_stg<ND, KIND, MODE, 0><<<bg, 32 * BAND_WARPS, 0, s>>>(c); break;
+            case 1: k_band_stg<ND, KIND, MODE, 1><<<bg, 32 * BAND_WARPS, 0, s>>>(c); break;
+            default: k_band_stg<ND, KIND, MODE, 2><<<bg, 32 * BAND_WARPS, 0, s>>>(c); break;
         }
     }
 }
