@@ -307,9 +307,12 @@ struct parm_system {
         }
         bucket_off[nsys] = total;
         c.any_wrap = 0;
-        for (uint32_t s2 = 0; s2 < nsys; s2++)
+        c.cell_mean = 0;
+        for (uint32_t s2 = 0; s2 < nsys; s2++) {
+            c.cell_mean = std::max(c.cell_mean, (natoms[s2] + sys[s2].ncell - 1u) / sys[s2].ncell);
             for (int d = 0; d < nd; d++)
                 if (sys[s2].nc[d] < 3) c.any_wrap = 1;
+        }
         // k_force64s (a thread per entry) for lists that leave a warp per list idle,
         // from where its CTAs of 16 atoms fill the SMs (force kernel, a warp per
         // list / a thread per entry: 16.4 / 17.4 us on 5003 spheres, 34.5 / 30.1 on
@@ -1064,8 +1067,9 @@ struct parm_system {
                (c.rsq_n ? (c.rsq_com ? 5 : 2) : 0);
     }
     uint64_t chain_len() const {
-        if (c.prec == PREC_FP64) return c.pairf ? 12 : 11;
-        return (!c.staged && c.ntile && c.tiled) ? 11 : 10;
+        const uint64_t common = c.nbucket <= 4096u ? 7 : 9;   // one-block scan, or three passes
+        if (c.prec == PREC_FP64) return common + (c.pairf ? 2 : 1);
+        return common + ((!c.staged && c.ntile && c.tiled) ? 1 : 0);
     }
 
     // sums of what was launched last: per-atom values in red (or, with

@@ -15,6 +15,8 @@
 //
 // Compiled with -fmad=false: every FP64 expression here must round exactly
 // like the reference's unfused CPU arithmetic.
+#include <algorithm>
+
 #include "parm_check.cuh"
 
 namespace parm {
@@ -40,14 +42,6 @@ __global__ void k_arm(DevCtx c, int count_step, int use_cond, cudaGraphCondition
 // ---------------------------------------------------------------------------
 // rebuild chain (every kernel skips systems whose flag is clear)
 // ---------------------------------------------------------------------------
-__global__ void k_zero_cells(DevCtx c) {
-    uint32_t s = blockIdx.x;
-    if (!c.flag[s]) return;
-    if (threadIdx.x == 0 && c.half_cnt) c.half_cnt[s] = 0u;
-    uint32_t b0 = c.bucket_off[s], nb = c.sys[s].ncell + 1;
-    for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) c.cell_count[b0 + b] = 0u;
-}
-
 template <int ND>
 __global__ void k_bin(DevCtx c) {
     // every lane of the warp reaches the cell-count update below (the grid is
@@ -109,6 +103,7 @@ __global__ void k_bin(DevCtx c) {
 constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
+constexpr uint32_t SCAN_ONE = 1;   // chunks up to which one block scans them all (three: 6 us slower than the passes)
 
 struct SegPair {
     uint32_t f;  // segment starts in this span
@@ -157,6 +152,15 @@ __device__ __forceinline__ SegPair seg_block_scan(SegPair x, SegPair& aggregate)
     SegPair carry = seg_combine(prev_w, prev_l);
     __syncthreads();
     return carry;
+}
+
+// offset of bucket b from the segmented prefix `run` before its item
+__device__ __forceinline__ void bucket_offset(const DevCtx& c, uint32_t b, const SegPair& item, const SegPair& run) {
+    const uint32_t s = c.bucket_sys[b];
+    if (!c.flag[s]) return;
+    c.cell_start[b] = c.sys[s].atom_off + (item.f ? 0u : run.v);   // exclusive, restarted per system
+    c.cell_count[b] = 0u;
+    if (item.f && c.half_cnt) c.half_cnt[s] = 0u;   // the rebuild hands out the system's pair slots anew
 }
 
 __device__ __forceinline__ SegPair bucket_item(const DevCtx& c, uint32_t b) {
@@ -211,10 +215,32 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_write(DevCtx c) {
     for (int k = 0; k < SCAN_ITEMS; k++) {
         const uint32_t b = base + k;
         if (b >= c.nbucket) break;
-        const uint32_t excl = items[k].f ? 0u : run.v;   // exclusive, restarted per system
+        bucket_offset(c, b, items[k], run);
         run = seg_combine(run, items[k]);
-        const uint32_t s = c.bucket_sys[b];
-        if (c.flag[s]) c.cell_start[b] = c.sys[s].atom_off + excl;
+    }
+}
+
+// the whole scan in one block
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_one(DevCtx c) {
+    SegPair carry{0u, 0u};
+    for (uint32_t b0 = 0; b0 < c.nbucket; b0 += SCAN_CHUNK) {
+        const uint32_t base = b0 + threadIdx.x * SCAN_ITEMS;
+        SegPair items[SCAN_ITEMS];
+        SegPair t{0u, 0u};
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            items[k] = bucket_item(c, base + k);
+            t = seg_combine(t, items[k]);
+        }
+        SegPair agg;
+        SegPair run = seg_combine(carry, seg_block_scan(t, agg));
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; k++) {
+            if (base + k >= c.nbucket) break;
+            bucket_offset(c, base + k, items[k], run);
+            run = seg_combine(run, items[k]);
+        }
+        carry = seg_combine(carry, agg);
     }
 }
 
@@ -397,15 +423,19 @@ __device__ __noinline__ bool keep_exact(const DevCtx& c, const SysConst& S, uint
 // the periodic continuation of the grid (axes with a single cell take a
 // per-pair minimum image instead).  Distances are screened in FP32; candidates
 // within 2e-4 (relative) of the threshold get the exact FP64 reference test.
+// `parts` warps share a cell, each taking every parts-th group of `per` of its
+// home atoms (grids of a few cells with tens of atoms each would otherwise run
+// on a few warps: 296 -> 25 us at 1000 LJ atoms in 27 cells).
 constexpr int BUILD_WARPS = 4;
 template <int ND, bool WRAP>
-__global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c) {
+__global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c, uint32_t parts, uint32_t per) {
     __shared__ float4 home[BUILD_WARPS][32];
     __shared__ uint32_t pre[BUILD_WARPS][32];
     __shared__ uint32_t jst[BUILD_WARPS][32];
     __shared__ float4 soff[BUILD_WARPS][32];
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const uint32_t b = blockIdx.x * BUILD_WARPS + wib;   // one warp per bucket
+    const uint32_t wid = blockIdx.x * BUILD_WARPS + wib;
+    const uint32_t b = wid / parts, part = wid % parts;   // bucket, share of its home atoms
     if (b >= c.nbucket) return;
     const uint32_t s = c.bucket_sys[b];
     if (!c.flag[s]) return;
@@ -418,7 +448,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c) {
         return;
     }
     const uint32_t cs = c.cell_start[b], ce = c.cell_start[b + 1];
-    if (cs == ce) return;
+    if (cs + part * per >= ce) return;
     const int nc0 = S.nc[0], nc1 = S.nc[1], nc2 = S.nc[2];
     const int ci0 = (int)(myb % (uint32_t)nc0);
     const int ci1 = (int)((myb / (uint32_t)nc0) % (uint32_t)nc1);
@@ -460,8 +490,8 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c) {
     const float skin32 = (float)S.skin;
     const bool uni_thr = c.uniform & UNI_DIAM;
     const uint32_t maxnb = c.maxnb;
-    for (uint32_t hb = cs; hb < ce; hb += 32) {
-        const uint32_t mh = min(32u, ce - hb);
+    for (uint32_t hb = cs + part * per; hb < ce; hb += parts * per) {
+        const uint32_t mh = min(per, ce - hb);
         if (lane < mh) home[wib][lane] = c.posw[hb + lane];
         uint32_t mycnt = 0;   // neighbours found so far for home atom hb + lane
         __syncwarp();
@@ -473,10 +503,12 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c) {
             uint32_t j = 0xFFFFFFFFu;
             float4 Q = make_float4(0.f, 0.f, 0.f, 0.f);
             if (valid) {
+                // the last stencil cell that starts at or before q (unused lanes
+                // hold the total)
                 uint32_t st = 0;
-#pragma unroll 1
-                for (uint32_t k = 1; k < nst; k++)
-                    if (pre[wib][k] <= q) st = k;
+#pragma unroll
+                for (uint32_t h = 16; h; h >>= 1)
+                    if (pre[wib][st + h] <= q) st += h;
                 j = jst[wib][st] + (q - pre[wib][st]);
                 const float4 R = c.posw[j];
                 const float4 O = soff[wib][st];
@@ -913,12 +945,15 @@ void launch_arm(const DevCtx& c, cudaStream_t s, int count_step, int use_cond,
 
 void launch_rebuild(const DevCtx& c, cudaStream_t s) {
     unsigned ga = grid_for(c.n);
-    k_zero_cells<<<c.nsys, 256, 0, s>>>(c);
     if (c.nd == 3) k_bin<3><<<ga, BLOCK, 0, s>>>(c); else k_bin<2><<<ga, BLOCK, 0, s>>>(c);
     const uint32_t nblk = (c.nbucket + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    k_scan_blocks<<<nblk, SCAN_THREADS, 0, s>>>(c);
-    k_scan_aux<<<1, SCAN_THREADS, 0, s>>>(c, nblk);
-    k_scan_write<<<nblk, SCAN_THREADS, 0, s>>>(c);
+    if (nblk <= SCAN_ONE) {
+        k_scan_one<<<1, SCAN_THREADS, 0, s>>>(c);
+    } else {
+        k_scan_blocks<<<nblk, SCAN_THREADS, 0, s>>>(c);
+        k_scan_aux<<<1, SCAN_THREADS, 0, s>>>(c, nblk);
+        k_scan_write<<<nblk, SCAN_THREADS, 0, s>>>(c);
+    }
     k_scatter<<<ga, BLOCK, 0, s>>>(c);
     k_cellsort<<<(unsigned)(((size_t)c.nbucket * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, s>>>(c);
     if (c.staged) {
@@ -945,16 +980,24 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
         launch_half(c, s, 0);
         return;
     }
+    // home atoms per warp: 32 (most cells whole) where the cells alone give every
+    // SM its warps, shared among a few where some system's cells hold many more;
+    // else as few as it takes to give every SM its warps
+    const uint32_t want = 152u * 32u, mean = c.n / c.nbucket + 1u;
+    uint32_t parts = std::min(std::max(want / c.nbucket, 1u), std::min(mean, 32u));
+    const uint32_t per = parts == 1u ? 32u : std::min(32u, (mean + parts - 1u) / parts);
+    if (c.cell_mean > 48u) parts = std::max(parts, std::min(8u, (c.cell_mean + 31u) / 32u));
+    const unsigned gb = (unsigned)(((size_t)c.nbucket * parts + BUILD_WARPS - 1) / BUILD_WARPS);
     if (c.nd == 3) {
         k_gather<3><<<ga, BLOCK, 0, s>>>(c);
         k_copyback<3><<<ga, BLOCK, 0, s>>>(c);
-        if (c.any_wrap) k_build<3, true><<<(c.nbucket + BUILD_WARPS - 1) / BUILD_WARPS, BUILD_WARPS * 32, 0, s>>>(c);
-        else k_build<3, false><<<(c.nbucket + BUILD_WARPS - 1) / BUILD_WARPS, BUILD_WARPS * 32, 0, s>>>(c);
+        if (c.any_wrap) k_build<3, true><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
+        else k_build<3, false><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
     } else {
         k_gather<2><<<ga, BLOCK, 0, s>>>(c);
         k_copyback<2><<<ga, BLOCK, 0, s>>>(c);
-        if (c.any_wrap) k_build<2, true><<<(c.nbucket + BUILD_WARPS - 1) / BUILD_WARPS, BUILD_WARPS * 32, 0, s>>>(c);
-        else k_build<2, false><<<(c.nbucket + BUILD_WARPS - 1) / BUILD_WARPS, BUILD_WARPS * 32, 0, s>>>(c);
+        if (c.any_wrap) k_build<2, true><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
+        else k_build<2, false><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
     }
     if (c.prec == PREC_FP64) {
         launch_half(c, s, 0);

@@ -64,6 +64,7 @@ struct DevCtx {
     // device word: nonzero once an upload gave two atoms different masses;
     // zero, a rebuild's permutation leaves m and invm32 as they are
     uint32_t* m_mixed;
+    uint32_t cell_mean;  // atoms per cell in the system of the fullest cells
     uint32_t nbucket;  // total buckets (sum over systems of ncell + 1)
     uint32_t any_wrap; // some system has an axis with a single cell (per-pair minimum image)
     uint32_t any_lees; // some system is a LeesEdwardsBox: all-pairs list builds
@@ -98,7 +99,7 @@ struct DevCtx {
     float4* posw;         // rebuild only: position relative to its cell's lower corner (FP32), w = list diameter
 
     // rebuild scratch
-    uint32_t* cell_count;
+    uint32_t* cell_count;   // zero between rebuilds
     uint32_t* cell_start;   // start of every bucket; the bucket after a system's cells holds its non-members
     const uint32_t* bucket_sys;  // system of each bucket
     uint32_t* scan_aux;     // per scan block: (segment flag, sum)
