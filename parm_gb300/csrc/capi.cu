@@ -744,8 +744,10 @@ struct parm_system {
                 CUDA_TRY(cudaEventRecord(ev_join, st3));
             }
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step + 1], st, cudaEventRecordExternal));
-            if (prec == PREC_FP64) launch_force64(c, st, fmode);
-            else launch_force32(c, st, fmode);
+            DevCtx cf = c;
+            cf.pdl = timing ? 0u : 1u;
+            if (prec == PREC_FP64) launch_force64(cf, st, fmode);
+            else launch_force32(cf, st, fmode);
             if (timing) CUDA_TRY(cudaEventRecordWithFlags(ge.ev[3 * step + 2], st, cudaEventRecordExternal));
             launch_rsq(c, st, 0);   // trackers, at the end of the step (positions final)
             CUDA_TRY(cudaGetLastError());

@@ -102,6 +102,7 @@ __device__ __forceinline__ void kick(const DevCtx& c, uint32_t i, double m, doub
 // blocks wait for their arrival), made 1,048,576 LJ atoms 54 -> 63 and 70 us.
 template <int ND, int MODE, bool KICK, bool MIXED>
 __global__ void __launch_bounds__(BLOCK, MIXED && MODE == DM_VERLET ? 8 : 1) k_kickdrift(DevCtx c) {
+    release_next();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     using V = typename DVec<ND>::T;
     bool valid = false;

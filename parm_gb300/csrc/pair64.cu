@@ -514,7 +514,7 @@ template <int ND, int KIND>
 __device__ __forceinline__ bool screen64(const DevCtx& c, const SysConst& S, const float4& Ai, const float4& Bi,
                                          const float4& Qi, uint32_t j, bool& wrap) {
     float4 Aj, Bj;
-    ld_pos(c.pos, j, Aj, Bj);
+    ld_pos_coherent(c.pos, j, Aj, Bj);
     float4 Qj = Qi;
     if ((c.uniform & UNI_ALL) != UNI_ALL) Qj = c.prm32[j];
     // (the screen is per-axis periodic: not for a sheared box)
@@ -600,11 +600,18 @@ __device__ __forceinline__ void forces64(const DevCtx& c) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t i0 = blockIdx.x * F64_ATOMS;
     const bool all_uni = (c.uniform & UNI_ALL) == UNI_ALL;
+    release_next();
+    // (list lengths and ranks do not change in the drift before)
+    bool go = false;
     if (tid < F64_ATOMS) {
         const uint32_t i = i0 + tid;
-        const bool go = i < c.n && c.active[c.atom_sys[i]] && c.rank[i] != NOT_MEMBER;
+        go = i < c.n && c.active[c.atom_sys[i]] && c.rank[i] != NOT_MEMBER;
         nn_s[tid] = !go ? 0u : (HALF ? c.half_n[i] : c.nnb[i]);
         slot0[tid] = HALF && go ? c.half_base[i] : 0u;
+    }
+    wait_previous();
+    if (tid < F64_ATOMS) {
+        const uint32_t i = i0 + tid;
         double xi[3] = {0, 0, 0};
         if (go) load3<ND>(c.x, i, xi);
 #pragma unroll
@@ -627,7 +634,7 @@ __device__ __forceinline__ void forces64(const DevCtx& c) {
                 const SysConst& S = c.sys[c.atom_sys[i]];
                 const uint32_t* nb = c.nbr + (size_t)i * c.maxnb;
                 float4 Ai, Bi;
-                ld_pos(c.pos, i, Ai, Bi);
+                ld_pos_coherent(c.pos, i, Ai, Bi);
                 const float4 Qi = c.prm32[i];
                 for (uint32_t k0 = base; k0 < hi; k0 += 32u) {
                     const uint32_t k = k0 + lane;
@@ -726,12 +733,14 @@ __global__ void __launch_bounds__(F64S_THREADS) k_force64s(DevCtx c) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
     const uint32_t i0 = blockIdx.x * F64S_ATOMS;
     const bool all_uni = (c.uniform & UNI_ALL) == UNI_ALL;
+    release_next();
     uint32_t nn = 0u, nmax = 0u;   // of atom i0 + lane, in every warp
     {
         const uint32_t i = i0 + lane;
         const bool go = lane < F64S_ATOMS && i < c.n && c.active[c.atom_sys[i]] && c.rank[i] != NOT_MEMBER;
         if (go) nn = c.nnb[i];
         nmax = __reduce_max_sync(0xFFFFFFFFu, nn);
+        wait_previous();
         if (tid < F64S_ATOMS) {
             double xi[3] = {0, 0, 0};
             if (go) load3<ND>(c.x, i, xi);
@@ -769,7 +778,7 @@ __global__ void __launch_bounds__(F64S_THREADS) k_force64s(DevCtx c) {
                 const uint32_t i = i0 + a;
                 j = __ldg(c.nbr + (size_t)i * c.maxnb + base + (t - off[a]));
                 float4 Ai, Bi;
-                ld_pos(c.pos, i, Ai, Bi);
+                ld_pos_coherent(c.pos, i, Ai, Bi);
                 keep = screen64<ND, KIND>(c, c.sys[c.atom_sys[i]], Ai, Bi, c.prm32[i], j, wrap);
                 if (!keep) {
 #pragma unroll
@@ -987,20 +996,21 @@ template <int ND, int KIND>
 static void force64_nd_kind(const DevCtx& c, cudaStream_t s, int mode) {
     const unsigned g = grid_for(c.n, F64_ATOMS);
     if (c.pairf) {
-        k_pair64<ND, KIND><<<g, F64_THREADS, 0, s>>>(c);
+        launch_after(c, k_pair64<ND, KIND>, g, F64_THREADS, 0, s, c);
         const unsigned gs = grid_for(c.n, (int)(SUM64_WARPS * sum64_atoms<ND>()));
+        // (not overlapped with k_pair64: its waiting CTAs cost that kernel's tail 5 us at 29,667 atoms)
         if (mode == FM_FORCES_A) k_sum64<ND, FM_FORCES_A><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
         else k_sum64<ND, FM_FORCES><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
         return;
     }
     if (c.short_lists) {
         const unsigned gs = grid_for(c.n, F64S_ATOMS);
-        if (mode == FM_FORCES_A) k_force64s<ND, KIND, FM_FORCES_A><<<gs, F64S_THREADS, 0, s>>>(c);
-        else k_force64s<ND, KIND, FM_FORCES><<<gs, F64S_THREADS, 0, s>>>(c);
+        if (mode == FM_FORCES_A) launch_after(c, k_force64s<ND, KIND, FM_FORCES_A>, gs, F64S_THREADS, 0, s, c);
+        else launch_after(c, k_force64s<ND, KIND, FM_FORCES>, gs, F64S_THREADS, 0, s, c);
         return;
     }
-    if (mode == FM_FORCES_A) k_force64<ND, KIND, FM_FORCES_A><<<g, F64_THREADS, 0, s>>>(c);
-    else k_force64<ND, KIND, FM_FORCES><<<g, F64_THREADS, 0, s>>>(c);
+    if (mode == FM_FORCES_A) launch_after(c, k_force64<ND, KIND, FM_FORCES_A>, g, F64_THREADS, 0, s, c);
+    else launch_after(c, k_force64<ND, KIND, FM_FORCES>, g, F64_THREADS, 0, s, c);
 }
 
 template <int ND>

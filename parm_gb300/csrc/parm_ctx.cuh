@@ -139,6 +139,7 @@ struct DevCtx {
 
     // cell-block kernels of the mixed path (staged.cu): blocks of Kx x Ky
     // cells whose neighbourhood is staged in shared memory; 16-bit lists
+    uint32_t pdl;         // host: launches of a captured step may overlap the kernel before them (launch_after)
     uint32_t staged;      // use them (every system has >= 3 cells per axis)
     uint32_t nblk;        // blocks over all systems
     uint32_t stg_cap;     // atoms staged in shared memory per block
@@ -369,6 +370,30 @@ constexpr int STG_PIECES_MAX = 3 * STG_ROWS_MAX;
 constexpr int STG_KX_MAX = 32;
 constexpr int STG_THREADS_HOST = 256;     // threads per block of the cell-block kernels
 constexpr uint32_t STG_TAB_WORDS = 160;   // 16-byte words per block table (>= its size)
+
+// Launch of a kernel that may start while the kernel before it on the stream
+// drains (programmatic dependent launch): it calls wait_previous() before it
+// reads anything that kernel writes, and that kernel calls release_next().
+// Only between kernels that follow each other directly (c.pdl: captured steps
+// without timing events between them).
+template <class K, class... A>
+inline void launch_after(const DevCtx& c, K kern, unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = c.pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}
+#if defined(__CUDACC__)
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
 
 inline unsigned grid_for(uint32_t n, int block = BLOCK) {
     unsigned g = (unsigned)((n + block - 1) / block);

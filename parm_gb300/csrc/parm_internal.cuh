@@ -197,4 +197,14 @@ __device__ __forceinline__ void ld_pos(const float4* pos, uint32_t j, float4& A,
         : "l"(q));
 }
 
+// the same through the coherent path, for kernels that may start before the one
+// that writes the positions has finished
+__device__ __forceinline__ void ld_pos_coherent(const float4* pos, uint32_t j, float4& A, float4& B) {
+    const double4_32a t = *(reinterpret_cast<const double4_32a*>(pos) + j);
+    A = make_float4(__int_as_float(__double2loint(t.x)), __int_as_float(__double2hiint(t.x)),
+                    __int_as_float(__double2loint(t.y)), __int_as_float(__double2hiint(t.y)));
+    B = make_float4(__int_as_float(__double2loint(t.z)), __int_as_float(__double2hiint(t.z)),
+                    __int_as_float(__double2loint(t.w)), __int_as_float(__double2hiint(t.w)));
+}
+
 }  // namespace parm

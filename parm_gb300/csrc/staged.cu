@@ -456,7 +456,11 @@ template <int ND, int KIND, int MODE, int PRM, bool MULTI>
 __global__ void __launch_bounds__(STG_THREADS, 5) k_force_stg(DevCtx c) {
     extern __shared__ float4 smem_f[];
     __shared__ StgTable T;
+    // until wait_previous() only what list builds and uploads set is read
+    // (never what the drift before writes), and nothing is written
+    release_next();
     if (blockIdx.x >= c.nblk) {
+        wait_previous();
         if (c.active[blockIdx.x - c.nblk]) stg_nonmembers(c, blockIdx.x - c.nblk, MODE == FM_FORCES_A);
         return;
     }
@@ -464,7 +468,7 @@ __global__ void __launch_bounds__(STG_THREADS, 5) k_force_stg(DevCtx c) {
     if (!c.active[bd.x]) return;   // frozen system: forces unchanged
     const SysConst& S = c.sys[bd.x];
     stg_load_table(c, T, blockIdx.x);
-    stg_prefetch<ND>(c, T, true);
+    stg_prefetch<ND>(c, T, true);   // (into L2, where the drift's writes land too)
     const uint32_t cap = c.stg_cap;
     float4* srec = smem_f;
     void* sext = smem_f + cap;
@@ -480,6 +484,7 @@ __global__ void __launch_bounds__(STG_THREADS, 5) k_force_stg(DevCtx c) {
         p0 = home_pre<MULTI>(c, a0, sub, lg);
     }
     __shared__ uint64_t bar;
+    wait_previous();
     if (!stg_load_bulk<ND, PRM>(c, T, srec, sext, cap, &bar)) return;
     const bool full = T.total <= cap;
     for (uint32_t h = hfirst; h < T.nhome; h += MULTI ? blockDim.x >> lg : blockDim.x) {
@@ -527,6 +532,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS) k_band_stg(DevCtx c) {
     __shared__ float4 corr[BAND_MAXK];
     __shared__ uint32_t flags[BAND_MAXK / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    wait_previous();
     const uint32_t nb = min(*c.bandn, c.n);
     for (uint32_t it_k = blockIdx.x; it_k < nb; it_k += gridDim.x) {
         const uint2 it = c.bandq[it_k];
@@ -763,8 +769,8 @@ constexpr unsigned BAND_CTAS = 2048;
 
 template <int ND, int KIND, int MODE, int PRM>
 static void force_stg_split(const DevCtx& c, cudaStream_t s, unsigned g, size_t sm) {
-    if (c.stg_lg) k_force_stg<ND, KIND, MODE, PRM, true><<<g, STG_THREADS, sm, s>>>(c);
-    else k_force_stg<ND, KIND, MODE, PRM, false><<<g, STG_THREADS, sm, s>>>(c);
+    if (c.stg_lg) launch_after(c, k_force_stg<ND, KIND, MODE, PRM, true>, g, STG_THREADS, sm, s, c);
+    else launch_after(c, k_force_stg<ND, KIND, MODE, PRM, false>, g, STG_THREADS, sm, s, c);
 }
 
 template <int ND, int KIND, int MODE>
@@ -780,9 +786,9 @@ static void force_stg_prm(const DevCtx& c, cudaStream_t s) {
         // about one atom in 1500 of an LJ liquid has a pair in the band
         const unsigned bg = std::max(16u, std::min(BAND_CTAS, c.n / 512u));
         switch (c.stg_prm) {
-            case 0: k_band_stg<ND, KIND, MODE, 0><<<bg, 32 * BAND_WARPS, 0, s>>>(c); break;
-            case 1: k_band_stg<ND, KIND, MODE, 1><<<bg, 32 * BAND_WARPS, 0, s>>>(c); break;
-            default: k_band_stg<ND, KIND, MODE, 2><<<bg, 32 * BAND_WARPS, 0, s>>>(c); break;
+            case 0: launch_after(c, k_band_stg<ND, KIND, MODE, 0>, bg, 32 * BAND_WARPS, 0, s, c); break;
+            case 1: launch_after(c, k_band_stg<ND, KIND, MODE, 1>, bg, 32 * BAND_WARPS, 0, s, c); break;
+            default: launch_after(c, k_band_stg<ND, KIND, MODE, 2>, bg, 32 * BAND_WARPS, 0, s, c); break;
         }
     }
 }
