@@ -102,6 +102,16 @@ PARM_FPB_HD float d2f_bits(double d) {
     return (float)d;
 }
 
+// (float)d rounded towards zero without a branch, for seeds and small terms:
+// below 2^-126 zero; |d| < 2^127
+PARM_FPB_HD float d2f_chop(double d) {
+    uint32_t hi, lo;
+    fpb_d2hilo(d, hi, lo);
+    const uint32_t e = (hi >> 20) & 0x7FFu;
+    const uint32_t f = ((e - 896u) << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+    return fpb_u2f((hi & 0x80000000u) | (e > 896u ? f : 0u));
+}
+
 PARM_FPB_HD float fpb_i2f(int32_t i) {
 #if defined(__CUDA_ARCH__)
     return __int2float_rn(i);

@@ -90,7 +90,7 @@ __device__ __forceinline__ double noise_radius(const NoiseTable* t, unsigned lon
     const int e = 9 - lz + (k >= NOISE_SPLIT ? 1 : 0);   // log2 of the leading bit - 54, + 1 above sqrt 2
     const double m = __hiloint2double((int)(0x3FF00000u | (uint32_t)(frac >> 44)), (int)(uint32_t)(frac >> 12));
     const double2 L = __ldg(reinterpret_cast<const double2*>(t->lg[k]));
-    const double ed = f2d_bits((float)e);
+    const double ed = f2d_flush((float)e);
     const double r = __fma_rn(m, L.x, -1.0);   // |r| < 2^-8
     // -2 log u = -2 ln2 e - 2 log c - 2 r + r^2 - 2/3 r^3 + ...; -2 ln2 in two parts, the first short enough
     // for an exact product with e
@@ -99,14 +99,14 @@ __device__ __forceinline__ double noise_radius(const NoiseTable* t, unsigned lon
     const double hi = __fma_rn(r, -2.0, T);
     double lo = __fma_rn(r, -2.0, __dsub_rn(T, hi));
     lo = __fma_rn(ed, L2L, lo);
-    const float rf = d2f_bits(r);
+    const float rf = d2f_chop(r);
     const float tail = rf * fmaf(rf, 1.0f / 3.0f, -0.4f);   // r^5 and r^6: below 2^-42 of the sum
-    const double P = __fma_rn(r, __fma_rn(r, __dadd_rn(f2d_bits(tail), 0.5), -2.0 / 3.0), 1.0);
+    const double P = __fma_rn(r, __fma_rn(r, __dadd_rn(f2d_flush(tail), 0.5), -2.0 / 3.0), 1.0);
     double x = __dadd_rn(hi, __fma_rn(__dmul_rn(r, r), P, lo));
     if (__double2hiint(x) <= 0x00100000) return 0.0;   // u = 1 (x is 0 to rounding)
     float y0;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d2f_bits(x)));
-    const double y = f2d_bits(y0), h = f2d_bits(0.5f * y0);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d2f_chop(x)));
+    const double y = f2d_flush(y0), h = f2d_flush(0.5f * y0);
     const double g = __dmul_rn(x, y);
     const double g1 = __fma_rn(g, __fma_rn(-g, h, 0.5), g);
     return __fma_rn(__fma_rn(-g1, g1, x), h, g1);
@@ -123,9 +123,9 @@ __device__ __forceinline__ void noise_turn(const NoiseTable* t, unsigned long lo
     const double a = __dmul_rn(dd, 0x1.921fb54442d18p-52);   // 2 pi 2^-54 d, |a| < 2^-7.3
     const double a2 = __dmul_rn(a, a);
     const double sa = __fma_rn(__dmul_rn(a, a2), __fma_rn(a2, 1.0 / 120.0, -1.0 / 6.0), a);
-    const float a2f = d2f_bits(a2);
+    const float a2f = d2f_chop(a2);
     const float tail = a2f * fmaf(a2f, -1.0f / 720.0f, 1.0f / 24.0f);
-    const double cm1 = __dmul_rn(a2, __dadd_rn(f2d_bits(tail), -0.5));   // cos a - 1
+    const double cm1 = __dmul_rn(a2, __dadd_rn(f2d_flush(tail), -0.5));   // cos a - 1
     cs = __dadd_rn(C.x, __fma_rn(C.x, cm1, -__dmul_rn(C.y, sa)));
     sn = __dadd_rn(C.y, __fma_rn(C.y, cm1, __dmul_rn(C.x, sa)));
 }
