@@ -252,68 +252,63 @@ __global__ void k_scatter(DevCtx c) {
     c.perm[c.cell_start[c.bucket[i]] + c.cslot[i]] = i;
 }
 
-// deterministic order inside a cell: ascending neighbour-list rank.  One warp
-// per cell: each lane holds one atom of the cell (one of every 32 in larger
-// cells: few-cell boxes put tens to hundreds of atoms in one) and counts the
-// atoms ranked before it, 32 at a time.  Larger cells are placed through the
-// slot array, which nothing reads any more once the atoms are scattered.
-// Sorting them serially on lane 0 took 81 us at 1000 LJ
-// atoms in 27 cells (now 6.8) and 164 us on 48 packings of 64 to 4096 spheres
-// (now 11.4).
-__global__ void k_cellsort(DevCtx c) {
+// Permutation of the atoms' arrays into their new order, one warp per cell: the
+// order inside a cell is ascending neighbour-list rank, so each lane holds one
+// of the cell's scattered atoms (one of every 32 in larger cells: few-cell boxes
+// put tens to hundreds of atoms in one), counts the atoms of the cell ranked
+// before it, 32 at a time, and moves its atom's entries to that place.  (Sorting
+// large cells serially on lane 0 took 164 us on 48 packings of 64 to 4096
+// spheres; sort and move as two kernels cost a batch of 48 replicas, one of
+// which rebuilds nearly every step, 1 % of the step.)
+template <int ND>
+__global__ void k_sortgather(DevCtx c) {
     const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (b >= c.nbucket) return;   // uniform in the warp
     const uint32_t s = c.bucket_sys[b];
     if (!c.flag[s]) return;
-    const uint32_t local = b - c.bucket_off[s];
-    if (local >= c.sys[s].ncell) return;  // non-member bucket is placed by nm_rank
-    const uint32_t lo = c.cell_start[b], hi = c.cell_start[b + 1];
-    const uint32_t cnt = hi - lo;
-    if (cnt < 2) return;
+    const uint32_t local = b - c.bucket_off[s], ncell = c.sys[s].ncell;
+    if (local > ncell) return;   // (past a grid that has shrunk)
+    const bool members = local < ncell;   // the bucket after the cells: non-members, placed by nm_rank
+    const uint32_t lo = c.cell_start[b];
+    const uint32_t cnt = (members ? c.cell_start[b + 1] : c.sys[s].atom_off + c.sys[s].natoms) - lo;
+    using V = typename DVec<ND>::T;
+    const bool masses = *c.m_mixed != 0u;
     for (uint32_t q0 = 0; q0 < cnt; q0 += 32u) {
         const uint32_t q = q0 + lane;
-        const uint32_t v = q < cnt ? c.perm[lo + q] : 0u;
-        const uint32_t rk = q < cnt ? c.rank[v] : 0xFFFFFFFFu;
-        uint32_t pos = 0;
-        for (uint32_t t0 = 0; t0 < cnt; t0 += 32u) {
-            const uint32_t m = min(32u, cnt - t0);
-            uint32_t kt = rk;
-            if (t0 != q0) kt = lane < m ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
-            for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j) < rk ? 1u : 0u;
+        const bool on = q < cnt;
+        const uint32_t o = on ? c.perm[lo + q] : 0u;
+        const uint32_t rk = on ? c.rank[o] : 0xFFFFFFFFu;
+        uint32_t pos = q;
+        if (members && cnt > 1u) {
+            pos = 0u;
+            for (uint32_t t0 = 0; t0 < cnt; t0 += 32u) {
+                const uint32_t m = min(32u, cnt - t0);
+                uint32_t kt = rk;
+                if (t0 != q0) kt = lane < m ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
+                for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j) < rk ? 1u : 0u;
+            }
         }
-        if (q < cnt) (cnt <= 32u ? c.perm : c.cslot)[lo + pos] = v;
+        if (!on) continue;
+        const uint32_t k = lo + pos;
+        static_cast<V*>(c.x2)[k] = static_cast<const V*>(c.x)[o];
+        static_cast<V*>(c.v2)[k] = static_cast<const V*>(c.v)[o];
+        static_cast<V*>(c.a2)[k] = static_cast<const V*>(c.a)[o];
+        if (c.prec != PREC_MIXED) static_cast<V*>(c.f2)[k] = static_cast<const V*>(c.f)[o];   // FP64 forces: FP64 path only
+        c.f32b[k] = c.f32[o];
+        // arrays whose entries are all equal are left as they are (copy back too)
+        if (masses) {
+            c.m2[k] = c.m[o];
+            c.invm32b[k] = c.invm32[o];
+        }
+        if (!c.same_prm) {
+            c.prm2[k] = c.prm[o];
+            c.prm32b[k] = c.prm32[o];
+            c.diam2[k] = c.diam[o];
+        }
+        c.rank2[k] = rk;
+        c.orig2[k] = c.orig[o];
+        c.bucket2[k] = b;
     }
-    if (cnt <= 32u) return;
-    __syncwarp();
-    for (uint32_t q = lane; q < cnt; q += 32u) c.perm[lo + q] = c.cslot[lo + q];
-}
-
-template <int ND>
-__global__ void k_gather(DevCtx c) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= c.n) return;
-    uint32_t s = c.atom_sys[k];
-    if (!c.flag[s]) return;
-    using V = typename DVec<ND>::T;
-    uint32_t o = c.perm[k];
-    static_cast<V*>(c.x2)[k] = static_cast<const V*>(c.x)[o];
-    static_cast<V*>(c.v2)[k] = static_cast<const V*>(c.v)[o];
-    static_cast<V*>(c.a2)[k] = static_cast<const V*>(c.a)[o];
-    if (c.prec != PREC_MIXED) static_cast<V*>(c.f2)[k] = static_cast<const V*>(c.f)[o];   // FP64 forces: FP64 path only
-    c.f32b[k] = c.f32[o];
-    // arrays whose entries are all equal are left as they are (copy back too)
-    if (*c.m_mixed) {
-        c.m2[k] = c.m[o];
-        c.invm32b[k] = c.invm32[o];
-    }
-    if (!c.same_prm) {
-        c.prm2[k] = c.prm[o];
-        c.prm32b[k] = c.prm32[o];
-        c.diam2[k] = c.diam[o];
-    }
-    c.rank2[k] = c.rank[o];
-    c.orig2[k] = c.orig[o];
-    c.bucket2[k] = c.bucket[o];
 }
 
 template <int ND>
@@ -955,13 +950,13 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
         k_scan_write<<<nblk, SCAN_THREADS, 0, s>>>(c);
     }
     k_scatter<<<ga, BLOCK, 0, s>>>(c);
-    k_cellsort<<<(unsigned)(((size_t)c.nbucket * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, s>>>(c);
+    const unsigned gw = (unsigned)(((size_t)c.nbucket * 32 + BLOCK - 1) / BLOCK);   // a warp per bucket
+    if (c.nd == 3) k_sortgather<3><<<gw, BLOCK, 0, s>>>(c);
+    else k_sortgather<2><<<gw, BLOCK, 0, s>>>(c);
     if (c.staged) {
         if (c.nd == 3) {
-            k_gather<3><<<ga, BLOCK, 0, s>>>(c);
             k_copyback<3><<<ga, BLOCK, 0, s>>>(c);
         } else {
-            k_gather<2><<<ga, BLOCK, 0, s>>>(c);
             k_copyback<2><<<ga, BLOCK, 0, s>>>(c);
         }
         launch_build_stg(c, s);
@@ -969,11 +964,9 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
     }
     if (c.any_lees) {   // FP64 handles only
         if (c.nd == 3) {
-            k_gather<3><<<ga, BLOCK, 0, s>>>(c);
             k_copyback<3><<<ga, BLOCK, 0, s>>>(c);
             k_build_lees<3><<<ga, BLOCK, 0, s>>>(c);
         } else {
-            k_gather<2><<<ga, BLOCK, 0, s>>>(c);
             k_copyback<2><<<ga, BLOCK, 0, s>>>(c);
             k_build_lees<2><<<ga, BLOCK, 0, s>>>(c);
         }
@@ -989,12 +982,10 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
     if (c.cell_mean > 48u) parts = std::max(parts, std::min(8u, (c.cell_mean + 31u) / 32u));
     const unsigned gb = (unsigned)(((size_t)c.nbucket * parts + BUILD_WARPS - 1) / BUILD_WARPS);
     if (c.nd == 3) {
-        k_gather<3><<<ga, BLOCK, 0, s>>>(c);
         k_copyback<3><<<ga, BLOCK, 0, s>>>(c);
         if (c.any_wrap) k_build<3, true><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
         else k_build<3, false><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
     } else {
-        k_gather<2><<<ga, BLOCK, 0, s>>>(c);
         k_copyback<2><<<ga, BLOCK, 0, s>>>(c);
         if (c.any_wrap) k_build<2, true><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
         else k_build<2, false><<<gb, BUILD_WARPS * 32, 0, s>>>(c, parts, per);
