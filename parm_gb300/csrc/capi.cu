@@ -250,6 +250,20 @@ struct parm_system {
         return PARM_OK;
     }
 
+    // Tiles of the cell order along y (cell_row).  Three z layers of a tile are
+    // what an atom's neighbours span: with slots for the pair forces (FP64 path,
+    // ~1 KB per LJ atom) whole layers of a large box outgrow the L2, so tiles
+    // hold about 24,000 atoms in three layers (k_sum64 at 1,048,576 LJ atoms 1.25
+    // -> 1.01 ms).  The cell-block kernels of the mixed path and smaller boxes
+    // keep one tile.
+    uint32_t y_tile(const SysConst& S, uint32_t na) const {
+        const uint32_t ny = (uint32_t)S.nc[1];
+        if (prec != PREC_FP64 || nd != 3 || S.nc[2] < 3) return ny;
+        const double row = (double)na / ((double)S.nc[1] * S.nc[2]);   // atoms per row of cells
+        const double rows = 24000.0 / (3.0 * std::max(row, 1.0));
+        return rows >= ny ? ny : std::max(4u, (uint32_t)rows);
+    }
+
     // ---- cell grids (depend on the boxes and on the largest list radius) ----
     int setup_cells() {
         double dmax = 0.0;
@@ -289,6 +303,7 @@ struct parm_system {
                 }
             }
             S.ncell = (uint32_t)(S.nc[0] * S.nc[1] * S.nc[2]);
+            S.ytile = y_tile(S, natoms[s]);
             for (int d = 0; d < 3; d++) {
                 S.cellw_inv[d] = (float)(S.nc[d] / S.L[d]);
                 S.cellw[d] = S.L[d] / S.nc[d];
@@ -571,7 +586,7 @@ struct parm_system {
     // take part in (LJ and its kin) from 16,384 atoms: evaluating each pair once
     // then saves more than the second kernel and the slots cost (in-graph forces
     // with / without: 45 / 37 us at 4096 LJ atoms, 57 / 59 at 8000, 115 / 158 at
-    // 29,667, 3350 / 4370 at 1,048,576; contact laws, where a few entries of
+    // 29,667, 3100 / 4390 at 1,048,576; contact laws, where a few entries of
     // each list interact: 20 / 16 us on 5003 spheres, 64 / 54 on 65,536 disks).
     // And where they take at most a quarter of the free device memory and 32 GB:
     // a larger handle evaluates each pair twice instead, which needs none of it.

@@ -72,7 +72,7 @@ __global__ void k_bin(DevCtx c) {
             ci[d] = cc;
         }
         if (bad) atomicOr(c.status, ST_NONFINITE);
-        b = c.bucket_off[s] + (uint32_t)((ci[2] * S.nc[1] + ci[1]) * S.nc[0] + ci[0]);
+        b = c.bucket_off[s] + cell_row(S, ci[1], ci[2]) * (uint32_t)S.nc[0] + (uint32_t)ci[0];
     }
     // one atomic per distinct cell of the warp (atoms arrive in cell order,
     // so a warp holds two or three cells): the lanes of a cell take
@@ -371,8 +371,8 @@ __global__ void k_copyback(DevCtx c) {
     if (!c.staged && c.rank[k] != NOT_MEMBER) {
         const SysConst& S = c.sys[s];
         const uint32_t myb = c.bucket[k] - c.bucket_off[s];
-        const uint32_t ci[3] = {myb % (uint32_t)S.nc[0], (myb / (uint32_t)S.nc[0]) % (uint32_t)S.nc[1],
-                                myb / (uint32_t)(S.nc[0] * S.nc[1])};
+        uint32_t ci[3];
+        cell_coords(S, myb, ci);
         float pr[3] = {0.f, 0.f, 0.f};
 #pragma unroll
         for (int d = 0; d < ND; d++) {
@@ -445,9 +445,9 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c, uint32_t p
     const uint32_t cs = c.cell_start[b], ce = c.cell_start[b + 1];
     if (cs + part * per >= ce) return;
     const int nc0 = S.nc[0], nc1 = S.nc[1], nc2 = S.nc[2];
-    const int ci0 = (int)(myb % (uint32_t)nc0);
-    const int ci1 = (int)((myb / (uint32_t)nc0) % (uint32_t)nc1);
-    const int ci2 = (int)(myb / (uint32_t)(nc0 * nc1));
+    uint32_t ci[3];
+    cell_coords(S, myb, ci);
+    const int ci0 = (int)ci[0], ci1 = (int)ci[1], ci2 = (int)ci[2];
     const int r0 = nc0 >= 3 ? 1 : 0, r1 = nc1 >= 3 ? 1 : 0;
     const int r2 = (ND == 3 && nc2 >= 3) ? 1 : 0;
     const int w0 = 2 * r0 + 1, w1 = 2 * r1 + 1, w2 = 2 * r2 + 1;
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build(DevCtx c, uint32_t p
         cx = cx < 0 ? cx + nc0 : (cx >= nc0 ? cx - nc0 : cx);
         cy = cy < 0 ? cy + nc1 : (cy >= nc1 ? cy - nc1 : cy);
         cz = cz < 0 ? cz + nc2 : (cz >= nc2 ? cz - nc2 : cz);
-        const uint32_t cb = b0 + (uint32_t)((cz * nc1 + cy) * nc0 + cx);
+        const uint32_t cb = b0 + cell_row(S, cy, cz) * (uint32_t)nc0 + (uint32_t)cx;
         const uint32_t js = c.cell_start[cb];
         cntl = c.cell_start[cb + 1] - js;
         jst[wib][lane] = js;

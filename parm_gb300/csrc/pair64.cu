@@ -501,8 +501,8 @@ __device__ __forceinline__ float image32(const SysConst& S, const float4& Ai, co
 // Measured, LJ, ~72 listed pairs per atom (one GB300): a thread per atom that
 // walked its list 379 us at 1000 atoms, 385 us at 29,667, 8.03 ms at 1,048,576
 // (a third of its lanes idle in the FP64 part, a serial chain over the list);
-// k_force64 23.4 us, 161 us, 4.39 ms; k_pair64 + k_sum64 115 us at 29,667 and
-// 3.35 ms at 1,048,576.
+// k_force64 23.4 us, 161 us, 4.39 ms; k_pair64 + k_sum64 114 us at 29,667 and
+// 3.10 ms at 1,048,576 (k_pair64: FP64 pipe 85 % busy).
 // ---------------------------------------------------------------------------
 constexpr int F64_THREADS = 128;
 constexpr uint32_t F64_ATOMS = 8;    // x 3 components: the lanes of k_force64's summing warp
@@ -587,6 +587,11 @@ __device__ __forceinline__ void store_force(const DevCtx& c, uint32_t i, const d
     }
 }
 
+// a pair force's slot: one 32-byte (2D: 16-byte) access
+template <int ND> struct SlotVec;
+template <> struct SlotVec<3> { using T = double4_32a; };
+template <> struct SlotVec<2> { using T = double2; };
+
 // The work of k_pair64 (HALF) and k_force64.
 template <int ND, int KIND, int MODE, bool HALF>
 __device__ __forceinline__ void forces64(const DevCtx& c) {
@@ -596,7 +601,7 @@ __device__ __forceinline__ void forces64(const DevCtx& c) {
     __shared__ uint16_t pk[HALF ? F64_ATOMS * F64_CHUNK : 1];   // their list entries
     __shared__ double xs[F64_ATOMS][4];
     __shared__ uint32_t nn_s[F64_ATOMS], cnt[F64_ATOMS], slot0[F64_ATOMS];
-    using V = typename DVec<ND>::T;
+    using V = typename SlotVec<ND>::T;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t i0 = blockIdx.x * F64_ATOMS;
     const bool all_uni = (c.uniform & UNI_ALL) == UNI_ALL;
@@ -837,7 +842,7 @@ __global__ void __launch_bounds__(F64_THREADS) k_pair64(DevCtx c) {
 // pairs are consecutive; another atom's pair is one 32-byte sector), drops the
 // zeros and stages the rest in list order, then one lane per (atom, component)
 // adds them.  Bound by those FP64 adds and the 32 B per entry from L2 and
-// memory: ~30 us of the 115 at 29,667 LJ atoms, 1.2 ms of 3.35 at 1,048,576.
+// memory: ~30 us of the 114 at 29,667 LJ atoms, 1.0 ms of 3.10 at 1,048,576.
 constexpr int SUM64_WARPS = 4;
 template <int ND>
 constexpr uint32_t sum64_atoms() { return ND == 3 ? 10u : 16u; }   // x ND components: one warp
@@ -845,7 +850,7 @@ template <int ND, int MODE>
 __global__ void __launch_bounds__(32 * SUM64_WARPS) k_sum64(DevCtx c) {
     constexpr uint32_t ATOMS = sum64_atoms<ND>(), GROUP = ATOMS / 2;
     __shared__ double pf_s[SUM64_WARPS][ND][ATOMS * 33];
-    using V = typename DVec<ND>::T;
+    using V = typename SlotVec<ND>::T;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t i0 = (blockIdx.x * SUM64_WARPS + warp) * ATOMS;   // uniform in the warp from here
     if (i0 >= c.n) return;

@@ -348,13 +348,6 @@ __device__ __forceinline__ float4 make_record(const float4& A, const float4& B, 
     return make_float4(B.x + fr.x, B.y + fr.y, B.z + fr.z, __uint_as_float(w));
 }
 
-// cell coordinates of local bucket b
-__device__ __forceinline__ void cell_coords(const SysConst& S, uint32_t b, uint32_t* ci) {
-    ci[0] = b % (uint32_t)S.nc[0];
-    ci[1] = (b / (uint32_t)S.nc[0]) % (uint32_t)S.nc[1];
-    ci[2] = b / (uint32_t)(S.nc[0] * S.nc[1]);
-}
-
 constexpr int BLOCK = 256;
 constexpr uint32_t NO_SLOT = 0xFFFFFFFFu;
 // atoms per reduction chunk: four per thread of a reducing block (16 of them left

@@ -80,12 +80,38 @@ struct SysConst {
     double cellw[3];    // L / nc
     float cellw32[3];   // L / nc in FP32
     uint32_t cell_off;  // first cell of this system in the global cell array
+    uint32_t ytile;     // rows of cells along y per tile of the cell order (>= nc[1]: one tile)
     uint32_t ncell;
     uint32_t atom_off;
     uint32_t natoms;
     int lees;           // a LeesEdwardsBox (FP64 path): the y image shifts x by gamma Lx
     double gamma;
 };
+
+// Order of the cells: rows along x; the rows of a tile of up to ytile cells
+// along y by z layer, then the next tile.  One tile: x fastest, then y, then z.
+__host__ __device__ __forceinline__ uint32_t cell_row(const SysConst& S, int cy, int cz) {
+    const uint32_t T = S.ytile, ny = (uint32_t)S.nc[1];
+    if (T >= ny) return (uint32_t)cz * ny + (uint32_t)cy;
+    const uint32_t y0 = (uint32_t)cy / T * T, w = ny - y0 < T ? ny - y0 : T;
+    return y0 * (uint32_t)S.nc[2] + (uint32_t)cz * w + ((uint32_t)cy - y0);
+}
+
+// cell coordinates of local bucket b
+__host__ __device__ __forceinline__ void cell_coords(const SysConst& S, uint32_t b, uint32_t* ci) {
+    const uint32_t nx = (uint32_t)S.nc[0], ny = (uint32_t)S.nc[1], nz = (uint32_t)S.nc[2], T = S.ytile;
+    const uint32_t row = b / nx;
+    ci[0] = b - row * nx;
+    if (T >= ny) {
+        ci[2] = row / ny;
+        ci[1] = row - ci[2] * ny;
+        return;
+    }
+    const uint32_t y0 = row / (T * nz) * T, w = ny - y0 < T ? ny - y0 : T;
+    const uint32_t in = row - y0 * nz;
+    ci[2] = in / w;
+    ci[1] = y0 + (in - ci[2] * w);
+}
 
 // per-atom FP64 parameters of the pair interaction (kind dependent)
 //   LJCUT:     p0 = epsilon, p1 = sigma, p2 = sigcut, p3 = 1 - 1/pow(sigcut, 6)
