@@ -1908,9 +1908,7 @@ int parm_sol(parm_system* S, double dt, double damping, double T, uint64_t seed,
     if (!S->c.noise) {
         NoiseTable* d = nullptr;
         TRY(S->alloc(d, 1));
-        const NoiseTable t = noise_table();
-        CUDA_TRY(cudaMemcpyAsync(d, &t, sizeof(t), cudaMemcpyHostToDevice, S->st));
-        CUDA_TRY(cudaStreamSynchronize(S->st));
+        CUDA_TRY(cudaMemcpyAsync(d, &noise_table(), sizeof(NoiseTable), cudaMemcpyHostToDevice, S->st));
         S->c.noise = d;
     }
     std::vector<unsigned long long> seeds(S->nsys);
@@ -2525,8 +2523,7 @@ int parm_debug_normals(uint64_t seed, uint32_t sys, uint64_t step, uint32_t nato
     CUDA_TRY(cudaMalloc(&buf, sizeof(NoiseTable) + 48 * (size_t)natoms));
     NoiseTable* dt = reinterpret_cast<NoiseTable*>(buf);
     double* res = reinterpret_cast<double*>(dt + 1);
-    const NoiseTable t = noise_table();
-    cudaError_t e = cudaMemcpy(dt, &t, sizeof(t), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpy(dt, &noise_table(), sizeof(NoiseTable), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         launch_normals_test(dt, splitmix64(seed + sys), step, natoms, res, 0);
         e = cudaGetLastError();
