@@ -1084,7 +1084,7 @@ struct parm_system {
                (c.rsq_n ? (c.rsq_com ? 5 : 2) : 0);
     }
     uint64_t chain_len() const {
-        const uint64_t common = c.nbucket <= 4096u ? 6 : 8;   // one-block scan, or three passes
+        const uint64_t common = c.nbucket <= 4096u ? 6 : 7;   // one-block scan, or two passes
         if (c.prec == PREC_FP64) return common + (c.pairf ? 2 : 1);
         return common + ((!c.staged && c.ntile && c.tiled) ? 1 : 0);
     }
