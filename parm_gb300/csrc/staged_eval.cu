@@ -26,12 +26,6 @@ namespace parm {
 // ---------------------------------------------------------------------------
 constexpr uint32_t EVQ = 96;   // queue per warp: fewer than 32 waiting and two entries of each lane
 
-// 1 / x to an ulp: the approximate reciprocal and one Newton step
-__device__ __forceinline__ float rcp_ulp(float x) {
-    const float y = rcp_approx(x);
-    return fmaf(y, fmaf(-x, y, 1.0f), y);
-}
-
 // pair energy of k_eval32 for global atoms i, j (its displacement and law)
 template <int ND, int KIND>
 __device__ __forceinline__ float eval_exactly(const DevCtx& c, const SysConst& S, uint32_t i, uint32_t j) {
@@ -48,25 +42,16 @@ __device__ __forceinline__ float eval_exactly(const DevCtx& c, const SysConst& S
     return energy32<KIND>(d2, Qi.x * Qj.x, 0.5f * (Qi.y + Qj.y), third, m6);
 }
 
-// pair energy; `doubt`: zero or not, or its sign, may hang on the last bits
+// whether a pair's energy e (energy32) is zero or not, or its sign, may hang on
+// the last bits of the displacement; NaN counts as in doubt
 template <int KIND>
-__device__ __forceinline__ float eval_energy(float d2, float eps, float sig, float isig2, float third, float m6,
-                                             bool& doubt) {
+__device__ __forceinline__ bool eval_in_doubt(float e, float d2, float eps, float sig, float third) {
+    const float s2 = sig * sig;
     if constexpr (KIND == KIND_REPULSION) {
-        const float s2 = sig * sig;
-        doubt = fabsf(d2 - s2) <= 1e-4f * s2;
-        if (d2 > s2) return 0.0f;
-        const float b = fmaxf(1.0f - sqrtf(d2) * rcp_ulp(sig), 0.0f);
-        const float pw = third == 2.0f ? b * b : (third == 2.5f ? b * b * sqrtf(b) : powf(b, third));
-        return eps * pw * rcp_ulp(third);
+        return fabsf(d2 - s2) <= 1e-4f * s2 || (d2 <= s2 && !(fabsf(e) > 1e-30f));
     } else {
-        const float rsq = d2 * isig2;
-        const float cut2 = KIND == KIND_LJCUT ? third * third : 1.0f;
-        const float mid = 1.0f - rcp_ulp(rsq * rsq * rsq);
-        float e = eps * (mid * mid);
-        if constexpr (KIND == KIND_LJCUT) e = eps * (mid * mid - 1.0f) - eps * (m6 * m6 - 1.0f);
-        doubt = fabsf(rsq - cut2) <= 1e-4f * cut2 || fabsf(e) <= 1e-4f * eps;
-        return rsq > cut2 ? 0.0f : e;
+        const float rsq = d2 / s2, cut2 = KIND == KIND_LJCUT ? third * third : 1.0f;
+        return fabsf(rsq - cut2) <= 1e-4f * cut2 || (!(rsq > cut2) && !(fabsf(e) > 1e-4f * eps));
     }
 }
 
@@ -125,22 +110,22 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
         float eps = QU.x * QU.x, sig = QU.y, isig2 = isig2_u, third = QU.z, m6 = QU.w;
         if constexpr (PRM == 1) {
             sig = 0.5f * (sigma(qi) + sigma(q));
-            isig2 = rcp_ulp(sig * sig);
+            isig2 = 1.0f / (sig * sig);
         } else if constexpr (PRM == 2) {
             const float4 Qi = prm(qi), Qj = prm(q);
             eps = Qi.x * Qj.x;
             sig = 0.5f * (Qi.y + Qj.y);
-            isig2 = rcp_ulp(sig * sig);
+            isig2 = 1.0f / (sig * sig);
             third = cut_kind<KIND>() ? fmaxf(Qi.z, Qj.z) : 0.5f * (Qi.z + Qj.z);
             m6 = Qj.z > Qi.z ? Qj.w : Qi.w;
         }
         if (!SUMS || what == EV_ENERGY) {
-            bool doubt;
-            float e = eval_energy<KIND>(d2, eps, sig, isig2, third, m6, doubt);
+            float e = energy32<KIND>(d2, eps, sig, third, m6);
             if constexpr (SUMS) {
                 acc[0] += f2d_flush(e);
             } else {
-                if (doubt) e = eval_exactly<ND, KIND>(c, S, stg_global(T, qi), stg_global(T, q));
+                if (eval_in_doubt<KIND>(e, d2, eps, sig, third))
+                    e = eval_exactly<ND, KIND>(c, S, stg_global(T, qi), stg_global(T, q));
                 count += (what == EV_CONTACTS ? e != 0.0f : e > 0.0f) ? 1u : 0u;
             }
         } else if constexpr (SUMS) {
