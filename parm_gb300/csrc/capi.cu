@@ -155,6 +155,10 @@ struct parm_system {
     void* rsq_mem = nullptr;     // mean-square-displacement tracker arrays
     bool want_staged = true;     // prefer them when the grids allow
     bool stg_ok = false;         // the current grids allow them
+    // a rebuild of every list is owed since parm_set_interaction: the lists there
+    // are (none on a new handle) are row-major, also when c.staged asks for the next
+    // ones as cell-block lists, whose tables and pair slots no build has written yet
+    bool unbuilt = false;
     bool stg_pending = false;    // grids changed under staged lists: switch back once every system rebuilt
     std::vector<uint32_t> stg_mark;   // which() of each system when the grids changed
     uint32_t stage_cap_override = 0;  // test hook (parm_debug_stage_cap)
@@ -354,8 +358,7 @@ struct parm_system {
         if (c.staged) {
             // the staged lists index the old grids: keep them as row-major lists
             // until every system has been rebuilt on the new grids
-            launch_expand_stg(c, st);
-            CUDA_TRY(cudaGetLastError());
+            TRY(rowmajor());
             TRY(sync_status());
             c.staged = 0;
             stg_pending = true;
@@ -514,17 +517,29 @@ struct parm_system {
         launch_reframe(c, st);
         CUDA_TRY(cudaGetLastError());
         c.staged = 1;
-        stg_pending = false;
+        stg_pending = unbuilt = false;
         clear_graphs();
         return sync_status();
     }
 
     // row-major lists for the kernels that read them (evaluation, pair listing)
     int rowmajor() {
-        if (!c.staged) return PARM_OK;
+        if (!staged_lists()) return PARM_OK;
         launch_expand_stg(c, st);
         CUDA_TRY(cudaGetLastError());
         return PARM_OK;
+    }
+
+    bool staged_lists() const { return c.staged && !unbuilt; }
+
+    // for the pair kernels on the current lists
+    DevCtx list_ctx() const {
+        DevCtx k = c;
+        if (unbuilt) {
+            if (k.staged) k.staged = k.tiled = 0;
+            k.pairf = nullptr;
+        }
+        return k;
     }
 
     // (re)allocate the neighbour list; the current lists are kept (a larger
@@ -532,7 +547,7 @@ struct parm_system {
     int set_capacity(uint32_t maxnb) {
         maxnb = std::max<uint32_t>(8, (maxnb + 7) / 8 * 8);
         void* fresh = nullptr;
-        if (c.staged && nbr_mem) launch_expand_stg(c, st);   // the staged layout depends on maxnb
+        if (nbr_mem) TRY(rowmajor());   // the staged layout depends on maxnb
         CUDA_TRY(cudaStreamSynchronize(st));
         CUDA_TRY(cudaMalloc(&fresh, (size_t)maxnb * n * 4 + 16));
         if (nbr_mem) {
@@ -569,7 +584,7 @@ struct parm_system {
             nbr16_mem = nullptr;
             CUDA_TRY(cudaMalloc(&nbr16_mem, (size_t)maxnb * n * 2 + 16));
             c.nbr16 = static_cast<uint16_t*>(nbr16_mem);
-            if (c.staged) {
+            if (staged_lists()) {
                 launch_compress_stg(c, st);
                 CUDA_TRY(cudaGetLastError());
                 TRY(sync_status());
@@ -612,6 +627,7 @@ struct parm_system {
         CUDA_TRY(cudaMalloc(&slots_mem, sb));
         c.pairf = pairf_mem;
         c.slots = static_cast<uint32_t*>(slots_mem);
+        if (unbuilt) return PARM_OK;
         launch_half(c, st, 1);   // of the current lists
         CUDA_TRY(cudaGetLastError());
         return sync_status();
@@ -713,6 +729,7 @@ struct parm_system {
             CUDA_TRY(cudaGraphLaunch(it->second.exec, st));
         }
         CUDA_TRY(cudaGetLastError());
+        unbuilt = false;   // (the test serves every system, frozen ones too)
         // no synchronisation here: the caller's own call ends with one, which
         // reports any error of these kernels
         return stg_pending ? maybe_restage() : PARM_OK;
@@ -972,7 +989,9 @@ struct parm_system {
         launch_nlcg_ctl(cb, st, NP_BEGIN);
         launch_nlcg_stepx(cb, st, false, 0, 0);
         launch_nlcg_box(cb, st);
-        nlcg_forces(cb, cs, st);
+        DevCtx cf = cs;
+        if (unbuilt) cf.pairf = nullptr;
+        nlcg_forces(cb, cf, st);
         launch_nlcg_dot(cb, st, NT_FV, c.nlcg_step, NP_ETA0, 0, 0);
         TRY(nlcg_step_track(cb, st, st2, graph));
         nlcg_forces(cb, cs, st);
@@ -1035,10 +1054,16 @@ struct parm_system {
             max_sec = std::max(max_sec, (uint32_t)std::min(1e6, hp[(size_t)s * (sizeof(NlcgSys) / 8) + 4]));
         uint64_t launches = 0;
         const int mode = nlcg_boxed ? SM_NLCG : SM_NLCGV;
-        if (graph_k == 0) {
-            for (uint32_t k = 0; k < nsteps; k++) TRY(nlcg_emit_step(false, max_sec));
-        } else {
-            uint32_t done = 0;
+        uint32_t done = 0;
+        // forces come before the first step's list test: while lists without pair
+        // slots are current, that step is launched directly (a graph would keep its
+        // kernels)
+        while (done < nsteps && (graph_k == 0 || (unbuilt && c.pairf))) {
+            TRY(nlcg_emit_step(false, max_sec));
+            unbuilt = false;
+            done++;
+        }
+        if (done < nsteps) {
             while (done < nsteps) {
                 const uint32_t k = std::min(graph_k, nsteps - done);
                 const uint64_t key = ((uint64_t)mode << 40) | ((uint64_t)k << 1);
@@ -1066,6 +1091,7 @@ struct parm_system {
                     it = graphs.emplace(key, ge).first;
                 }
                 CUDA_TRY(cudaGraphLaunch(it->second.exec, st));
+                unbuilt = false;
                 launches += 1;
                 done += k;
             }
@@ -1617,6 +1643,7 @@ int parm_set_interaction(parm_system* S, int kind, const double* params, const u
     }
     S->c.kind = device_kind(kind);
     S->c.uniform = uni;
+    if (S->prec == PREC_FP64) S->unbuilt = true;   // (pair slots are by the ranks of the last build)
     launch_posq(S->c, S->st);
     CUDA_TRY(cudaGetLastError());
     TRY(S->setup_cells());
@@ -1628,6 +1655,7 @@ int parm_set_interaction(parm_system* S, int kind, const double* params, const u
     }
     // every list is rebuilt next (ignorechanged), in the preferred format
     const uint32_t was = S->c.staged;
+    if (!was) S->unbuilt = true;
     S->c.staged = (S->stg_ok && S->want_staged) ? 1u : 0u;
     S->stg_pending = false;
     if (S->c.staged != was) S->clear_graphs();
@@ -1725,6 +1753,7 @@ int parm_nlist_update(parm_system* S, int force, uint8_t* rebuilt) {
     launch_arm(S->c, S->st, 0, 0, 0);
     launch_rebuild(S->c, S->st);
     CUDA_TRY(cudaGetLastError());
+    S->unbuilt = false;
     TRY(S->sync_status());
     TRY(S->maybe_restage());
     if (rebuilt) {
@@ -1746,7 +1775,7 @@ int parm_nlist_which(parm_system* S, uint32_t* which) {
 int parm_nlist_numpairs(parm_system* S, uint64_t* numpairs) {
     if (!S || !numpairs) return fail(PARM_ERR_ARG, "NULL argument");
     TRY(S->flush());
-    const bool blocks = S->c.staged != 0;
+    const bool blocks = S->staged_lists();
     if (blocks) launch_eval_stg(S->c, S->st, EV_PAIRS);
     else launch_numpairs(S->c, S->st);
     std::vector<double> out;
@@ -1799,8 +1828,9 @@ int parm_set_forces(parm_system* S, int constraints_and_a) {
     if (!S) return fail(PARM_ERR_ARG, "NULL handle");
     TRY(S->flush());
     const int mode = constraints_and_a ? FM_FORCES_A : FM_FORCES;
-    if (S->prec == PREC_FP64) launch_force64(S->c, S->st, mode);
-    else launch_force32(S->c, S->st, mode);
+    const DevCtx c = S->list_ctx();
+    if (S->prec == PREC_FP64) launch_force64(c, S->st, mode);
+    else launch_force32(c, S->st, mode);
     CUDA_TRY(cudaGetLastError());
     return S->sync_status();
 }
@@ -1814,7 +1844,7 @@ int parm_evaluate(parm_system* S, int what, double* out) {
         std::fill(out, out + (size_t)S->nsys * ncomp, 0.0);
         return PARM_OK;
     }
-    const bool blocks = S->prec == PREC_MIXED && S->c.staged;
+    const bool blocks = S->staged_lists();
     if (S->prec == PREC_FP64) launch_eval64(S->c, S->st, what);
     else if (blocks) launch_eval_stg(S->c, S->st, what);
     else launch_eval32(S->c, S->st, what);
@@ -2080,11 +2110,11 @@ static int set_staged(parm_system* S, bool on) {
     if (on) {
         if (!S->stg_ok) return fail(PARM_ERR_ARG, "the cell-block kernel needs >= 3 cells per axis in every system");
         if (S->stg_pending) return PARM_OK;   // switches after the next rebuild of every system
-        launch_compress_stg(S->c, S->st);
+        if (!S->unbuilt) launch_compress_stg(S->c, S->st);
         launch_reframe(S->c, S->st);
         S->c.staged = 1;
     } else {
-        launch_expand_stg(S->c, S->st);
+        TRY(S->rowmajor());
         S->c.staged = 0;
     }
     CUDA_TRY(cudaGetLastError());
@@ -2182,6 +2212,7 @@ int parm_autotune(parm_system* S, uint32_t* tpa_out) {
         return PARM_OK;
     }
     TRY(S->flush());
+    if (S->unbuilt) TRY(parm_nlist_update(S, 0, nullptr));   // both formats of the lists are timed
     // keep the current forces: the candidates' sums round differently
     CUDA_TRY(cudaMemcpyAsync(S->c.f32b, S->c.f32, sizeof(float4) * (size_t)S->n, cudaMemcpyDeviceToDevice,
                              S->st));
@@ -2407,6 +2438,7 @@ int parm_nlcg_set_state(parm_system* S, const double* state) {
 static int nlcg_set_forces_impl(parm_system* S, bool c_and_a) {
     DevCtx cb, cs;
     S->nlcg_ctx(cb, cs);
+    if (S->unbuilt) cb.pairf = cs.pairf = nullptr;
     if (!S->nlcg_boxed) {
         const int mode = c_and_a ? FM_FORCES_A : FM_FORCES;
         if (S->prec == PREC_FP64) launch_force64(cb, S->st, mode);
@@ -2462,6 +2494,7 @@ int parm_nlcg_descend(parm_system* S) {
     launch_nlcg_atoms(cb, S->st, NA_DESCEND);
     launch_nlcg_ctl(cb, S->st, NP_DESCEND);
     TRY(S->nlcg_step_track(cb, S->st, nullptr, false));
+    S->unbuilt = false;
     TRY(S->sync_status());
     return S->nlcg_sync_boxes();
 }
