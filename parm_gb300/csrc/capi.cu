@@ -347,12 +347,12 @@ struct parm_system {
                                      cudaMemcpyHostToDevice, st));
             CUDA_TRY(cudaStreamSynchronize(st));
             clear_graphs();
+            const bool lists = staged_lists();
             TRY(plan_blocks());
-            if (c.staged) {
-                launch_reframe(c, st);
-                CUDA_TRY(cudaGetLastError());
-                TRY(sync_status());
-            }
+            if (c.staged) launch_reframe(c, st);
+            else if (lists) launch_expand_stg(c, st);   // the new law has no cell-block kernels: keep the lists
+            CUDA_TRY(cudaGetLastError());
+            if (c.staged || lists) TRY(sync_status());
             return PARM_OK;
         }
         if (c.staged) {

@@ -116,3 +116,16 @@ def test_minimiser_before_the_first_build(boxed):
         out.append((g.get_atoms()["x"], g.get_atoms()["f"], g.which()))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_old_lists_under_a_law_without_cell_blocks():
+    """The attractive LJ on the grid of the LJ lists: the per-atom kernels take over, on the same pairs."""
+    w = _work(kind=0)
+    g, ref = make_gpu(w, precision="mixed"), make_gpu(w, precision="mixed")
+    ref.set_threads_per_atom(101)
+    for h in (g, ref):
+        h.nlist_update(False)
+        h.set_interaction(3, w.params, w.skin)
+    got, want = _all(g), _all(ref)
+    assert want[5][0] > 1000
+    _same(got, want)
