@@ -603,8 +603,9 @@ struct parm_system {
     // with / without: 45 / 37 us at 4096 LJ atoms, 57 / 59 at 8000, 115 / 158 at
     // 29,667, 3100 / 4390 at 1,048,576; contact laws, where a few entries of
     // each list interact: 20 / 16 us on 5003 spheres, 64 / 54 on 65,536 disks).
-    // And where they take at most a quarter of the free device memory and 32 GB:
-    // a larger handle evaluates each pair twice instead, which needs none of it.
+    // And where they take at most a quarter of the free device memory and 32 GB,
+    // and the allocation succeeds: another handle evaluates each pair twice
+    // instead, which needs none of it.
     bool slots_pay() const {
         if (want_slots >= 0) return want_slots != 0;
         const bool lj = kind == PARM_LJCUT || kind == PARM_LJATTRACTCUT ||
@@ -623,8 +624,15 @@ struct parm_system {
         size_t freeb = 0, totalb = 0;
         CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
         if (!slots_pay() || pb + sb > std::min<size_t>(freeb / 4, (size_t)32 << 30)) return PARM_OK;
-        CUDA_TRY(cudaMalloc(&pairf_mem, pb));
-        CUDA_TRY(cudaMalloc(&slots_mem, sb));
+        cudaError_t e = cudaMalloc(&pairf_mem, pb);
+        if (e == cudaSuccess) e = cudaMalloc(&slots_mem, sb);
+        if (e == cudaErrorMemoryAllocation) {   // (taken by others since, or fragmented)
+            cudaGetLastError();
+            if (pairf_mem) cudaFree(pairf_mem);
+            pairf_mem = nullptr;
+            return PARM_OK;
+        }
+        CUDA_TRY(e);
         c.pairf = pairf_mem;
         c.slots = static_cast<uint32_t*>(slots_mem);
         if (unbuilt) return PARM_OK;
