@@ -797,21 +797,22 @@ __global__ void __launch_bounds__(SORT_WARPS * 32) k_sort_lists(DevCtx c, int al
         sysw[w] = go ? s : 0xFFFFFFFFu;
     }
     __syncthreads();
-    // warp 0: one atomic per run of lists of one system
-    if (w != 0 || lane >= SORT_WARPS) return;
-    const uint32_t my = sysw[lane];
-    if (my == 0xFFFFFFFFu) return;
+    // warp 0, all of its lanes: one atomic per system with lists in the CTA
+    if (w != 0) return;
+    constexpr uint32_t NONE = 0xFFFFFFFFu;
+    const uint32_t my = lane < SORT_WARPS ? sysw[lane] : NONE;
     uint32_t before = 0u, total = 0u, leader = lane;
     for (uint32_t k = 0; k < SORT_WARPS; k++) {
-        if (sysw[k] != my) continue;
-        leader = min(leader, k);
-        total += low[k];
-        if (k < lane) before += low[k];
+        if (sysw[k] == my) {
+            leader = min(leader, k);
+            total += low[k];
+            if (k < lane) before += low[k];
+        }
     }
-    const uint32_t live = __activemask();
     uint32_t first = 0u;
-    if (leader == lane) first = atomicAdd(&c.half_cnt[my], total);
-    first = __shfl_sync(live, first, leader);
+    if (my != NONE && leader == lane) first = atomicAdd(&c.half_cnt[my], total);
+    first = __shfl_sync(0xFFFFFFFFu, first, leader);
+    if (my == NONE) return;
     const uint32_t me = blockIdx.x * SORT_WARPS + lane;
     // lists cut at their capacity (reported) need not be symmetric: never past the system's slots
     const bool fits = (size_t)first + before + low[lane] <= (size_t)c.sys[my].natoms * c.maxnb / 2;

@@ -100,3 +100,25 @@ def test_cluster_in_a_large_box(n, ndim):
     st, ref = g.get_atoms(), o.get_state()
     assert np.array_equal(st["f"][:n], ref["f"]) and not st["f"][n:].any()
     assert np.array_equal(st["a"][:n], ref["a"])
+
+
+def test_slots_of_tiny_systems():
+    """Eight lists of a CTA out of up to eight systems, of which some rebuild and others do not."""
+    sizes = [1, 2, 3, 1, 5, 8, 9, 1, 1, 1, 7, 16, 17, 2, 30, 1, 4, 6]
+    ws = [W.small_random(n=n, ndim=3, kind=0, seed=k, phi=0.2, skin=0.3) for k, n in enumerate(sizes)]
+    w = W.Workload("t", 3, sizes, np.concatenate([k.L for k in ws]), np.concatenate([k.x for k in ws]),
+                   np.concatenate([k.v for k in ws]), np.concatenate([k.m for k in ws]), 0,
+                   np.concatenate([k.params for k in ws]), 0.3)
+    out = []
+    for keep in (True, False):
+        g = make_gpu(w)
+        g.debug_pair_slots(keep)
+        g.nlist_update(False)
+        g.set_forces(True)
+        for q in range(3):
+            g.set_active([(k + q) % 3 != 0 for k in range(len(sizes))])
+            g.damped(1e-4, 5.0, 30)
+        out.append((g.get_atoms(), g.which()))
+    for k in ("x", "v", "a", "f"):
+        assert np.array_equal(out[0][0][k], out[1][0][k])
+    assert np.array_equal(out[0][1], out[1][1]) and out[0][1].max() > 1
