@@ -234,70 +234,76 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_one(DevCtx c) {
     }
 }
 
+// the entries of atom o of the old order, at place k of the new one in bucket b
+template <int ND>
+__device__ __forceinline__ void move_atom(const DevCtx& c, uint32_t o, uint32_t k, uint32_t rk, uint32_t b) {
+    using V = typename DVec<ND>::T;
+    static_cast<V*>(c.x2)[k] = static_cast<const V*>(c.x)[o];
+    static_cast<V*>(c.v2)[k] = static_cast<const V*>(c.v)[o];
+    static_cast<V*>(c.a2)[k] = static_cast<const V*>(c.a)[o];
+    if (c.prec != PREC_MIXED) static_cast<V*>(c.f2)[k] = static_cast<const V*>(c.f)[o];   // FP64 forces: FP64 path only
+    c.f32b[k] = c.f32[o];
+    // arrays whose entries are all equal are left as they are (copy back too)
+    if (*c.m_mixed) {
+        c.m2[k] = c.m[o];
+        c.invm32b[k] = c.invm32[o];
+    }
+    if (!c.same_prm) {
+        c.prm2[k] = c.prm[o];
+        c.prm32b[k] = c.prm32[o];
+        c.diam2[k] = c.diam[o];
+    }
+    c.rank2[k] = rk;
+    c.orig2[k] = c.orig[o];
+    c.bucket2[k] = b;
+}
+
+// Members into their cells, in any order; non-members, whose order nm_rank
+// gives, with all their entries to their place at the system's end, a thread
+// each (rebuild with 399,000 of 400,000 atoms outside the list: 0.91 ms; with a
+// warp for all of them 55.9 ms).
+template <int ND>
 __global__ void k_scatter(DevCtx c) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     uint32_t s = c.atom_sys[i];
     if (!c.flag[s]) return;
-    c.perm[c.cell_start[c.bucket[i]] + c.cslot[i]] = i;
+    const uint32_t b = c.bucket[i], k = c.cell_start[b] + c.cslot[i];
+    if (b - c.bucket_off[s] == c.sys[s].ncell) move_atom<ND>(c, i, k, NOT_MEMBER, b);
+    else c.perm[k] = i;
 }
 
-// Permutation of the atoms' arrays into their new order, one warp per cell: the
-// order inside a cell is ascending neighbour-list rank, so each lane holds one
-// of the cell's scattered atoms (one of every 32 in larger cells: few-cell boxes
-// put tens to hundreds of atoms in one), counts the atoms of the cell ranked
-// before it, 32 at a time, and moves its atom's entries to that place.  (Sorting
-// large cells serially on lane 0 took 164 us on 48 packings of 64 to 4096
-// spheres; sort and move as two kernels cost a batch of 48 replicas, one of
+// Permutation of the members' arrays into their new order: the order inside a
+// cell is ascending neighbour-list rank, so each lane of a warp holds one of
+// the cell's scattered atoms, counts the atoms of the cell ranked before it, 32
+// at a time, and moves its atom's entries to that place.  `parts` warps share a
+// cell, each taking every parts-th 32 of its atoms: one for cells of up to 32
+// atoms, more where few-cell boxes put hundreds in one (rebuild of 1000 / 3000
+// atoms in one cell: 0.31 / 2.0 ms; with one warp for it 0.83 / 6.5 ms).
+// (Sorting large cells serially on lane 0 took 164 us on 48 packings of 64 to
+// 4096 spheres; sort and move as two kernels cost a batch of 48 replicas, one of
 // which rebuilds nearly every step, 1 % of the step.)
 template <int ND>
-__global__ void k_sortgather(DevCtx c) {
-    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+__global__ void k_sortgather(DevCtx c, uint32_t parts) {
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint32_t b = w / parts, part = w - b * parts;
     if (b >= c.nbucket) return;   // uniform in the warp
     const uint32_t s = c.bucket_sys[b];
     if (!c.flag[s]) return;
-    const uint32_t local = b - c.bucket_off[s], ncell = c.sys[s].ncell;
-    if (local > ncell) return;   // (past a grid that has shrunk)
-    const bool members = local < ncell;   // the bucket after the cells: non-members, placed by nm_rank
-    const uint32_t lo = c.cell_start[b];
-    const uint32_t cnt = (members ? c.cell_start[b + 1] : c.sys[s].atom_off + c.sys[s].natoms) - lo;
-    using V = typename DVec<ND>::T;
-    const bool masses = *c.m_mixed != 0u;
-    for (uint32_t q0 = 0; q0 < cnt; q0 += 32u) {
-        const uint32_t q = q0 + lane;
-        const bool on = q < cnt;
-        const uint32_t o = on ? c.perm[lo + q] : 0u;
+    if (b - c.bucket_off[s] >= c.sys[s].ncell) return;   // non-members; past a grid that has shrunk
+    const uint32_t lo = c.cell_start[b], cnt = c.cell_start[b + 1] - lo;
+    for (uint32_t q0 = 32u * part; q0 < cnt; q0 += 32u * parts) {
+        const bool on = q0 + lane < cnt;
+        const uint32_t o = on ? c.perm[lo + q0 + lane] : 0u;
         const uint32_t rk = on ? c.rank[o] : 0xFFFFFFFFu;
-        uint32_t pos = q;
-        if (members && cnt > 1u) {
-            pos = 0u;
-            for (uint32_t t0 = 0; t0 < cnt; t0 += 32u) {
-                const uint32_t m = min(32u, cnt - t0);
-                uint32_t kt = rk;
-                if (t0 != q0) kt = lane < m ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
-                for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j) < rk ? 1u : 0u;
-            }
+        uint32_t pos = 0u;
+        for (uint32_t t0 = 0; t0 < cnt; t0 += 32u) {
+            const uint32_t m = min(32u, cnt - t0);
+            uint32_t kt = rk;
+            if (t0 != q0) kt = lane < m ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
+            for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j) < rk ? 1u : 0u;
         }
-        if (!on) continue;
-        const uint32_t k = lo + pos;
-        static_cast<V*>(c.x2)[k] = static_cast<const V*>(c.x)[o];
-        static_cast<V*>(c.v2)[k] = static_cast<const V*>(c.v)[o];
-        static_cast<V*>(c.a2)[k] = static_cast<const V*>(c.a)[o];
-        if (c.prec != PREC_MIXED) static_cast<V*>(c.f2)[k] = static_cast<const V*>(c.f)[o];   // FP64 forces: FP64 path only
-        c.f32b[k] = c.f32[o];
-        // arrays whose entries are all equal are left as they are (copy back too)
-        if (masses) {
-            c.m2[k] = c.m[o];
-            c.invm32b[k] = c.invm32[o];
-        }
-        if (!c.same_prm) {
-            c.prm2[k] = c.prm[o];
-            c.prm32b[k] = c.prm32[o];
-            c.diam2[k] = c.diam[o];
-        }
-        c.rank2[k] = rk;
-        c.orig2[k] = c.orig[o];
-        c.bucket2[k] = b;
+        if (on) move_atom<ND>(c, o, lo + pos, rk, b);
     }
 }
 
@@ -939,10 +945,18 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
         k_scan_blocks<<<nblk, SCAN_THREADS, 0, s>>>(c);
         k_scan_write<<<nblk, SCAN_THREADS, 0, s>>>(c);
     }
-    k_scatter<<<ga, BLOCK, 0, s>>>(c);
-    const unsigned gw = (unsigned)(((size_t)c.nbucket * 32 + BLOCK - 1) / BLOCK);   // a warp per bucket
-    if (c.nd == 3) k_sortgather<3><<<gw, BLOCK, 0, s>>>(c);
-    else k_sortgather<2><<<gw, BLOCK, 0, s>>>(c);
+    // warps per cell: one per 32 atoms of the system of the fullest cells, at most
+    // eight where other systems' cells alone give every SM its warps
+    const uint32_t share = std::min((c.cell_mean + 31u) / 32u, std::max(8u, 152u * 32u / c.nbucket));
+    const uint32_t sort_warps = std::max(share, 1u);
+    const unsigned gw = (unsigned)(((size_t)c.nbucket * sort_warps * 32 + BLOCK - 1) / BLOCK);
+    if (c.nd == 3) {
+        k_scatter<3><<<ga, BLOCK, 0, s>>>(c);
+        k_sortgather<3><<<gw, BLOCK, 0, s>>>(c, sort_warps);
+    } else {
+        k_scatter<2><<<ga, BLOCK, 0, s>>>(c);
+        k_sortgather<2><<<gw, BLOCK, 0, s>>>(c, sort_warps);
+    }
     if (c.staged) {
         if (c.nd == 3) {
             k_copyback<3><<<ga, BLOCK, 0, s>>>(c);

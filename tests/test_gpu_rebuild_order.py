@@ -1,0 +1,83 @@
+"""The permutation of a rebuild where it has large groups to move: atoms outside the neighbour list, and cells of
+hundreds of atoms, each with a time that a single warp for the group would miss by far."""
+import time
+
+import numpy as np
+import pytest
+
+from helpers import make_gpu, make_oracle
+from parm_gb300 import workloads as W
+from parm_gb300.capi import NOT_MEMBER
+
+pytestmark = pytest.mark.gpu
+
+
+def _fastest_rebuild(g, times=5):
+    best = 1e9
+    for _ in range(times):
+        t = time.perf_counter()
+        g.nlist_update(True)
+        best = min(best, time.perf_counter() - t)
+    return best
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("masses", [False, True])
+def test_few_members_among_many_atoms(ndim, masses):
+    """Two systems with every seventh and every second atom in the list: the members move as they do alone, bit for bit,
+    the others on their own."""
+    ws = [W.small_random(n=n, ndim=ndim, kind=1, seed=n, phi=2.0, skin=0.2) for n in (3001, 500)]
+    m = np.concatenate([k.m for k in ws]) if masses else np.full(3501, 2.0)
+    w = W.Workload("nm", ndim, [k.n for k in ws], np.concatenate([k.L for k in ws]), np.concatenate([k.x for k in ws]),
+                   np.concatenate([k.v for k in ws]), m, 1, np.concatenate([k.params for k in ws]), 0.2)
+    member = np.concatenate([np.arange(3001) % 7 == 3, np.arange(500) % 2 == 1])
+    rng = np.random.default_rng(ndim)
+    rank = np.full(w.n, NOT_MEMBER, dtype=np.uint32)
+    parts = np.split(np.arange(w.n), [3001])
+    for p in parts:
+        k = p[member[p]]
+        rank[k] = rng.permutation(len(k))
+    g = make_gpu(w, rank=rank)
+    alone = W.Workload("m", ndim, [int(member[p].sum()) for p in parts], w.L, w.x[member], w.v[member], m[member], 1,
+                       w.params[member], 0.2)
+    h = make_gpu(alone, rank=rank[member])
+    for s in (g, h):
+        s.nlist_update(False)
+        s.set_forces(True)
+        s.verlet(0.01, 60)
+    assert g.which().min() > 2 and np.array_equal(g.which(), h.which())
+    a, b = g.get_atoms(), h.get_atoms()
+    for k in ("x", "v", "a", "f"):
+        assert np.array_equal(a[k][member], b[k])
+    assert not a["f"][~member].any()
+    assert np.array_equal(a["v"][~member], w.v[~member]) and np.array_equal(a["m"], m)
+    x = w.x[~member] + 60 * 0.01 * w.v[~member]
+    assert np.abs(a["x"][~member] - x).max() < 1e-11
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_rebuild_time_with_few_members(precision):
+    """400,000 atoms, 1000 of them in the list, against all of them in it: less to do, so not longer (a warp for all the
+    others takes tens of times as long)."""
+    n = 400_000
+    w = W.soft_disks(n=n, phi=0.5)
+    rank = np.full(n, NOT_MEMBER, dtype=np.uint32)
+    rank[:1000] = np.arange(1000)
+    t = [_fastest_rebuild(make_gpu(w, precision=precision, rank=r)) for r in (rank, None)]
+    print("few / all members: %.0f / %.0f us" % (1e6 * t[0], 1e6 * t[1]))
+    assert t[0] < 2.0 * t[1]
+
+
+def test_one_cell_of_hundreds_in_order():
+    """700 atoms in a single cell in a shuffled list order: lists and forces as the oracle's, bit for bit."""
+    w = W.small_random(n=700, ndim=3, kind=0, seed=8, phi=0.62, skin=0.4)
+    order = np.random.default_rng(8).permutation(w.n)
+    rank = np.empty(w.n, dtype=np.uint32)
+    rank[order] = np.arange(w.n)
+    g, o = make_gpu(w, rank=rank), make_oracle(w, order=[int(i) for i in order])
+    g.nlist_update(True)
+    o.nl_update(True)
+    assert np.array_equal(g.pairs(), o.pairs())
+    g.set_forces(True)
+    o.set_forces(True)
+    assert np.array_equal(g.get_atoms()["f"], o.get_state()["f"])
