@@ -274,34 +274,45 @@ __global__ void k_scatter(DevCtx c) {
 }
 
 // Permutation of the members' arrays into their new order: the order inside a
-// cell is ascending neighbour-list rank, so each lane of a warp holds one of
-// the cell's scattered atoms, counts the atoms of the cell ranked before it, 32
-// at a time, and moves its atom's entries to that place.  `parts` warps share a
-// cell, each taking every parts-th 32 of its atoms: one for cells of up to 32
-// atoms, more where few-cell boxes put hundreds in one (rebuild of 1000 / 3000
-// atoms in one cell: 0.31 / 2.0 ms; with one warp for it 0.83 / 6.5 ms).
-// (Sorting large cells serially on lane 0 took 164 us on 48 packings of 64 to
-// 4096 spheres; sort and move as two kernels cost a batch of 48 replicas, one of
-// which rebuilds nearly every step, 1 % of the step.)
-template <int ND>
+// cell is ascending neighbour-list rank, so each of LANES lanes holds one of
+// the cell's scattered atoms, counts the atoms of the cell ranked before it,
+// LANES at a time, and moves its atom's entries to that place.  Bound by those
+// moves' memory latency, so few lanes may idle: with a warp per cell / eight /
+// four lanes, 400,000 disks in cells of one 219 / 74 / 45 us, of two 124 / 40 /
+// 35 us, 48 WCA replicas (427,107 atoms, two a cell) 98 / 34 / 25 us, 65,536
+// disks 26.8 / 10.9 / 13.5 us, 20,011 disks 14.7 / 9.4 / 11.9 us; 343,000 LJ
+// atoms (17 a cell) 18.9 / 26.2 / 44.1 us; 48 packings of 64 to 4096 spheres,
+// one cell of 86 among 10,693: a warp / sixteen / eight lanes 25.2 / 21.4 / 32.0
+// us.  `parts` groups share a cell, each taking every parts-th
+// LANES of its atoms: one for cells of up to 32 atoms, more where few-cell boxes
+// put hundreds in one (rebuild of 1000 / 3000 atoms in one cell: 0.31 / 2.0 ms;
+// with one warp for it 0.83 / 6.5 ms).  (Sort and move as two kernels cost a
+// batch of 48 replicas, one of which rebuilds nearly every step, 1 % of the
+// step.)
+template <int ND, uint32_t LANES>
 __global__ void k_sortgather(DevCtx c, uint32_t parts) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / LANES, lane = threadIdx.x % LANES;
     const uint32_t b = w / parts, part = w - b * parts;
-    if (b >= c.nbucket) return;   // uniform in the warp
-    const uint32_t s = c.bucket_sys[b];
-    if (!c.flag[s]) return;
-    if (b - c.bucket_off[s] >= c.sys[s].ncell) return;   // non-members; past a grid that has shrunk
-    const uint32_t lo = c.cell_start[b], cnt = c.cell_start[b + 1] - lo;
-    for (uint32_t q0 = 32u * part; q0 < cnt; q0 += 32u * parts) {
+    uint32_t lo = 0u, cnt = 0u;
+    if (b < c.nbucket) {
+        const uint32_t s = c.bucket_sys[b];
+        // (not: non-members, buckets past a grid that has shrunk)
+        if (c.flag[s] && b - c.bucket_off[s] < c.sys[s].ncell) {
+            lo = c.cell_start[b];
+            cnt = c.cell_start[b + 1] - lo;
+        }
+    }
+    const uint32_t most = LANES == 32u ? cnt : __reduce_max_sync(0xFFFFFFFFu, cnt);   // uniform in the warp
+    for (uint32_t q0 = LANES * part; q0 < most; q0 += LANES * parts) {
         const bool on = q0 + lane < cnt;
         const uint32_t o = on ? c.perm[lo + q0 + lane] : 0u;
         const uint32_t rk = on ? c.rank[o] : 0xFFFFFFFFu;
         uint32_t pos = 0u;
-        for (uint32_t t0 = 0; t0 < cnt; t0 += 32u) {
-            const uint32_t m = min(32u, cnt - t0);
+        for (uint32_t t0 = 0; t0 < most; t0 += LANES) {
             uint32_t kt = rk;
-            if (t0 != q0) kt = lane < m ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
-            for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j) < rk ? 1u : 0u;
+            if (t0 != q0) kt = t0 + lane < cnt ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
+            const uint32_t m = min(LANES, most - t0);
+            for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j, LANES) < rk ? 1u : 0u;
         }
         if (on) move_atom<ND>(c, o, lo + pos, rk, b);
     }
@@ -935,6 +946,22 @@ void launch_arm(const DevCtx& c, cudaStream_t s, int count_step, int use_cond,
     k_arm<<<1, threads, 0, s>>>(c, count_step, use_cond, (cudaGraphConditionalHandle)handle);
 }
 
+template <int ND>
+static void sortgather(const DevCtx& c, cudaStream_t s) {
+    // warps per cell: one per 32 atoms of the system of the fullest cells, at most
+    // eight where other systems' cells alone give every SM its warps
+    const uint32_t parts = std::max(1u, std::min((c.cell_mean + 31u) / 32u, std::max(8u, 152u * 32u / c.nbucket)));
+    const auto grid = [&](uint32_t lanes) { return (unsigned)(((size_t)c.nbucket * parts * lanes + BLOCK - 1) / BLOCK); };
+    // lanes per cell: a warp where cells hold more than eight atoms, else eight
+    // lanes, or four where eight for each cell would fill the SMs more than once;
+    // sixteen where a few large cells among them would otherwise be what all wait for
+    const uint32_t mean = c.n / c.nbucket + 1u;
+    if (mean > 8u) k_sortgather<ND, 32><<<grid(32), BLOCK, 0, s>>>(c, parts);
+    else if (c.cell_mean > 32u && c.nbucket < 20000u) k_sortgather<ND, 16><<<grid(16), BLOCK, 0, s>>>(c, parts);
+    else if (mean > 4u || c.nbucket < 40000u) k_sortgather<ND, 8><<<grid(8), BLOCK, 0, s>>>(c, parts);
+    else k_sortgather<ND, 4><<<grid(4), BLOCK, 0, s>>>(c, parts);
+}
+
 void launch_rebuild(const DevCtx& c, cudaStream_t s) {
     unsigned ga = grid_for(c.n);
     if (c.nd == 3) k_bin<3><<<ga, BLOCK, 0, s>>>(c); else k_bin<2><<<ga, BLOCK, 0, s>>>(c);
@@ -945,17 +972,12 @@ void launch_rebuild(const DevCtx& c, cudaStream_t s) {
         k_scan_blocks<<<nblk, SCAN_THREADS, 0, s>>>(c);
         k_scan_write<<<nblk, SCAN_THREADS, 0, s>>>(c);
     }
-    // warps per cell: one per 32 atoms of the system of the fullest cells, at most
-    // eight where other systems' cells alone give every SM its warps
-    const uint32_t share = std::min((c.cell_mean + 31u) / 32u, std::max(8u, 152u * 32u / c.nbucket));
-    const uint32_t sort_warps = std::max(share, 1u);
-    const unsigned gw = (unsigned)(((size_t)c.nbucket * sort_warps * 32 + BLOCK - 1) / BLOCK);
     if (c.nd == 3) {
         k_scatter<3><<<ga, BLOCK, 0, s>>>(c);
-        k_sortgather<3><<<gw, BLOCK, 0, s>>>(c, sort_warps);
+        sortgather<3>(c, s);
     } else {
         k_scatter<2><<<ga, BLOCK, 0, s>>>(c);
-        k_sortgather<2><<<gw, BLOCK, 0, s>>>(c, sort_warps);
+        sortgather<2>(c, s);
     }
     if (c.staged) {
         if (c.nd == 3) {

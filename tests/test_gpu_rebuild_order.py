@@ -81,3 +81,23 @@ def test_one_cell_of_hundreds_in_order():
     g.set_forces(True)
     o.set_forces(True)
     assert np.array_equal(g.get_atoms()["f"], o.get_state()["f"])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("ndim,n,side", [(2, 9001, 1.0), (2, 30011, 0.5), (2, 60007, 1.1), (3, 20011, 0.75),
+                                         (3, 50021, 1.4)])
+def test_sparse_cells(precision, ndim, n, side):
+    """One to seven atoms a cell in the mean: no atom is lost or doubled, the pairs are those of a tree."""
+    cKDTree = pytest.importorskip("scipy.spatial").cKDTree
+    rl = 1.3
+    L = side * n ** (1.0 / ndim)
+    x = np.random.default_rng(n).uniform(0, L, size=(n, ndim))
+    m = 1.0 + np.arange(n) % 3
+    w = W.Workload("s", ndim, [n], np.full((1, ndim), L), x, x * 0.5, m, 1, np.tile([1.0, 1.0, 2.0], (n, 1)), rl - 1.0)
+    g = make_gpu(w, precision=precision)
+    for _ in range(3):
+        g.nlist_update(True)
+    st = g.get_atoms()
+    assert np.array_equal(st["x"], x) and np.array_equal(st["v"], w.v) and np.array_equal(st["m"], m)
+    tree = cKDTree(np.mod(x, L), boxsize=L)
+    assert int(g.numpairs()[0]) == len(tree.query_pairs(rl, output_type="ndarray"))
