@@ -336,7 +336,8 @@ struct parm_system {
         // from where its CTAs of 16 atoms fill the SMs (force kernel, a warp per
         // list / a thread per entry: 16.4 / 17.4 us on 5003 spheres, 34.5 / 30.1 on
         // 20,000, 54.8 / 42.9 on 65,536 disks, 290 / 179 on 48 WCA replicas)
-        c.short_lists = n >= 8192 && mean_list() <= 32.0 ? 1u : 0u;
+        c.list_mean = (uint32_t)std::ceil(std::min(1e6, mean_list()));
+        c.short_lists = n >= 8192 && c.list_mean <= 32u ? 1u : 0u;
         std::vector<int> newnc;
         for (uint32_t s2 = 0; s2 < nsys; s2++)
             for (int d = 0; d < 3; d++) newnc.push_back(sys[s2].nc[d]);

@@ -749,77 +749,135 @@ __global__ void __launch_bounds__(TILE_ATOMS) k_tile(DevCtx c, int all) {
 // FP64 path: order each list by neighbour-list rank, which reproduces the
 // reference's summation order (pairs (i, j<i) in ascending j, then (i'>i, i)
 // in ascending i').
-// One warp per list: the ranks are staged in shared memory and every lane
-// counts, for its entries (three of a list of up to 96), the ranks below them;
-// that count is the entry's place.  A thread that insertion-sorted its own
-// list kept both arrays in local memory and moved ~n^2/4 entries there:
-// 268 -> 7.5 us at 1000 LJ atoms, 427 -> 31 us at 29,667, 7.57 -> 0.89 ms at
-// 1,048,576 (~72 entries; one GB300).
+// The place of an entry is the number of entries with ranks below its own.
 // Entries of smaller rank than the atom's come first; with pair slots
 // (c.pairf), the CTA hands each list as many consecutive slots of its system.
 constexpr uint32_t SORT_CAP = 256;   // longer lists are reported, not sorted
 constexpr uint32_t SORT_WARPS = 8, SORT_SLOTS = 3;
+
+// One list by one warp: the ranks are staged in shared memory and every lane
+// counts for its entries (three of a list of up to 96).  A thread that
+// insertion-sorted its own list kept both arrays in local memory and moved
+// ~n^2/4 entries there: 268 -> 7.5 us at 1000 LJ atoms, 427 -> 31 us at 29,667,
+// 7.57 -> 0.89 ms at 1,048,576 (~72 entries; one GB300).  All arguments are
+// uniform in the warp; returns the number of entries ranked before the atom.
+__device__ __forceinline__ uint32_t sort_list(const DevCtx& c, uint32_t i, uint32_t cnt, uint32_t lane, uint32_t* rk,
+                                              uint32_t* jv) {
+    if (!cnt) return 0u;
+    uint32_t* row = c.nbr + (size_t)i * c.maxnb;
+    const uint32_t ri = c.rank[i];
+    const uint32_t padded = (cnt + 3u) & ~3u;   // <= SORT_CAP
+    uint32_t below = 0u;
+    for (uint32_t q = lane; q < padded; q += 32u) {
+        const uint32_t j = q < cnt ? row[q] : 0u;
+        const uint32_t r = q < cnt ? c.rank[j] : 0xFFFFFFFFu;
+        jv[q] = j;
+        rk[q] = r;
+        below += r < ri ? 1u : 0u;
+    }
+    below = __reduce_add_sync(0xFFFFFFFFu, below);
+    __syncwarp();
+    for (uint32_t q0 = 0; q0 < cnt; q0 += 32u * SORT_SLOTS) {
+        uint32_t mine[SORT_SLOTS], pos[SORT_SLOTS];
+#pragma unroll
+        for (uint32_t u = 0; u < SORT_SLOTS; u++) {
+            const uint32_t q = q0 + lane + 32u * u;
+            mine[u] = q < cnt ? rk[q] : 0u;
+            pos[u] = 0u;
+        }
+#pragma unroll 2
+        for (uint32_t t = 0; t < padded; t += 4u) {
+            const uint4 K = *reinterpret_cast<const uint4*>(&rk[t]);
+#pragma unroll
+            for (uint32_t u = 0; u < SORT_SLOTS; u++)
+                pos[u] += (K.x < mine[u] ? 1u : 0u) + (K.y < mine[u] ? 1u : 0u) + (K.z < mine[u] ? 1u : 0u) +
+                          (K.w < mine[u] ? 1u : 0u);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < SORT_SLOTS; u++) {
+            const uint32_t q = q0 + lane + 32u * u;
+            if (q < cnt) row[pos[u]] = jv[q];
+        }
+    }
+    return below;
+}
+
+// LANES lanes per list.  Eight, for lists of a few entries: where none of a
+// warp's four lists is longer than four entries a lane, entries and ranks stay
+// in registers; else the warp takes its lists one after the other.  With a warp
+// per list / eight lanes: 400,000 disks with lists of 2.3 / 10 / 23 entries 123
+// / 28, 140 / 37, 172 / 72 us, 65,536 disks (5 entries) 24 / 8.5 us, 48 WCA
+// replicas (7) 143 / 33 us, 5003 spheres 4.9 / 5.0 us; 1000 and 29,667 LJ atoms
+// (80) 6.4 / 14 and 34 / 37 us.
+template <uint32_t LANES>
 __global__ void __launch_bounds__(SORT_WARPS * 32) k_sort_lists(DevCtx c, int all) {
+    constexpr uint32_t LISTS = SORT_WARPS * 32u / LANES, GROUPS = 32u / LANES, EACH = 4;
+    static_assert(LISTS <= 32, "one warp hands out the slots");
     __shared__ __align__(16) uint32_t rk[SORT_WARPS][SORT_CAP], jv[SORT_WARPS][SORT_CAP];
-    __shared__ uint32_t low[SORT_WARPS], sysw[SORT_WARPS];
+    __shared__ uint32_t low[LISTS], sysw[LISTS];
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t i = blockIdx.x * SORT_WARPS + w;   // uniform in the warp from here
+    const uint32_t gl = lane % LANES, group = lane / LANES, list = threadIdx.x / LANES;
+    const uint32_t i = blockIdx.x * LISTS + list;   // uniform in the group from here
     const uint32_t s = i < c.n ? c.atom_sys[i] : 0u;
     const bool go = i < c.n && (all || c.flag[s]);
     uint32_t cnt = go ? min(c.nnb[i], c.maxnb) : 0u;
     if (cnt > SORT_CAP) {
-        if (lane == 0) atomicOr(c.status, ST_SORT_CAP);
+        if (gl == 0) atomicOr(c.status, ST_SORT_CAP);
         cnt = 0u;
     }
     uint32_t below = 0u;
-    if (cnt) {
+    const uint32_t most = LANES == 32u ? cnt : __reduce_max_sync(0xFFFFFFFFu, cnt);   // uniform in the warp
+    if (LANES < 32u && most <= EACH * LANES) {
         uint32_t* row = c.nbr + (size_t)i * c.maxnb;
-        const uint32_t ri = c.rank[i];
-        const uint32_t padded = (cnt + 3u) & ~3u;   // <= SORT_CAP
-        for (uint32_t q = lane; q < padded; q += 32u) {
-            const uint32_t j = q < cnt ? row[q] : 0u;
-            const uint32_t r = q < cnt ? c.rank[j] : 0xFFFFFFFFu;
-            jv[w][q] = j;
-            rk[w][q] = r;
-            below += r < ri ? 1u : 0u;
+        const uint32_t ri = cnt ? c.rank[i] : 0u;
+        uint32_t j[EACH], r[EACH], pos[EACH];
+#pragma unroll
+        for (uint32_t u = 0; u < EACH; u++) {
+            const uint32_t q = gl + LANES * u;
+            j[u] = q < cnt ? row[q] : 0u;
+            pos[u] = 0u;
         }
-        below = __reduce_add_sync(0xFFFFFFFFu, below);
-        __syncwarp();
-        for (uint32_t q0 = 0; q0 < cnt; q0 += 32u * SORT_SLOTS) {
-            uint32_t mine[SORT_SLOTS], pos[SORT_SLOTS];
 #pragma unroll
-            for (uint32_t u = 0; u < SORT_SLOTS; u++) {
-                const uint32_t q = q0 + lane + 32u * u;
-                mine[u] = q < cnt ? rk[w][q] : 0u;
-                pos[u] = 0u;
-            }
-#pragma unroll 2
-            for (uint32_t t = 0; t < padded; t += 4u) {
-                const uint4 K = *reinterpret_cast<const uint4*>(&rk[w][t]);
+        for (uint32_t u = 0; u < EACH; u++) {
+            r[u] = gl + LANES * u < cnt ? c.rank[j[u]] : 0xFFFFFFFFu;
+            below += r[u] < ri ? 1u : 0u;
+        }
 #pragma unroll
-                for (uint32_t u = 0; u < SORT_SLOTS; u++)
-                    pos[u] += (K.x < mine[u] ? 1u : 0u) + (K.y < mine[u] ? 1u : 0u) + (K.z < mine[u] ? 1u : 0u) +
-                              (K.w < mine[u] ? 1u : 0u);
-            }
+        for (uint32_t v = 0; v < EACH; v++) {
+            if (LANES * v >= most) break;
+            for (uint32_t t = 0; t < min(LANES, most - LANES * v); t++) {
+                const uint32_t k = __shfl_sync(0xFFFFFFFFu, r[v], t, LANES);
 #pragma unroll
-            for (uint32_t u = 0; u < SORT_SLOTS; u++) {
-                const uint32_t q = q0 + lane + 32u * u;
-                if (q < cnt) row[pos[u]] = jv[w][q];
+                for (uint32_t u = 0; u < EACH; u++) pos[u] += k < r[u] ? 1u : 0u;
             }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < EACH; u++)
+            if (gl + LANES * u < cnt) row[pos[u]] = j[u];
+#pragma unroll
+        for (uint32_t o = LANES / 2; o; o >>= 1) below += __shfl_xor_sync(0xFFFFFFFFu, below, o, LANES);
+    } else if (LANES == 32u) {
+        below = sort_list(c, i, cnt, lane, rk[w], jv[w]);
+    } else {
+        for (uint32_t g = 0; g < GROUPS; g++) {
+            const uint32_t ig = __shfl_sync(0xFFFFFFFFu, i, g * LANES), cg = __shfl_sync(0xFFFFFFFFu, cnt, g * LANES);
+            const uint32_t bg = sort_list(c, ig, cg, lane, rk[w], jv[w]);
+            __syncwarp();
+            if (group == g) below = bg;
         }
     }
     if (!c.pairf) return;
-    if (lane == 0) {
-        low[w] = below;
-        sysw[w] = go ? s : 0xFFFFFFFFu;
+    if (gl == 0) {
+        low[list] = below;
+        sysw[list] = go ? s : 0xFFFFFFFFu;
     }
     __syncthreads();
     // warp 0, all of its lanes: one atomic per system with lists in the CTA
     if (w != 0) return;
     constexpr uint32_t NONE = 0xFFFFFFFFu;
-    const uint32_t my = lane < SORT_WARPS ? sysw[lane] : NONE;
+    const uint32_t my = lane < LISTS ? sysw[lane] : NONE;
     uint32_t before = 0u, total = 0u, leader = lane;
-    for (uint32_t k = 0; k < SORT_WARPS; k++) {
+    for (uint32_t k = 0; k < LISTS; k++) {
         if (sysw[k] == my) {
             leader = min(leader, k);
             total += low[k];
@@ -830,7 +888,7 @@ __global__ void __launch_bounds__(SORT_WARPS * 32) k_sort_lists(DevCtx c, int al
     if (my != NONE && leader == lane) first = atomicAdd(&c.half_cnt[my], total);
     first = __shfl_sync(0xFFFFFFFFu, first, leader);
     if (my == NONE) return;
-    const uint32_t me = blockIdx.x * SORT_WARPS + lane;
+    const uint32_t me = blockIdx.x * LISTS + lane;
     // lists cut at their capacity (reported) need not be symmetric: never past the system's slots
     const bool fits = (size_t)first + before + low[lane] <= (size_t)c.sys[my].natoms * c.maxnb / 2;
     c.half_n[me] = fits ? low[lane] : 0u;
@@ -860,7 +918,8 @@ __global__ void __launch_bounds__(BLOCK) k_slots(DevCtx c, int all) {
 
 void launch_half(const DevCtx& c, cudaStream_t s, int all) {
     if (all && c.pairf) cudaMemsetAsync(c.half_cnt, 0, 4 * (size_t)c.nsys, s);
-    k_sort_lists<<<grid_for(c.n, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(c, all);
+    if (c.list_mean <= 24u) k_sort_lists<8><<<grid_for(c.n, SORT_WARPS * 4), SORT_WARPS * 32, 0, s>>>(c, all);
+    else k_sort_lists<32><<<grid_for(c.n, SORT_WARPS), SORT_WARPS * 32, 0, s>>>(c, all);
     if (c.pairf) k_slots<<<grid_for(c.n, BLOCK / 32), BLOCK, 0, s>>>(c, all);
 }
 

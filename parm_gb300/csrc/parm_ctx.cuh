@@ -114,6 +114,7 @@ struct DevCtx {
     // neighbour list
     uint32_t* nbr;
     uint32_t* nnb;
+    uint32_t list_mean;    // expected entries per list, in the densest system
     uint32_t short_lists;  // FP64 path: lists of about 32 entries or fewer (k_force64s)
     // FP64 path: each listed pair's force, computed once for its first atom (the
     // one of higher rank) in slot half_base[first] + entry; null: not kept
