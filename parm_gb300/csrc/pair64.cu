@@ -962,13 +962,13 @@ __global__ void __launch_bounds__(BLOCK) k_eval64(DevCtx c, int what) {
                                        __float_as_uint(c.prm32[j].x), uni);
             else
                 pc = combine<KIND>(Pi, c.prm[j], uni);
-            pc.set_derived();
             if (what == EV_ENERGY || what == EV_CONTACTS || what == EV_OVERLAPS) {
                 double e = pair_energy<KIND>(pc, dsq, uni);
                 if (what == EV_ENERGY) acc[0] = acc[0] + e;
                 else if (what == EV_CONTACTS) acc[0] += (e != 0.0) ? 1.0 : 0.0;
                 else acc[0] += (e > 0.0) ? 1.0 : 0.0;
             } else {
+                pc.set_derived();   // (the energies do not use these)
                 double sc;
                 double fo[3] = {0, 0, 0};
                 if constexpr (KIND == KIND_REPULSIONDRAG) {
