@@ -332,12 +332,16 @@ struct parm_system {
             for (int d = 0; d < nd; d++)
                 if (sys[s2].nc[d] < 3) c.any_wrap = 1;
         }
-        // k_force64s (a thread per entry) for lists that leave a warp per list idle,
-        // from where its CTAs of 16 atoms fill the SMs (force kernel, a warp per
-        // list / a thread per entry: 16.4 / 17.4 us on 5003 spheres, 34.5 / 30.1 on
-        // 20,000, 54.8 / 42.9 on 65,536 disks, 290 / 179 on 48 WCA replicas)
+        // Forces without pair slots: k_force64s (a thread per entry) for lists that
+        // leave a warp per list idle, from where its CTAs of 16 atoms fill the SMs
+        // (force kernel, a warp per list / a thread per entry: 16.4 / 17.4 us on 5003
+        // spheres, 34.5 / 30.1 on 20,000, 54.8 / 42.9 on 65,536 disks); k_force64w (a
+        // warp per 32 atoms) from 15 of its warps an SM, for short lists and for the
+        // laws that few pairs of a long one take part in (both sides at its kernel).
         c.list_mean = (uint32_t)std::ceil(std::min(1e6, mean_list()));
-        c.short_lists = n >= 8192 && c.list_mean <= 32u ? 1u : 0u;
+        const bool many = n >= 152u * 15u * 32u;
+        c.f64_way = c.list_mean <= 32u ? (many ? F64_MANY : (n >= 8192 ? F64_SHORT : F64_LISTS))
+                                       : (many && !lj_law() ? F64_MANY : F64_LISTS);
         std::vector<int> newnc;
         for (uint32_t s2 = 0; s2 < nsys; s2++)
             for (int d = 0; d < 3; d++) newnc.push_back(sys[s2].nc[d]);
@@ -607,11 +611,13 @@ struct parm_system {
     // And where they take at most a quarter of the free device memory and 32 GB,
     // and the allocation succeeds: another handle evaluates each pair twice
     // instead, which needs none of it.
+    bool lj_law() const {
+        return kind == PARM_LJCUT || kind == PARM_LJATTRACTCUT ||
+               (kind >= PARM_LJCUT_IEPSISIG && kind <= PARM_LJISH) || kind == PARM_LJATTRACTREPULSESIGS;
+    }
     bool slots_pay() const {
         if (want_slots >= 0) return want_slots != 0;
-        const bool lj = kind == PARM_LJCUT || kind == PARM_LJATTRACTCUT ||
-                        (kind >= PARM_LJCUT_IEPSISIG && kind <= PARM_LJISH) || kind == PARM_LJATTRACTREPULSESIGS;
-        return lj && n >= 16384;
+        return lj_law() && n >= 16384;
     }
     int plan_slots() {
         if (prec != PREC_FP64 || (!c.pairf && !slots_pay())) return PARM_OK;

@@ -720,7 +720,8 @@ __global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
 // the screen, and eight atoms too few survivors for a warp): F64S_ATOMS atoms
 // a CTA, their entries numbered consecutively and screened one per thread, the
 // survivors evaluated one per thread in any order, each force stored at its
-// entry's place, and every entry added in order, zeros included.
+// entry's place, and every entry added in order, zeros included (nothing is
+// added where no pair of the CTA survives).
 // FP64-bound from there (a soft-sphere pair takes ~55 FP64 operations): 54.8 ->
 // 42.9 us on 65,536 harmonic disks, 290 -> 179 us on 48 WCA replicas (~330,000
 // atoms).
@@ -802,6 +803,10 @@ __global__ void __launch_bounds__(F64S_THREADS) k_force64s(DevCtx c) {
         }
         __syncthreads();
         const uint32_t ns = nsurv;
+        if (ns == 0u) {   // (no pair of the CTA interacts: nothing to add)
+            if (base + F64S_CHUNK < nmax) __syncthreads();
+            continue;
+        }
         for (uint32_t q = tid; q < ns; q += F64S_THREADS) {
             const uint32_t a = pa[q] & 127u, i = i0 + a, j = pj[q];
             if (!all_uni || !have) {
@@ -832,6 +837,120 @@ __global__ void __launch_bounds__(F64S_THREADS) k_force64s(DevCtx c) {
     for (int d = 0; d < ND; d++) f[d] = pf[d][tid];
     store_force<ND, MODE>(c, i, f);
 }
+// k_force64 for many atoms: a warp per 32 of them, on its own.  Every lane screens
+// its atom's list, the survivors are numbered consecutively (in list order by
+// atom) and evaluated one per lane, each lane then adds its atom's in order.  No
+// barrier and little work besides the screen, which is all there is to do where
+// few listed pairs interact; its latencies need some fifteen warps an SM.
+// k_force64s / k_force64w, WCA just below contact: 25.5 / 15.5 us at 80,000 atoms
+// in 2D, 175 / 67 us at 600,000, 242 / 123 us in 3D (a thread per atom that
+// walked its list 16, 66 and 175 us); 48 WCA replicas (427,107 atoms) 270 / 191
+// us, 400,000 disks 243 / 199 us; but 100,000 overlapping spheres 102 / 117 us,
+// 65,536 disks 42 / 48 us.  Lists of 55 entries, of which a few interact:
+// k_force64 / k_force64w 95 / 79 us at 80,000 spheres, 521 / 319 us at 400,000.
+constexpr int F64W_WARPS = 4;
+constexpr uint32_t F64W_CHUNK = 16, F64W_BATCH = 128;   // list entries per atom and round; pair forces held at once
+template <int ND, int KIND, int MODE>
+__global__ void __launch_bounds__(32 * F64W_WARPS) k_force64w(DevCtx c) {
+    __shared__ double pf_s[F64W_WARPS][ND][F64W_BATCH];
+    __shared__ double xs_s[F64W_WARPS][ND][32];
+    __shared__ uint32_t pj_s[F64W_WARPS][32u * F64W_CHUNK];   // survivors: neighbour,
+    __shared__ uint8_t pa_s[F64W_WARPS][32u * F64W_CHUNK];    // atom | 128 when the image needs the remainder
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t i0 = (blockIdx.x * F64W_WARPS + warp) * 32u, i = i0 + lane;
+    release_next();
+    // (list lengths, lists and ranks do not change in the drift before)
+    const bool all_uni = (c.uniform & UNI_ALL) == UNI_ALL;
+    const uint32_t s = i < c.n ? c.atom_sys[i] : 0u;
+    const bool live = i < c.n && c.active[s];
+    const uint32_t nn = live && c.rank[i] != NOT_MEMBER ? c.nnb[i] : 0u;
+    const uint32_t nmax = __reduce_max_sync(0xFFFFFFFFu, nn);
+    const SysConst& S = c.sys[s];
+    double (*pf)[F64W_BATCH] = pf_s[warp];
+    double (*xs)[32] = xs_s[warp];
+    uint32_t* pj = pj_s[warp];
+    uint8_t* pa = pa_s[warp];
+    wait_previous();
+    float4 Ai, Bi, Qi = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (nn) {
+        double xi[3] = {0, 0, 0};
+        load3<ND>(c.x, i, xi);
+#pragma unroll
+        for (int d = 0; d < ND; d++) xs[d][lane] = xi[d];
+        ld_pos_coherent(c.pos, i, Ai, Bi);
+        Qi = c.prm32[i];
+    }
+    const uint4* row = reinterpret_cast<const uint4*>(c.nbr + (size_t)i * c.maxnb);   // (maxnb: a multiple of 8)
+    double f[3] = {0, 0, 0};
+    PairC pc;
+    bool have = false;
+    for (uint32_t base = 0; base < nmax; base += F64W_CHUNK) {
+        uint32_t keep = 0u, wraps = 0u;
+        uint4 J[F64W_CHUNK / 4];
+#pragma unroll
+        for (uint32_t g = 0; g < F64W_CHUNK / 4; g++)
+            J[g] = base + 4u * g < nn ? __ldg(row + (base >> 2) + g) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (uint32_t g = 0; g < F64W_CHUNK / 4; g++) {
+            if (base + 4u * g >= nmax) break;   // uniform in the warp
+            const uint32_t js[4] = {J[g].x, J[g].y, J[g].z, J[g].w};
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                bool wrap;
+                if (base + 4u * g + u < nn && screen64<ND, KIND>(c, S, Ai, Bi, Qi, js[u], wrap)) {
+                    keep |= 1u << (4u * g + u);
+                    wraps |= (wrap ? 1u : 0u) << (4u * g + u);
+                }
+            }
+        }
+        uint32_t end = __popc(keep);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, end, o);
+            if (lane >= (uint32_t)o) end += u;
+        }
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, end, 31), first = end - __popc(keep);
+        uint32_t q = first;
+#pragma unroll
+        for (uint32_t g = 0; g < F64W_CHUNK / 4; g++) {
+            const uint32_t js[4] = {J[g].x, J[g].y, J[g].z, J[g].w};
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                if ((keep >> (4u * g + u)) & 1u) {
+                    pj[q] = js[u];
+                    pa[q] = (uint8_t)(lane | (((wraps >> (4u * g + u)) & 1u) << 7));
+                    q++;
+                }
+            }
+        }
+        __syncwarp();
+        for (uint32_t b0 = 0; b0 < total; b0 += F64W_BATCH) {
+            const uint32_t b1 = min(total, b0 + F64W_BATCH);
+            for (uint32_t t = b0 + lane; t < b1; t += 32u) {
+                const uint32_t w = pa[t], a = w & 31u, ia = i0 + a, j = pj[t];
+                if (!all_uni || !have) {
+                    pc = pair_constants<KIND>(c, ia, j, c.rank[ia] > c.rank[j]);
+                    have = true;
+                }
+                double xi[3] = {0, 0, 0}, fo[3];
+#pragma unroll
+                for (int d = 0; d < ND; d++) xi[d] = xs[d][a];
+                force_of_pair<ND, KIND>(c, c.sys[c.atom_sys[ia]], ia, j, xi, (w & 128u) != 0u, pc, fo);
+#pragma unroll
+                for (int d = 0; d < ND; d++) pf[d][t - b0] = fo[d];
+            }
+            __syncwarp();
+            const uint32_t hi = min(end, b1);
+            for (uint32_t t = max(first, b0); t < hi; t++) {
+#pragma unroll
+                for (int d = 0; d < ND; d++) f[d] = f[d] + pf[d][t - b0];
+            }
+            __syncwarp();
+        }
+    }
+    if (live) store_force<ND, MODE>(c, i, f);
+}
+
 template <int ND, int KIND>
 __global__ void __launch_bounds__(F64_THREADS) k_pair64(DevCtx c) {
     forces64<ND, KIND, FM_FORCES, true>(c);
@@ -1008,7 +1127,13 @@ static void force64_nd_kind(const DevCtx& c, cudaStream_t s, int mode) {
         else k_sum64<ND, FM_FORCES><<<gs, 32 * SUM64_WARPS, 0, s>>>(c);
         return;
     }
-    if (c.short_lists) {
+    if (c.f64_way == F64_MANY) {
+        const unsigned gs = grid_for(c.n, 32 * F64W_WARPS);
+        if (mode == FM_FORCES_A) launch_after(c, k_force64w<ND, KIND, FM_FORCES_A>, gs, 32 * F64W_WARPS, 0, s, c);
+        else launch_after(c, k_force64w<ND, KIND, FM_FORCES>, gs, 32 * F64W_WARPS, 0, s, c);
+        return;
+    }
+    if (c.f64_way == F64_SHORT) {
         const unsigned gs = grid_for(c.n, F64S_ATOMS);
         if (mode == FM_FORCES_A) launch_after(c, k_force64s<ND, KIND, FM_FORCES_A>, gs, F64S_THREADS, 0, s, c);
         else launch_after(c, k_force64s<ND, KIND, FM_FORCES>, gs, F64S_THREADS, 0, s, c);

@@ -47,6 +47,12 @@ struct NlcgSys {
     double iters;   // secant iterations of this time step (a bound on the loop besides sec)
 };
 
+enum F64Way : uint32_t {
+    F64_LISTS = 0,   // a warp per list (k_force64)
+    F64_SHORT = 1,   // a thread per list entry (k_force64s)
+    F64_MANY = 2,    // a warp per 32 atoms (k_force64w)
+};
+
 struct DevCtx {
     int nd;
     int prec;
@@ -115,7 +121,7 @@ struct DevCtx {
     uint32_t* nbr;
     uint32_t* nnb;
     uint32_t list_mean;    // expected entries per list, in the densest system
-    uint32_t short_lists;  // FP64 path: lists of about 32 entries or fewer (k_force64s)
+    uint32_t f64_way;      // FP64 path: kernel for forces without pair slots (F64Way)
     // FP64 path: each listed pair's force, computed once for its first atom (the
     // one of higher rank) in slot half_base[first] + entry; null: not kept
     // (pair64.cu).  A system's slots start at atom_off * maxnb / 2.

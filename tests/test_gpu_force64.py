@@ -122,3 +122,54 @@ def test_slots_of_tiny_systems():
     for k in ("x", "v", "a", "f"):
         assert np.array_equal(out[0][0][k], out[1][0][k])
     assert np.array_equal(out[0][1], out[1][1]) and out[0][1].max() > 1
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("n", [2, 16, 17, 18, 33, 130, 240])
+def test_cluster_among_many_atoms(ndim, n):
+    """The kernel for many atoms on lists of one round and more, with more survivors than it holds at once."""
+    w = W.small_random(n=n, ndim=ndim, kind=1, seed=n, phi=3.0, skin=30.0)
+    w.L[:] = 400.0
+    o = make_oracle(w)
+    gap = 40.0   # beyond every list
+    k = 42 if ndim == 3 else 271
+    x = (np.stack(np.meshgrid(*[np.arange(k)] * ndim, indexing="ij"), -1).reshape(-1, ndim) + 0.5) * gap
+    lone = len(x)
+    assert lone > 152 * 15 * 32
+    g = make_gpu(W.Workload("c", ndim, [n, lone], np.array([[400.0] * ndim, [k * gap] * ndim]),
+                            np.concatenate([w.x, x]), np.zeros((n + lone, ndim)),
+                            np.concatenate([w.m, np.ones(lone)]), 1,
+                            np.concatenate([w.params, np.tile(w.params[:1], (lone, 1))]), 30.0))
+    g.set_capacity(n)
+    g.nlist_update(True)
+    o.nl_update(True)
+    assert g.numpairs()[0] == n * (n - 1) // 2
+    g.set_forces(True)
+    o.set_forces(True)
+    st, ref = g.get_atoms(), o.get_state()
+    assert np.array_equal(st["f"][:n], ref["f"]) and not st["f"][n:].any()
+    assert np.array_equal(st["a"][:n], ref["a"])
+
+
+@pytest.mark.parametrize("kind,ndim,expo,skin", [(1, 2, 2.0, 0.2), (1, 3, 2.5, 0.2), (2, 3, 2.0, 0.2), (2, 2, 2.0, 1.5),
+                                                 (1, 2, 3.0, 0.1)])
+def test_many_atoms_and_slots_agree(kind, ndim, expo, skin):
+    """The kernel for many atoms against pair forces kept once per pair: the same bits on ragged batches, one frozen."""
+    ws = [W.small_random(n=n, ndim=ndim, kind=kind, seed=n, phi=0.7, skin=skin, exponent=expo) for n in (70001, 3001, 61)]
+    w = W.Workload("b", ndim, [k.n for k in ws], np.concatenate([k.L for k in ws]), np.concatenate([k.x for k in ws]),
+                   np.concatenate([k.v for k in ws]), np.concatenate([k.m for k in ws]), kind,
+                   np.concatenate([k.params for k in ws]), skin)
+    assert w.n > 152 * 15 * 32
+    dt = 1e-5 if kind == 1 else 1e-14   # (random positions: WCA forces of 1e30)
+    out = []
+    for keep in (True, False):
+        g = make_gpu(w)
+        g.debug_pair_slots(keep)
+        g.nlist_update(False)
+        g.set_forces(True)
+        g.damped(dt, 5.0, 5)
+        g.set_active([1, 0, 1])
+        g.damped(dt, 5.0, 10)
+        out.append(g.get_atoms())
+    for k in ("x", "v", "a", "f"):
+        assert np.array_equal(out[0][k], out[1][k])
