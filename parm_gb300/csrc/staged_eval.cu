@@ -66,6 +66,14 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
     const uint4 bd = c.blk[blockIdx.x];
     const SysConst& S = c.sys[bd.x];
     stg_load_table(c, T, blockIdx.x);
+    const int nc = what == EV_STRESS ? ND * ND : 1;
+    // nothing listed in the block (dilute systems)
+    uint32_t longest = 0u;
+    for (int r = 0; r < T.y1 - T.y0; r++) longest = max(longest, T.hnmax[r]);
+    if (longest == 0u) {
+        if (threadIdx.x < (uint32_t)nc) c.blk_part[(size_t)blockIdx.x * nc + threadIdx.x] = 0.0;
+        return;
+    }
     stg_prefetch<ND>(c, T, true);
     const uint32_t cap = c.stg_cap_eval, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     float4* srec = smem_e;
@@ -206,7 +214,6 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
     }
     if constexpr (!SUMS) acc[0] = (double)count;
     // fixed-order sums over the block
-    const int nc = what == EV_STRESS ? ND * ND : 1;
 #pragma unroll
     for (int q = 0; q < (SUMS ? ND * ND : 1); q++) {
         if (q < nc) {
