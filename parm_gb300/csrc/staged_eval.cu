@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
     const SysConst& S = c.sys[bd.x];
     stg_load_table(c, T, blockIdx.x);
     const int nc = what == EV_STRESS ? ND * ND : 1;
+    const bool pairs_only = !SUMS && what == EV_PAIRS;
     // nothing listed in the block (dilute systems)
     uint32_t longest = 0u;
     for (int r = 0; r < T.y1 - T.y0; r++) longest = max(longest, T.hnmax[r]);
@@ -74,7 +75,7 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
         if (threadIdx.x < (uint32_t)nc) c.blk_part[(size_t)blockIdx.x * nc + threadIdx.x] = 0.0;
         return;
     }
-    stg_prefetch<ND>(c, T, true);
+    if (!pairs_only) stg_prefetch<ND>(c, T, true);
     const uint32_t cap = c.stg_cap_eval, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     float4* srec = smem_e;
     void* sext = smem_e + cap;
@@ -97,7 +98,9 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
             for (uint32_t t = lane + 32u; t < T.cnt[p] && o + t < cap; t += 32u) srank[o + t] = __ldg(&c.rank[T.g0[p] + t]);
         }
     }
-    if (!stg_load_bulk<ND, PRM>(c, T, srec, sext, cap, &bar)) return;   // ends with a barrier
+    // (counting the pairs takes the ranks alone; both ways end with a barrier)
+    if (pairs_only) __syncthreads();
+    else if (!stg_load_bulk<ND, PRM>(c, T, srec, sext, cap, &bar)) return;
     const float* ssig = static_cast<const float*>(sext);
     const float4* sprm = static_cast<const float4*>(sext);
     uint32_t* queue = queue_s[warp];
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
             w0 = w1;
             w1 = p + 2u < nw ? __ldg(row + (size_t)(p + 2u) * a.H) : 0u;
             const bool v0 = 2u * p < nn, v1 = 2u * p + 1u < nn;
-            if (!SUMS && what == EV_PAIRS) {
+            if (pairs_only) {
                 count += (v0 && of_mine(word & 0xFFFFu) ? 1u : 0u) + (v1 && of_mine(word >> 16) ? 1u : 0u);
                 continue;
             }
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(STG_THREADS, 4) k_eval_stg(DevCtx c, int what)
             }
         }
     }
-    if (SUMS || what != EV_PAIRS) {
+    if (!pairs_only) {
         __syncwarp();
         if (lane < waiting) evaluate(queue[lane]);
     }
