@@ -191,11 +191,11 @@ __device__ __forceinline__ PairC combine(const AtomPrm& A, const AtomPrm& B, uin
 }
 
 // b^(n - 1) of the soft repulsions: pow(b, 1) == b exactly; the Hertzian
-// exponent 5/2 as b sqrt(b), two roundings (within an ulp and a half, closer
-// to b^1.5 than the device's pow in general, at a tenth of its FP64 operations)
+// exponent 5/2 rounded once (three_halves), in a fraction of the FP64 operations of
+// the device's pow
 __device__ __forceinline__ double power_m1(double b, double n) {
     if (n == 2.0) return b;
-    if (n == 2.5) return b * sqrt(b);
+    if (n == 2.5) return three_halves(b);
     return pow(b, n - 1);
 }
 
