@@ -96,6 +96,7 @@ __device__ __forceinline__ void kick(const DevCtx& c, uint32_t i, double m, doub
 
 // Fused time-step kernel: [kick of the previous step] + drift of this step +
 // FP32 position view + the neighbour-list displacement test (the reference
+// runs that test at the end of the step; positions do not change after the
 // drift, so testing here sees the same values).  Bound by the ~260 B per atom,
 // which takes every warp an SM holds: issuing all of an atom's loads before the
 // first use (58 registers), or arming the next rebuild in the last block (the
@@ -206,16 +207,19 @@ __global__ void __launch_bounds__(BLOCK, MIXED && MODE == DM_VERLET ? 8 : 1) k_k
         if (KICK && !MIXED) static_cast<V*>(c.a)[i] = av;
         if (mob) {
             // fine part of the FP32 position view against the coarse part fixed
-            // at the last rebuild or upload, on the bit patterns (integer and
-            // FP32 instructions only, within one ulp of (float)(x - X) and equal
-            // to it but for rare roundings); an atom that has moved more than
-            // 1/4 from its coarse point is re-anchored (any multiple of 1/8 is a
-            // valid coarse point)
+            // at the last rebuild or upload; an atom that has moved more than 1/4
+            // from its coarse point is re-anchored (any multiple of 1/8 is a valid
+            // coarse point).  FP64 path: x - X in FP64 (exact), rounded; mixed path:
+            // on the bit patterns (integer and FP32 instructions only, within one
+            // ulp of that and equal to it but for rare roundings)
             float4 A = c.pos[2 * (size_t)i], B;
-            B.x = fine_bits(x[0], A.x);
-            B.y = fine_bits(x[1], A.y);
+            const auto fine = [](double xd, float Xf) {
+                return MIXED ? fine_bits(xd, Xf) : d2f_bits(xd - f2d_bits(Xf));
+            };
+            B.x = fine(x[0], A.x);
+            B.y = fine(x[1], A.y);
             B.z = 0.f;
-            if constexpr (ND == 3) B.z = fine_bits(x[2], A.z);
+            if constexpr (ND == 3) B.z = fine(x[2], A.z);
             B.w = 0.f;
             if (fabsf(B.x) > 0.25f || fabsf(B.y) > 0.25f || fabsf(B.z) > 0.25f) {
                 posq_split2(x[0], A.x, B.x);
