@@ -18,9 +18,9 @@
 //            512th of a turn from the table, the rest by angle addition;
 //   sqrt:    Newton's method on the reciprocal root with a final correction by
 //            the exact remainder.
-// Error in units of 2^-53 of the radius, 1.2 million normals against 113-bit
-// arithmetic: at most 3.4, 0.59 rms (log, sqrt and sincos of the library: 9.4
-// and 2.2, mostly the rounded angle).  48 WCA replicas of 256 to 32768 atoms,
+// Error in units of 2^-53 of the radius, against 113-bit arithmetic: at most 3.2,
+// 0.58 rms over 1.2 million normals (log, sqrt and sincos of the library: 9.4 and
+// 2.2, mostly the rounded angle).  48 WCA replicas of 256 to 32768 atoms,
 // 16 steps with the records read back: 6.11 -> 4.54 ms.
 #pragma once
 #include <cmath>
@@ -108,10 +108,12 @@ __device__ __forceinline__ double noise_radius(const NoiseTable* t, unsigned lon
     double lo = __fma_rn(r, -2.0, __dsub_rn(T, hi));
     lo = __fma_rn(ed, L2L, lo);
     const float rf = d2f_chop(r);
-    const float tail = rf * fmaf(rf, 1.0f / 3.0f, -0.4f);   // r^5 and r^6: below 2^-42 of the sum
+    // r^5 to r^7, below 2^-33 of the sum; without r^7 the radius of u just above 255 / 256, where r is -2^-8 and the
+    // first term is all there is beside it, was off by 2.8 units
+    const float tail = rf * fmaf(rf, fmaf(rf, -2.0f / 7.0f, 1.0f / 3.0f), -0.4f);
     const double P = __fma_rn(r, __fma_rn(r, __dadd_rn(f2d_flush(tail), 0.5), -2.0 / 3.0), 1.0);
     double x = __dadd_rn(hi, __fma_rn(__dmul_rn(r, r), P, lo));
-    if (__double2hiint(x) <= 0x00100000) return 0.0;   // u = 1 (x is 0 to rounding)
+    if (w >> 54) return 0.0;   // u = 1 (x is 0 only to rounding, of either sign)
     float y0;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d2f_chop(x)));
     const double y = f2d_flush(y0), h = f2d_flush(0.5f * y0);
