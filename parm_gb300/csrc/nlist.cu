@@ -292,7 +292,7 @@ __global__ void k_scatter(DevCtx c) {
 template <int ND, uint32_t LANES>
 __global__ void k_sortgather(DevCtx c, uint32_t parts) {
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / LANES, lane = threadIdx.x % LANES;
-    const uint32_t b = w / parts, part = w - b * parts;
+    const uint32_t b = parts == 1u ? w : w / parts, part = w - b * parts;
     uint32_t lo = 0u, cnt = 0u;
     if (b < c.nbucket) {
         const uint32_t s = c.bucket_sys[b];
@@ -308,11 +308,21 @@ __global__ void k_sortgather(DevCtx c, uint32_t parts) {
         const uint32_t o = on ? c.perm[lo + q0 + lane] : 0u;
         const uint32_t rk = on ? c.rank[o] : 0xFFFFFFFFu;
         uint32_t pos = 0u;
-        for (uint32_t t0 = 0; t0 < most; t0 += LANES) {
-            uint32_t kt = rk;
-            if (t0 != q0) kt = t0 + lane < cnt ? c.rank[c.perm[lo + t0 + lane]] : 0xFFFFFFFFu;
-            const uint32_t m = min(LANES, most - t0);
-            for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt, j, LANES) < rk ? 1u : 0u;
+        for (uint32_t t0 = 0; t0 < most; t0 += 4u * LANES) {
+            uint32_t kt[4];   // four groups of ranks, their loads in flight together
+#pragma unroll
+            for (uint32_t g = 0; g < 4u; g++) {
+                const uint32_t t = t0 + g * LANES;
+                kt[g] = rk;
+                if (t != q0) kt[g] = t + lane < cnt ? c.rank[c.perm[lo + t + lane]] : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (uint32_t g = 0; g < 4u; g++) {
+                const uint32_t t = t0 + g * LANES;
+                if (t >= most) break;   // uniform in the warp
+                const uint32_t m = min(LANES, most - t);
+                for (uint32_t j = 0; j < m; j++) pos += __shfl_sync(0xFFFFFFFFu, kt[g], j, LANES) < rk ? 1u : 0u;
+            }
         }
         if (on) move_atom<ND>(c, o, lo + pos, rk, b);
     }
@@ -1014,11 +1024,12 @@ static void sortgather(const DevCtx& c, cudaStream_t s) {
     // eight where other systems' cells alone give every SM its warps
     const uint32_t parts = std::max(1u, std::min((c.cell_mean + 31u) / 32u, std::max(8u, 152u * 32u / c.nbucket)));
     const auto grid = [&](uint32_t lanes) { return (unsigned)(((size_t)c.nbucket * parts * lanes + BLOCK - 1) / BLOCK); };
-    // lanes per cell: a warp where cells hold more than eight atoms, else eight
-    // lanes, or four where eight for each cell would fill the SMs more than once;
-    // sixteen where a few large cells among them would otherwise be what all wait for
+    // lanes per cell: a warp where cells hold more than eight atoms or a warp each
+    // does not fill the SMs, else eight lanes, or four where eight for each cell
+    // would fill the SMs more than once; sixteen where a few large cells among them
+    // would otherwise be what all wait for
     const uint32_t mean = c.n / c.nbucket + 1u;
-    if (mean > 8u) k_sortgather<ND, 32><<<grid(32), BLOCK, 0, s>>>(c, parts);
+    if (mean > 8u || c.nbucket < 152u * 32u) k_sortgather<ND, 32><<<grid(32), BLOCK, 0, s>>>(c, parts);
     else if (c.cell_mean > 32u && c.nbucket < 20000u) k_sortgather<ND, 16><<<grid(16), BLOCK, 0, s>>>(c, parts);
     else if (mean > 4u || c.nbucket < 40000u) k_sortgather<ND, 8><<<grid(8), BLOCK, 0, s>>>(c, parts);
     else k_sortgather<ND, 4><<<grid(4), BLOCK, 0, s>>>(c, parts);
