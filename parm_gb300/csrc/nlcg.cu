@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(BLOCK) k_nlcg_stepx(DevCtx c, int use_cond, cu
 // OriginBox::resize(Lfac) (src/box.hpp:125-128) of the systems that stepped,
 // with every quantity derived from the box; when a cell becomes narrower than
 // the list radius the system's grid shrinks in place (fewer cells along that
-// axis; its bucket range keeps its size, the unused tail is zeroed).  A grid
+// axis; its bucket range keeps its size).  A grid
 // only shrinks here; the host regrids wider boxes between calls.
 // ---------------------------------------------------------------------------
 template <int ND>
@@ -178,7 +178,6 @@ __global__ void k_nlcg_box(DevCtx c) {
     SysConst& S = const_cast<SysConst&>(c.sys[s]);
     const double f = c.nlcg[s].lfac;
     const double w = S.cellmin;
-    const uint32_t ncell_old = S.ncell;
     bool regrid = false;
 #pragma unroll
     for (int d = 0; d < ND; d++) {
@@ -203,10 +202,8 @@ __global__ void k_nlcg_box(DevCtx c) {
     }
     if (regrid) {
         S.ncell = (uint32_t)(S.nc[0] * S.nc[1] * S.nc[2]);
-        // counts left in buckets past the new non-member bucket would be
-        // scanned into nothing but must not carry stale sums
-        const uint32_t b0 = c.bucket_off[s];
-        for (uint32_t b = S.ncell + 1; b <= ncell_old; b++) c.cell_count[b0 + b] = 0u;
+        // (the counts of the buckets past the new non-member bucket are zero, as all
+        // counts are between rebuilds)
         // the current lists index atoms, not cells: they stay valid, and the
         // next rebuild (when the displacement test asks for one) bins on this grid
     }

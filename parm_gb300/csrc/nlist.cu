@@ -99,8 +99,7 @@ __global__ void k_bin(DevCtx c) {
 // two passes (block aggregates; offsets, where each block first sums the
 // aggregates before its own: a pass for that sum in between cost 20,011 disks,
 // which rebuild every other step, 0.8 us of their 49 us a step).  Only buckets of
-// flagged systems are written; other systems' counts are stale but never cross a
-// segment boundary.
+// flagged systems are written, and their counts cleared; other systems have none.
 // ---------------------------------------------------------------------------
 constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_ITEMS = 8;

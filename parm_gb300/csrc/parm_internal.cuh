@@ -57,7 +57,7 @@ enum StatusBits : uint32_t {
     ST_NBR_OVERFLOW = 1u << 0,   // an atom had more neighbours than the list capacity
     ST_NONFINITE = 1u << 1,      // a non-finite position was binned
     ST_CELL_RANGE = 1u << 2,     // a cell index fell outside its system's grid (bug guard)
-    ST_SORT_CAP = 1u << 3,       // FP64 path: a neighbour list longer than the in-thread sort buffer
+    ST_SORT_CAP = 1u << 3,       // FP64 path: a neighbour list longer than the list sort takes
     ST_TILE_OVERFLOW = 1u << 4,  // a tile had more distinct neighbours than its capacity
     ST_IMAGE_RANGE = 1u << 5,    // an atom is more than 7 box lengths from its tile frame
     ST_STAGE_TIMEOUT = 1u << 6,  // a cell block's bulk copies did not complete within the wait limit
