@@ -192,7 +192,9 @@ PARM_FPB_HD double three_halves(double b) {
 #if defined(__CUDA_ARCH__)
     const double s = __dsqrt_rn(b), p = __dmul_rn(b, s);
     const double e = __fma_rn(-s, s, b), d = __fma_rn(b, s, -p);
-    return __dadd_rn(p, __fma_rn(__dmul_rn(0.5, s), e, d));
+    // s / 2 by its exponent (0 stays 0), off the FP64 pipe
+    const double h = __hiloint2double(max(__double2hiint(s), 0x00100000) - 0x00100000, __double2loint(s));
+    return __dadd_rn(p, __fma_rn(h, e, d));
 #else
     const double s = std::sqrt(b), p = b * s;
     const double e = std::fma(-s, s, b), d = std::fma(b, s, -p);
