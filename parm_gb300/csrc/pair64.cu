@@ -722,9 +722,8 @@ __global__ void __launch_bounds__(F64_THREADS) k_force64(DevCtx c) {
 // survivors evaluated one per thread in any order, each force stored at its
 // entry's place, and every entry added in order, zeros included (nothing is
 // added where no pair of the CTA survives).
-// FP64-bound from there (a soft-sphere pair takes ~55 FP64 operations): 54.8 ->
-// 42.9 us on 65,536 harmonic disks, 290 -> 179 us on 48 WCA replicas (~330,000
-// atoms).
+// FP64-bound from there (a soft-sphere pair takes ~55 FP64 operations): k_force64 /
+// this 54.8 / 42.9 us on 65,536 harmonic disks, 34.5 / 30.1 us on 20,000 spheres.
 constexpr int F64S_THREADS = 128;
 constexpr uint32_t F64S_ATOMS = 16, F64S_CHUNK = 32;   // entries per atom and round
 constexpr uint32_t F64S_CAP = F64S_ATOMS * F64S_CHUNK;

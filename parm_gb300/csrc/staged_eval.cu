@@ -18,11 +18,11 @@ namespace parm {
 // energy is near zero or whose distance is near its cut-off, where the last
 // bit of the displacement or a quotient may decide, is evaluated with that
 // kernel's own arithmetic.
-// Measured at 131,072 LJ atoms (one GB300): energy 100 us, virial 123, stress
-// 229, contacts 86, pairs 36; bound by the staging's latency and, the stress, by
-// its FP64 sums.  (Expanding the lists to row-major ones, 101 to 124 us a call,
-// and walking those with a thread per atom took 215 us on top on average, 338
-// for the stress.)
+// Measured at 131,072 LJ atoms (one GB300, cold caches): energy 123 us, virial
+// 141, stress 238, contacts 89, pairs 51; bound by the staging's latency (no unit
+// above half) and, the stress, by its FP64 sums (71 % of the pipe).  (Expanding
+// the lists to row-major ones, 101 to 124 us a call, and walking those with a
+// thread per atom took 215 us on top on average, 338 for the stress.)
 // ---------------------------------------------------------------------------
 constexpr uint32_t EVQ = 96;   // queue per warp: fewer than 32 waiting and two entries of each lane
 
