@@ -1659,6 +1659,7 @@ int parm_set_interaction(parm_system* S, int kind, const double* params, const u
     S->c.kind = device_kind(kind);
     S->c.uniform = uni;
     if (S->prec == PREC_FP64) S->unbuilt = true;   // (pair slots are by the ranks of the last build)
+    TRY(S->request_rebuild_all());   // ignorechanged = true; before anything below can fail
     launch_posq(S->c, S->st);
     CUDA_TRY(cudaGetLastError());
     TRY(S->setup_cells());
@@ -1674,7 +1675,7 @@ int parm_set_interaction(parm_system* S, int kind, const double* params, const u
     S->c.staged = (S->stg_ok && S->want_staged) ? 1u : 0u;
     S->stg_pending = false;
     if (S->c.staged != was) S->clear_graphs();
-    return S->request_rebuild_all();  // ignorechanged = true
+    return PARM_OK;
 }
 
 int parm_set_lees_edwards(parm_system* S, const double* gamma) {
