@@ -302,7 +302,9 @@ __global__ void k_sortgather(DevCtx c, uint32_t parts) {
         }
     }
     const uint32_t most = LANES == 32u ? cnt : __reduce_max_sync(0xFFFFFFFFu, cnt);   // uniform in the warp
-    for (uint32_t q0 = LANES * part; q0 < most; q0 += LANES * parts) {
+    // (the groups of a warp may be different parts of a cell: all stay for the shuffles of the longest)
+    for (uint32_t q0 = LANES * part; LANES == 32u ? q0 < most : __any_sync(0xFFFFFFFFu, q0 < most) != 0;
+         q0 += LANES * parts) {
         const bool on = q0 + lane < cnt;
         const uint32_t o = on ? c.perm[lo + q0 + lane] : 0u;
         const uint32_t rk = on ? c.rank[o] : 0xFFFFFFFFu;

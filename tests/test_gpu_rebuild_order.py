@@ -101,3 +101,22 @@ def test_sparse_cells(precision, ndim, n, side):
     assert np.array_equal(st["x"], x) and np.array_equal(st["v"], w.v) and np.array_equal(st["m"], m)
     tree = cKDTree(np.mod(x, L), boxsize=L)
     assert int(g.numpairs()[0]) == len(tree.query_pairs(rl, output_type="ndarray"))
+
+
+@pytest.mark.parametrize("n,side", [(9001, 1.0), (30011, 1.2), (50021, 1.4)])
+def test_dense_cells_among_sparse_ones(n, side):
+    """Four cells of some 70 atoms in a batch of cells of one or two: sixteen, eight and four lanes a group, three groups
+    a cell.  The pairs of both systems are those of a tree, and no atom is lost."""
+    cKDTree = pytest.importorskip("scipy.spatial").cKDTree
+    rng, rl = np.random.default_rng(n), 1.29
+    sizes, L = [280, n], [2.59, side * n ** 0.5]
+    x = np.concatenate([rng.uniform(0, b, size=(k, 2)) for k, b in zip(sizes, L)])
+    w = W.Workload("d", 2, sizes, np.repeat(np.array(L)[:, None], 2, axis=1), x, x * 0.5, 1.0 + np.arange(len(x)) % 3, 1,
+                   np.tile([1.0, 1.0, 2.0], (len(x), 1)), rl - 1.0)
+    g = make_gpu(w)
+    for _ in range(3):
+        g.nlist_update(True)
+    st = g.get_atoms()
+    assert np.array_equal(st["x"], x) and np.array_equal(st["v"], w.v) and np.array_equal(st["m"], w.m)
+    trees = [cKDTree(p, boxsize=b) for p, b in zip(np.split(x, [280]), L)]
+    assert [int(k) for k in g.numpairs()] == [len(t.query_pairs(rl, output_type="ndarray")) for t in trees]
